@@ -44,12 +44,13 @@ constexpr int kCounterWords = 8;   // cwgpu_context::d_counter
 // 5 CTAs (20 warps) per SM, i.e. 96 registers: measured faster than the 113
 // registers and 4 CTAs per SM the compiler picks for the long-pair kernel
 // unbounded (1000 x 1523 protein family, 200 sequences: 110.3 vs 114.7 ms).
-template <int RS>
+// GEN: any gap penalties (cwgpu::padding_sound says when the other form holds).
+template <int RS, bool GEN>
 __global__ void __launch_bounds__(kWarpsPerBlock * 32, 5)
     k_pairwise(cwgpu::PairArgs g, long long single) {
-    __shared__ int smat[CWGPU_NUMRES * CWGPU_NUMRES];
+    __shared__ int smat[cwgpu::kSmatWords];
     extern __shared__ __align__(16) uint16_t region_all[];
-    for (int i = threadIdx.x; i < CWGPU_NUMRES * CWGPU_NUMRES; i += blockDim.x) smat[i] = g.matrix[i];
+    cwgpu::stage_matrix(smat, g.matrix);
     __syncthreads();
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int wpb = blockDim.x >> 5;
@@ -67,14 +68,14 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32, 5)
     int2* bufB = bufA + (g.lmax + 1);
     unsigned long long acc[3] = {0, 0, 0};
     if (single >= 0) {
-        if (slot == 0) cwgpu::align_pair<RS>(g, single, X, bufA, bufB, acc);
+        if (slot == 0) cwgpu::align_pair<RS, GEN>(g, single, X, bufA, bufB, acc);
     } else {
         for (;;) {
             unsigned long long k = 0;
             if (lane == 0) k = atomicAdd(g.counter, 1ULL);
             k = __shfl_sync(cwgpu::kFull, k, 0);
             if (k >= (unsigned long long)g.npairs) break;
-            cwgpu::align_pair<RS>(g, (long long)g.order[k], X, bufA, bufB, acc);
+            cwgpu::align_pair<RS, GEN>(g, (long long)g.order[k], X, bufA, bufB, acc);
         }
     }
     if (lane == 0 && g.cells && (acc[0] | acc[1] | acc[2])) {
@@ -149,7 +150,7 @@ constexpr int kShareRows = 64;  // frames with fewer rows stay with the warp tha
 // that idle warps can take it. The phase ends when the stack is empty and no
 // warp holds a frame. A warp that finds the stack empty while others still
 // hold frames waits (bounded, like the stripe hand-overs).
-template <int RS>
+template <int RS, bool GEN>
 __device__ void cta_small_frames(CtaCtl& C, const int8_t* s1, const int8_t* s1r, int n, const int8_t* s2,
                                  const int8_t* s2r, int m, int go, int ge, int2* bufA, int2* bufB, const cwgpu::Env& X,
                                  const CtaArgs& ca, int& ident, int& match, long long& cells) {
@@ -215,7 +216,7 @@ __device__ void cta_small_frames(CtaCtl& C, const int8_t* s1, const int8_t* s1r,
         fn = __shfl_sync(cwgpu::kFull, fn, 0);
         int mmf = 0, id = 0, mt = 0;
         long long ce = 0;
-        cwgpu::mm_align<RS, true, true>(s1, s1r, n, s2, s2r, m, fa, fb, fm & ~kRootBit, fn, go, ge, bufA, bufB, X, mmf,
+        cwgpu::mm_align<RS, GEN, true, true>(s1, s1r, n, s2, s2r, m, fa, fb, fm & ~kRootBit, fn, go, ge, bufA, bufB, X, mmf,
                                         id, mt, ce, &fs);
         ident += id;
         match += mt;
@@ -233,7 +234,7 @@ __device__ void cta_small_frames(CtaCtl& C, const int8_t* s1, const int8_t* s1r,
 }
 
 // diff() + tracePath of one pair by the whole CTA (every thread calls).
-template <int RS>
+template <int RS, bool GEN>
 __device__ void cta_diff(CtaCtl& C, const int8_t* s1, const int8_t* s1r, int n, const int8_t* s2, const int8_t* s2r,
                          int m, int A0, int B0, int M0, int N0, int go, int ge, int2* bufs, size_t stride, int nw,
                          const cwgpu::Env& X, cwgpu::MwSync& mw, unsigned long long& epoch, const CtaArgs& ca,
@@ -300,7 +301,7 @@ __device__ void cta_diff(CtaCtl& C, const int8_t* s1, const int8_t* s1r, int n, 
         t.fo = go;
         mw.epoch = (++epoch) << 32;
         cwgpu::Best unused;
-        cwgpu::sweep_mw<RS, cwgpu::MODE_GLOBAL>(t, go, ge, 0, X, unused, bufs, stride, slot0, warp - slot0, gw, mw,
+        cwgpu::sweep_mw<RS, cwgpu::MODE_GLOBAL, GEN>(t, go, ge, 0, X, unused, bufs, stride, slot0, warp - slot0, gw, mw,
                                                 &C.stop);
         __syncthreads();
         if (warp == 0) {
@@ -338,9 +339,9 @@ __device__ void cta_diff(CtaCtl& C, const int8_t* s1, const int8_t* s1r, int n, 
         }
         __syncthreads();
         if (C.nsmall > kCtaSmall - 4)
-            cta_small_frames<RS>(C, s1, s1r, n, s2, s2r, m, go, ge, bufA, bufB, X, ca, ident, match, ncell);
+            cta_small_frames<RS, GEN>(C, s1, s1r, n, s2, s2r, m, go, ge, bufA, bufB, X, ca, ident, match, ncell);
     }
-    cta_small_frames<RS>(C, s1, s1r, n, s2, s2r, m, go, ge, bufA, bufB, X, ca, ident, match, ncell);
+    cta_small_frames<RS, GEN>(C, s1, s1r, n, s2, s2r, m, go, ge, bufA, bufB, X, ca, ident, match, ncell);
     if (lane == 0) {
         C.ident[warp] = ident;
         C.match[warp] = match;
@@ -359,7 +360,7 @@ __device__ void cta_diff(CtaCtl& C, const int8_t* s1, const int8_t* s1r, int n, 
 }
 
 // FullPairwiseAlign.cpp:112-183 for pair q by the whole CTA.
-template <int RS>
+template <int RS, bool GEN>
 __device__ void cta_pair(const cwgpu::PairArgs& g, long long q, CtaCtl& C, const cwgpu::Env& X, int2* bufs,
                          size_t stride, int nw, const CtaArgs& ca, unsigned long long& epoch,
                          unsigned long long (&acc)[3]) {
@@ -394,7 +395,7 @@ __device__ void cta_pair(const cwgpu::PairArgs& g, long long q, CtaCtl& C, const
         t.buf = nullptr;
         mw.epoch = (++epoch) << 32;
         cwgpu::Best b;
-        cwgpu::sweep_mw<RS, cwgpu::MODE_LOCAL_FWD>(t, go, ge, 0, X, b, bufs, stride, 0, warp, nw, mw, &C.stop);
+        cwgpu::sweep_mw<RS, cwgpu::MODE_LOCAL_FWD, GEN>(t, go, ge, 0, X, b, bufs, stride, 0, warp, nw, mw, &C.stop);
         if (lane == 0) {
             C.bval[warp] = b.val;
             C.bkey[warp] = b.key;
@@ -423,8 +424,8 @@ __device__ void cta_pair(const cwgpu::PairArgs& g, long long q, CtaCtl& C, const
             r.fo = 0;
             r.buf = nullptr;
             mw.epoch = (++epoch) << 32;
-            cwgpu::sweep_mw<RS, cwgpu::MODE_LOCAL_REV>(r, go, ge, max_score, X, b, bufs, stride, 0, warp, nw, mw,
-                                                       &C.stop);
+            cwgpu::sweep_mw<RS, cwgpu::MODE_LOCAL_REV, GEN>(r, go, ge, max_score, X, b, bufs, stride, 0, warp, nw, mw,
+                                                            &C.stop);
             if (lane == 0) {
                 C.bval[warp] = b.val;
                 C.bkey[warp] = b.key;
@@ -445,7 +446,7 @@ __device__ void cta_pair(const cwgpu::PairArgs& g, long long q, CtaCtl& C, const
         // diff + tracePath
         int mm = 0, ident = 0, matches = 0;
         long long dcells = 0;
-        cta_diff<RS>(C, s1, s1r, n, s2, s2r, m, sb1 - 1, sb2 - 1, se1 - sb1 + 1, se2 - sb2 + 1, go, ge, bufs, stride,
+        cta_diff<RS, GEN>(C, s1, s1r, n, s2, s2r, m, sb1 - 1, sb2 - 1, se1 - sb1 + 1, se2 - sb2 + 1, go, ge, bufs, stride,
                      nw, X, mw, epoch, ca, mm, ident, matches, dcells);
         acc[2] += (unsigned long long)dcells;
         // distance (:170-181), float arithmetic with IEEE rounding.
@@ -472,11 +473,12 @@ __device__ void cta_pair(const cwgpu::PairArgs& g, long long q, CtaCtl& C, const
 }
 
 // Persistent: each CTA takes the next pair of the longest-first queue.
+template <bool GEN>
 __global__ void __launch_bounds__(kCtaMaxWarps * 32, 1) k_pairwise_cta(cwgpu::PairArgs g, CtaArgs ca) {
-    __shared__ int smat[CWGPU_NUMRES * CWGPU_NUMRES];
+    __shared__ int smat[cwgpu::kSmatWords];
     __shared__ CtaCtl C;
     extern __shared__ __align__(16) uint16_t region_all[];
-    for (int i = threadIdx.x; i < CWGPU_NUMRES * CWGPU_NUMRES; i += blockDim.x) smat[i] = g.matrix[i];
+    cwgpu::stage_matrix(smat, g.matrix);
     const int nw = blockDim.x >> 5, warp = threadIdx.x >> 5;
     if (threadIdx.x < kCtaMaxWarps) C.prog[threadIdx.x] = 0;
     if (threadIdx.x == 0) {
@@ -503,7 +505,7 @@ __global__ void __launch_bounds__(kCtaMaxWarps * 32, 1) k_pairwise_cta(cwgpu::Pa
         const long long k = C.q;
         __syncthreads();
         if (k >= g.npairs) break;
-        cta_pair<cwgpu::kR>(g, (long long)g.order[k], C, X, bufs, stride, nw, ca, epoch, acc);
+        cta_pair<cwgpu::kR, GEN>(g, (long long)g.order[k], C, X, bufs, stride, nw, ca, epoch, acc);
     }
     if (threadIdx.x == 0 && g.cells && (acc[0] | acc[1] | acc[2])) {
         atomicAdd(g.cells + 0, acc[0]);
@@ -598,6 +600,12 @@ cudaError_t pinned_grow(unsigned char*& p, size_t& cap, size_t need) {
     return e;
 }
 
+int gap_extend_of(const cwgpu_params& p) {
+    int32_t g = 0, e = 0;
+    cwgpu_gap_penalties(&p, 1, 1, &g, &e);
+    return e;
+}
+
 // Everything the pair kernels and the quick path read, in one arena: the code
 // layout, both offset arrays and the lengths; with params, the residue counts
 // (len1/len2 of FullPairwiseAlign.cpp:100-127) and the gap-open table by
@@ -659,6 +667,7 @@ int stage_inputs(cwgpu_context* ctx) {
             go.push_back(g);
         }
         memcpy(h + o_go, go.data(), 4 * (size_t)(ctx->lmax + 1));
+        ctx->general_gaps = cwgpu_general_gaps(go.data(), ctx->lmax, gap_extend_of(ctx->params));
     }
     if (ctx->has_matrix) {  // over the dense codes, row stride 32 (entries past K unused)
         int32_t* dm = reinterpret_cast<int32_t*>(h + o_mat);
@@ -689,25 +698,25 @@ int refresh_derived(cwgpu_context* ctx) {
     return stage_inputs(ctx);
 }
 
-int gap_extend_of(const cwgpu_params& p) {
-    int32_t g = 0, e = 0;
-    cwgpu_gap_penalties(&p, 1, 1, &g, &e);
-    return e;
-}
-
 size_t block_smem(int K, int warps) { return (size_t)cwgpu::warp_region_bytes(K) * warps; }
 
-// CTAs of k_pairwise<RS> that fit on all SMs at once for an alphabet of K codes.
+// CTAs of k_pairwise<RS> (either form) that fit on all SMs at once for an
+// alphabet of K codes.
 template <int RS>
 cudaError_t pair_grid(int K, int sm_count, int* grid) {
-    int per_sm = 0;
-    cudaError_t e = cudaFuncSetAttribute(k_pairwise<RS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)block_smem(CWGPU_NUMRES, kWarpsPerBlock));
-    if (e == cudaSuccess)
-        e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_pairwise<RS>, kWarpsPerBlock * 32,
-                                                          block_smem(K, kWarpsPerBlock));
-    *grid = (per_sm < 1 ? 1 : per_sm) * sm_count;
-    return e;
+    int fit = INT_MAX;
+    for (auto* k : {k_pairwise<RS, false>, k_pairwise<RS, true>}) {
+        int per_sm = 0;
+        cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                             (int)block_smem(CWGPU_NUMRES, kWarpsPerBlock));
+        if (e == cudaSuccess)
+            e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, kWarpsPerBlock * 32,
+                                                              block_smem(K, kWarpsPerBlock));
+        if (e != cudaSuccess) return e;
+        fit = std::min(fit, std::max(per_sm, 1));
+    }
+    *grid = fit * sm_count;
+    return cudaSuccess;
 }
 
 template <int RS>
@@ -734,18 +743,22 @@ size_t cta_smem(int K, int warps) { return block_smem(K, warps); }
 // 0 when the CTA's shared memory (a score-profile region per warp) does not
 // fit; launches then keep one warp per pair.
 int cta_grid(cwgpu_context* ctx, int warps, int* grid) {
-    int per_sm = 0, optin = 0;
+    int fit = INT_MAX, optin = 0;
     const size_t smem = cta_smem(ctx->K, warps);
-    cudaFuncAttributes fa;
-    CW_CUDA(ctx, cudaFuncGetAttributes(&fa, k_pairwise_cta));
     CW_CUDA(ctx, cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, ctx->device));
     *grid = 0;
-    if (smem + fa.sharedSizeBytes > (size_t)optin) return CWGPU_OK;
-    CW_CUDA(ctx, cudaFuncSetAttribute(k_pairwise_cta, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                      std::max(fa.maxDynamicSharedSizeBytes, (int)smem)));
-    CW_CUDA(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_pairwise_cta, warps * 32, smem));
-    if (per_sm < 1) return CWGPU_OK;
-    *grid = std::min(per_sm * ctx->sm_count, ctx->grid * kWarpsPerBlock / warps);
+    for (auto* k : {k_pairwise_cta<false>, k_pairwise_cta<true>}) {
+        int per_sm = 0;
+        cudaFuncAttributes fa;
+        CW_CUDA(ctx, cudaFuncGetAttributes(&fa, k));
+        if (smem + fa.sharedSizeBytes > (size_t)optin) return CWGPU_OK;
+        CW_CUDA(ctx, cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                          std::max(fa.maxDynamicSharedSizeBytes, (int)smem)));
+        CW_CUDA(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, warps * 32, smem));
+        fit = std::min(fit, per_sm);
+    }
+    if (fit < 1) return CWGPU_OK;
+    *grid = std::min(fit * ctx->sm_count, ctx->grid * kWarpsPerBlock / warps);
     return CWGPU_OK;
 }
 
@@ -797,6 +810,7 @@ cwgpu::PairArgs make_args(cwgpu_context* ctx, const int32_t* d_pairs, const int3
     g.K = ctx->K;
     g.tiny_m = ctx->tiny_m;
     g.tiny_n = ctx->tiny_n;
+    g.general = ctx->general_gaps;
     return g;
 }
 
@@ -846,7 +860,7 @@ cudaError_t launch_persistent(const cwgpu::PairArgs& g, int max_grid, size_t sme
     attr[0].val.priority = priority;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, k_pairwise<RS>, g, -1LL);
+    return cudaLaunchKernelEx(&cfg, g.general ? k_pairwise<RS, true> : k_pairwise<RS, false>, g, -1LL);
 }
 
 // Warps per CTA for a launch of nlong long pairs: the knob, or, when it is 0,
@@ -880,7 +894,7 @@ cudaError_t launch_cta(const cwgpu_context* ctx, const cwgpu::PairArgs& g, int p
     attr[0].val.priority = priority;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, k_pairwise_cta, g, ca);
+    return cudaLaunchKernelEx(&cfg, g.general ? k_pairwise_cta<true> : k_pairwise_cta<false>, g, ca);
 }
 
 // Long pairs of a launch run one CTA per pair when there are few of them: at
@@ -953,6 +967,12 @@ int check_kernel_error(cwgpu_context* ctx) {
 }  // namespace
 
 int cwgpu_stage_inputs(cwgpu_context* ctx) { return stage_inputs(ctx); }
+
+bool cwgpu_general_gaps(const int32_t* go, int lmax, int ge) {
+    for (int L = 1; L <= lmax; ++L)
+        if (!cwgpu::padding_sound(go[L], ge)) return true;
+    return false;
+}
 
 cudaError_t cwgpu_pair_kernel_grids(int K, int sm_count, int* grid, int* grid_short) {
     cudaError_t e = pair_grid<cwgpu::kR>(K, sm_count, grid);
@@ -1367,10 +1387,10 @@ int cwgpu_align_pairs_plain(cwgpu_context* ctx, const int32_t* pairs, int64_t np
     if (e == cudaSuccess) {
         cwgpu::PairArgs g = make_args(ctx, d_pairs, nullptr, npairs, d_dist, d_stats);
         for (int64_t q = 0; q < npairs && e == cudaSuccess; ++q) {
-            if (short_pair(ctx, pairs, q))
-                k_pairwise<cwgpu::kRShort><<<1, 32, block_smem(ctx->K, 1), ctx->stream>>>(g, (long long)q);
-            else
-                k_pairwise<cwgpu::kR><<<1, 32, block_smem(ctx->K, 1), ctx->stream>>>(g, (long long)q);
+            auto* const k = short_pair(ctx, pairs, q)
+                                ? (g.general ? k_pairwise<cwgpu::kRShort, true> : k_pairwise<cwgpu::kRShort, false>)
+                                : (g.general ? k_pairwise<cwgpu::kR, true> : k_pairwise<cwgpu::kR, false>);
+            k<<<1, 32, block_smem(ctx->K, 1), ctx->stream>>>(g, (long long)q);
             e = cudaGetLastError();
         }
     }

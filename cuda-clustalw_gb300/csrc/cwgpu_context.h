@@ -29,6 +29,9 @@ struct PairArgs;
 }
 cudaError_t cwgpu_pair_kernel_grids(int K, int sm_count, int* grid, int* grid_short);
 int cwgpu_pair_kernel_warps_per_cta();
+// Whether some gap-open penalty go[1..lmax] or the extension needs the pair
+// kernels' general form (PairArgs::general).
+bool cwgpu_general_gaps(const int32_t* go, int lmax, int ge);
 cudaError_t cwgpu_enqueue_pair_kernels(const cwgpu::PairArgs& gl, const cwgpu::PairArgs& gs, int grid,
                                        int grid_short, int prio_high, int prio_low, cudaStream_t s, cudaStream_t s2,
                                        cudaEvent_t fork, cudaEvent_t join);
@@ -71,6 +74,7 @@ struct cwgpu_context {
     std::vector<int8_t> host_layout;  // d_codes as built on the host
     std::vector<int64_t> host_poffs;
     std::vector<int32_t> host_go;     // gap open by length 0..: valid for go_params
+    bool general_gaps = false;        // cwgpu_general_gaps of the staged table
     cwgpu_params go_params;
     int8_t* d_codes = nullptr;   // pair kernels' layout (cwgpu_layout.h): guards, forward and reversed copies
     int64_t* d_poffs = nullptr;  // forward copy of each sequence in d_codes

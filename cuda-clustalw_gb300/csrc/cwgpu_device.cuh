@@ -17,12 +17,18 @@
 // the segment reads W columns at a time with one coalesced load and hands to
 // that lane by shuffle, or from the closed-form boundary of the first stripe.
 //
-// E and F are carried shifted by gapOpen+gapExtend (E' = E + goe, F' = F + goe)
-// so each cell costs five integer operations, three of them DPX:
-//   E'(r,c) = max(E'(r-1,c) - ge, H(r-1,c))                __viaddmax_s32
-//   F'(r,c) = max(F'(r,c-1) - ge, H(r,c-1))                __viaddmax_s32
-//   H(r,c)  = max(H(r-1,c-1) + s, max(E', F') - goe [, 0]) max + add + __viaddmax_s32[_relu]
-// which is the reference's recurrence written with fewer operations.
+// A cell costs five integer instructions, three of them on the ALU pipe (64
+// lanes per SM and clock, the pipe that bounds every sweep):
+//   t = H(r-1,c-1) + s                          dp2a (picks one int16 score and adds: FMA pipe)
+//   H = max(E, F, t [, 0])                      __vimax3_s32[_relu]
+//   g = H - (gapOpen + gapExtend)               add (either pipe)
+//   E(r+1,c) = max(E(r,c) - ge, g)              __viaddmax_s32
+//   F(r,c+1) = max(F(r,c) - ge, g)              __viaddmax_s32
+// which is the reference's recurrence with E and F carried one cell ahead.
+// Measured with all operands in registers: 20.2 cells per SM and clock, against
+// 12.7 for the form with two more ALU instructions (an unpack of the score and
+// a second two-way max in place of the three-way one); the 200 x 1523 protein
+// family 110.4 -> 89.0 ms.
 //
 // Scores come from a per-stripe int16 profile in shared memory,
 // prof[code][lane][row], one conflict-free 16-byte load per step and lane
@@ -65,7 +71,7 @@ __host__ __device__ constexpr int warp_region_bytes(int K) {
 //   H(-1, c) = ht0 - c*hts        E(-1, c) = H(-1, c) - eo      (c >= 1)
 //   H(r, 0)  = hl0 - (r+1)*hls    F(r, 0)  = H(r, 0) - fo
 //   H(-1, 0) = 0
-// buf[c] (c = 1..cols) carries (H, E') of the last row of a stripe to the next
+// buf[c] (c = 1..cols) carries (H, E) of the last row of a stripe to the next
 // stripe, and in MODE_GLOBAL holds the final row on return.
 struct Task {
     const int8_t* rseq;
@@ -83,9 +89,14 @@ struct Best {
     unsigned key;  // (row << 16) | col of the winning cell
 };
 
+// Rows of the shared matrix: 32 codes and a padding row of kPadScore.
+constexpr int kPadRow = 32;
+constexpr int kSmatWords = (kPadRow + 1) * 32;
+constexpr int kPadScore = -32768;
+
 // Per-block constants the device functions read.
 struct Env {
-    const int* smat;     // shared 32x32 matrix over remapped codes
+    const int* smat;     // shared matrix over remapped codes: 32x32, then the padding row
     uint16_t* region;    // this warp's shared region (profile or tiny rows)
     int K;               // number of remapped codes
     int gp1, gp2;        // remapped gapPos1 / gapPos2 (-1 if absent)
@@ -96,12 +107,13 @@ struct Env {
 template <int R>
 struct SweepState {
     int hl[R];  // H(r, c-1)
-    int fp[R];  // F'(r, c-1)
-    int rm[R];  // tracked maximum per row
-    int rc[R];  // its first column
+    int fp[R];  // F(r, c)
     int diag;   // H of the row above the lane's first row, column c-1
-    int hout, eout, thr;
-    int ch, ce, nh, ne;  // boundary chunks: current and next W columns
+    int hout, eout;  // H of the lane's last row, E of the row below it
+    int thr;         // the lane's tracked maximum: columns that reach it are examined
+    int bv;          // the maximum of the lane's rows in this stripe
+    unsigned bk;     // its first cell in row-major order: (row in lane << 16) | column
+    int ch, ce, nh, ne;  // boundary chunks (H above, E of the stripe's first row): current and next W columns
 };
 
 // Residue load. NC: through the read-only data path (codes written before the
@@ -114,27 +126,29 @@ __device__ __forceinline__ int ldres(const int8_t* p) {
         return (int)*p;
 }
 
-__device__ __forceinline__ void unpack2(unsigned w, int& lo, int& hi) {
-    lo = (int)(int16_t)(w & 0xffffu);
-    hi = ((int)w) >> 16;
-}
-
-// The R int16 scores of one (code, lane) profile entry: one 16-byte (R == 8)
-// or 8-byte (R == 4) shared load.
+// The R int16 scores of one (code, lane) profile entry, two per word: one
+// 16-byte (R == 8) or 8-byte (R == 4) shared load.
 template <int R>
-__device__ __forceinline__ void load_scores(const uint16_t* p, int (&s)[R]) {
+__device__ __forceinline__ void load_scores(const uint16_t* p, int (&w)[R / 2]) {
     static_assert(R == 8 || R == 4, "profile entries hold 4 or 8 rows");
     if constexpr (R == 8) {
-        const uint4 w = *reinterpret_cast<const uint4*>(p);
-        unpack2(w.x, s[0], s[1]);
-        unpack2(w.y, s[2], s[3]);
-        unpack2(w.z, s[4], s[5]);
-        unpack2(w.w, s[6], s[7]);
+        const int4 v = *reinterpret_cast<const int4*>(p);
+        w[0] = v.x;
+        w[1] = v.y;
+        w[2] = v.z;
+        w[3] = v.w;
     } else {
-        const uint2 w = *reinterpret_cast<const uint2*>(p);
-        unpack2(w.x, s[0], s[1]);
-        unpack2(w.y, s[2], s[3]);
+        const int2 v = *reinterpret_cast<const int2*>(p);
+        w[0] = v.x;
+        w[1] = v.y;
     }
+}
+
+// d + one of the two int16 scores of w, in one instruction: the dot product
+// of w's halves with (1, 0) or (0, 1).
+template <bool HI>
+__device__ __forceinline__ int add_score(int w, int d) {
+    return __dp2a_lo(w, HI ? 0x0100 : 0x0001, d);
 }
 
 __device__ __forceinline__ unsigned pack2(int lo, int hi) {
@@ -231,120 +245,245 @@ struct StripeIO {
     int own_slot;   // progress word of this warp
 };
 
+// E of a task's first row, given H of the row above it.
+__device__ __forceinline__ int first_row_e(const Task& T, int h, int ge, int goe) {
+    return max(h - T.eo - ge, h - goe);
+}
+
+// Whether the padding rows of the sweeps are sound for these penalties; the
+// others (negative ones, or extensions beyond the padding score) take GEN.
+constexpr int kMaxPaddedOpen = 1 << 27;
+__host__ __device__ inline bool padding_sound(int go, int ge) {
+    return go >= 0 && go <= kMaxPaddedOpen && ge >= 0 && ge <= -kPadScore - 1;
+}
+
 // The steps of one stripe. Lane sl processes column c = t - sl + 1 at step t.
 // Lane 0 of the segment takes the row above from the chunk registers (W columns
 // per lane-wide load: the previous stripe's last row, or the closed-form top
-// boundary for the first stripe). PARTIAL: some rows of the stripe are past the
-// task's last row; they pass the row above through so the segment's last used
-// lane still emits the last real row. One loop body per (MODE, PARTIAL) keeps
-// the hot code small enough for the instruction cache (unrolling the step loop
-// made it slower for that reason); lanes outside their column range skip the
-// body. The next step's residue is loaded one step ahead from the lane's own
-// pointer, without clamping (the layout's guard bytes make the reads of fill
-// and drain steps safe; those residues are never used).
+// boundary for the first stripe). The next step's residue is loaded one step
+// ahead from the lane's own pointer, without clamping (the layout's guard bytes
+// make the reads of fill and drain steps safe).
+// The first `fill` steps (at least the used lanes less one, even, at most W),
+// in which lanes wait for their first column, test each lane's column range;
+// the steps after them do not: a lane past its last column computes on, from
+// residues and boundary values that nothing else reads, and only its stores
+// and its tracked maximum are held to the range. Those steps run two per
+// iteration and a chunk (W of them) per turn of the outer loop. The sweeps are
+// bound by issue slots and the ALU pipe together (40 instructions per 8 cells
+// are the cells', 24 of them on that pipe), so the rest of the step counts: with
+// a range test and a chunk test in every step a 1523-residue protein pair took
+// 3.89 M warp instructions and 200 x 1523 89.0 ms, this way 3.16 M and 80.8 ms
+// (110.4 ms before the cells' own change). Four steps per iteration overflow
+// the instruction cache.
+// The maximum is tracked per lane on the step's maximum over the lane's rows;
+// only when it reaches the lane's own maximum is its row looked up.
+// GEN: gap penalties outside the range the padding rows are sound for
+// (padding_sound): rows of the stripe past the task's last row pass the row
+// above through, two selects per cell, so the segment's last used lane still
+// emits the last real row.
 // MW: the stripe is one of a sweep shared by several warps (MwSync): before a
 // chunk of the row above is loaded the predecessor's progress is awaited, and
 // the writer publishes its progress every W columns and at the last one.
-template <int R, int W, int MODE, bool PARTIAL, bool NC, bool MW = false>
-__device__ __forceinline__ void run_stripe(int nsteps, bool first, const Task& T, SweepState<R>& S, int sl,
+template <int R, int W, int MODE, bool GEN, bool NC, bool MW = false>
+__device__ __forceinline__ void run_stripe(int nsteps, int fill, bool first, const Task& T, SweepState<R>& S, int sl,
                                            int nvalid, bool writer, int ge, int goe, int thresh,
                                            const uint16_t* prof_lane, const StripeIO& io = StripeIO{},
                                            const MwSync* mw = nullptr) {
-    const unsigned ucols = (unsigned)T.cols;
     const int8_t* cp = T.cseq - sl;                 // residue of step t: cp[t]
     int2* wp = (MW ? io.wbuf : T.buf) + 1 - sl;     // boundary-row entry of step t: wp[t]
-    const int2* rb = MW ? io.rbuf : T.buf;
+    const int wend = writer ? T.cols + sl : INT_MIN;  // the writer stores in steps below this
     int bnext = ldres<NC>(cp);
-    for (int t = 0; t < nsteps; ++t) {
+
+    auto step = [&](int t, bool test) {
         int hin = __shfl_up_sync(kFull, S.hout, 1, W);
         int ein = __shfl_up_sync(kFull, S.eout, 1, W);
-        const int idx = t & (W - 1);
-        const int bh = __shfl_sync(kFull, S.ch, idx, W);
-        const int be = __shfl_sync(kFull, S.ce, idx, W);
+        const int bh = __shfl_sync(kFull, S.ch, t, W);
+        const int be = __shfl_sync(kFull, S.ce, t, W);
         if (sl == 0) {
             hin = bh;
             ein = be;
         }
-        if (idx == W - 1) {
-            S.ch = S.nh;
-            S.ce = S.ne;
-            const int col = (t / W + 2) * W + 1 + sl;
-            if (first) {
-                S.nh = T.ht0 - col * T.hts;
-                S.ne = S.nh - T.eo + goe;
-            } else {
-                if constexpr (MW) {
-                    const int cfirst = (t / W + 2) * W + 1;
-                    if (cfirst <= T.cols)
-                        mw_wait(*mw, io.pred_slot, mw_word(*mw, io.stripe - 1, min(T.cols, cfirst + W - 1)));
-                }
-                if (col <= T.cols) {
-                    const int2 v = rb[col];
-                    S.nh = v.x;
-                    S.ne = v.y;
-                }
-            }
-        }
         const int b = bnext;
         bnext = ldres<NC>(cp + t + 1);
-        if ((unsigned)(t - sl) < ucols) {
-            int sc[R];
-            load_scores<R>(prof_lane + b * (32 * R), sc);
-            int hup = hin, eup = ein, d = S.diag;
-            int hs[R];
+        if (test && (unsigned)(t - sl) >= (unsigned)T.cols) return;
+        int w[R / 2];
+        load_scores<R>(prof_lane + b * (32 * R), w);
+        int e = ein, d = S.diag, hup = hin, elast = ein;
+        int hs[R];
 #pragma unroll
-            for (int k = 0; k < R; ++k) {
-                int e = __viaddmax_s32(eup, -ge, hup);
-                const int f = __viaddmax_s32(S.fp[k], -ge, S.hl[k]);
-                const int mx = max(e, f);
-                int h;
-                if (MODE == MODE_LOCAL_FWD)
-                    h = __viaddmax_s32_relu(mx, -goe, d + sc[k]);
-                else
-                    h = __viaddmax_s32(mx, -goe, d + sc[k]);
-                if (PARTIAL) {
-                    const bool v = k < nvalid;
-                    h = v ? h : hup;
-                    e = v ? e : eup;
-                }
-                d = S.hl[k];
-                S.hl[k] = h;
-                S.fp[k] = f;
-                hup = h;
-                eup = e;
-                hs[k] = h;
+        for (int k = 0; k < R; ++k) {
+            const int diag = (k & 1) ? add_score<true>(w[k / 2], d) : add_score<false>(w[k / 2], d);
+            int h = MODE == MODE_LOCAL_FWD ? __vimax3_s32_relu(e, S.fp[k], diag) : __vimax3_s32(e, S.fp[k], diag);
+            const int g = h - goe;
+            d = S.hl[k];
+            S.fp[k] = __viaddmax_s32(S.fp[k], -ge, g);
+            if (GEN) {
+                const bool v = k < nvalid;
+                const int en = __viaddmax_s32(e, -ge, g);
+                elast = v ? e : elast;
+                e = v ? en : e;
+                h = v ? h : hup;
+            } else {
+                elast = e;
+                e = __viaddmax_s32(e, -ge, g);
             }
-            S.hout = hup;
-            S.eout = eup;
-            S.diag = hin;
-            if (MODE != MODE_GLOBAL) {
-                int sm = hs[0];
+            S.hl[k] = h;
+            hup = h;
+            hs[k] = h;
+        }
+        S.hout = hup;
+        S.eout = e;
+        S.diag = hin;
+        if (MODE != MODE_GLOBAL) {
+            int sm = hs[0];
 #pragma unroll
-                for (int k = 1; k + 1 < R; k += 2) sm = __vimax3_s32(sm, hs[k], hs[k + 1]);
-                if ((R & 1) == 0) sm = max(sm, hs[R - 1]);
+            for (int k = 1; k + 1 < R; k += 2) sm = __vimax3_s32(sm, hs[k], hs[k + 1]);
+            if ((R & 1) == 0) sm = max(sm, hs[R - 1]);
+            if (sm >= S.thr && t - sl < T.cols) {
+                // First row holding the maximum (of min(H, thresh) in the reverse sweep).
                 if (MODE == MODE_LOCAL_REV) sm = min(sm, thresh);
-                if (sm >= S.thr) {
-                    const int c = t - sl + 1;
+                unsigned kk = R - 1;
 #pragma unroll
-                    for (int k = 0; k < R; ++k) {
-                        const int hv = (MODE == MODE_LOCAL_REV) ? min(hs[k], thresh) : hs[k];
-                        if (hv > S.rm[k]) {
-                            S.rm[k] = hv;
-                            S.rc[k] = c;
-                        }
-                    }
-                    S.thr = sm;
-                }
-            }
-            if (writer) {
-                wp[t] = make_int2(hup, eup);
-                if constexpr (MW) {
-                    const int c = t - sl + 1;
-                    if ((c & (W - 1)) == 0 || c == T.cols) mw_publish(*mw, io.own_slot, io.stripe, c);
-                }
+                for (int k = R - 2; k >= 0; --k) kk = hs[k] >= sm ? k : kk;
+                const unsigned key = (kk << 16) | (unsigned)(t - sl + 1);
+                S.bk = sm > S.bv ? key : min(S.bk, key);
+                S.bv = S.thr = sm;
             }
         }
+        if (t < wend) {
+            wp[t] = make_int2(hup, elast);
+            if constexpr (MW) {
+                const int c = t - sl + 1;
+                if ((c & (W - 1)) == 0 || c == T.cols) mw_publish(*mw, io.own_slot, io.stripe, c);
+            }
+        }
+    };
+    // After the last step of a chunk (t: the step after it).
+    auto next_chunk = [&](int t) {
+        S.ch = S.nh;
+        S.ce = S.ne;
+        const int cfirst = t + W + 1, col = cfirst + sl;
+        if (first) {
+            S.nh = T.ht0 - col * T.hts;
+            S.ne = first_row_e(T, S.nh, ge, goe);
+        } else {
+            if constexpr (MW) {
+                if (cfirst <= T.cols)
+                    mw_wait(*mw, io.pred_slot, mw_word(*mw, io.stripe - 1, min(T.cols, cfirst + W - 1)));
+            }
+            if (col <= T.cols) {
+                const int2 v = (MW ? io.rbuf : T.buf)[col];
+                S.nh = v.x;
+                S.ne = __viaddmax_s32(v.y, -ge, v.x - goe);
+            }
+        }
+    };
+
+    int t = 0;
+    for (; t < fill; ++t) step(t, true);
+    if (t == W) next_chunk(t);
+    while (t < nsteps) {
+        const int tend = min(nsteps, (t | (W - 1)) + 1);
+        for (; t < tend; t += 2) {  // fill and W are even: at most one step past nsteps
+            step(t, false);
+            step(t + 1, false);
+        }
+        if (t < nsteps) next_chunk(t);
     }
+}
+
+// Checked steps of a stripe whose segments use at most `lused` lanes.
+__device__ __forceinline__ int fill_steps(int lused) { return lused & ~1; }
+
+// A lane's share of a stripe: rows lrow0 .. lrow0 + R - 1 of the task. Rows
+// outside [0, rows) are padding, with kPadScore against every residue (GEN:
+// rows past the end pass the row above through instead).
+// MODE_GLOBAL pads above the first row (pad < R rows, all in the first lane), so
+// that the last row is always the last register of the last used lane. A
+// padding row r < 0 reproduces the top boundary in every column: its F starts
+// at H(-1, 1) and loses ge per column as the boundary does (hts == ge), and E
+// and the diagonal term stay below it as long as gapOpen >= 0 and 0 <= ge <=
+// -kPadScore. The local modes pad below the last row: such a row's H never
+// exceeds one already seen above or to the left of it (gapOpen, ge >= 0), so
+// it is never the first maximum.
+template <int R, int MODE, bool GEN, bool NC>
+__device__ __forceinline__ void stripe_begin(const Task& T, SweepState<R>& S, int lrow0, int gbest, int ge, int goe,
+                                             int thresh, const Env& X, int lane) {
+    int a[R];
+#pragma unroll
+    for (int k = 0; k < R; ++k) {
+        const int r = lrow0 + k;
+        a[k] = (r >= 0 && r < T.rows) ? ldres<NC>(T.rseq + r) : (GEN ? 0 : kPadRow);
+    }
+    __syncwarp();  // previous users of the shared region are done
+    build_profile<R>(X.region, X.smat, a, lane, X.K);
+    __syncwarp();  // previous stripe's buf writes visible to the whole segment
+    constexpr int kLow = -(1 << 29);  // below every boundary value
+#pragma unroll
+    for (int k = 0; k < R; ++k) {
+        const int r = lrow0 + k;
+        S.hl[k] = T.hl0 - (r + 1) * T.hls;
+        S.fp[k] = max(S.hl[k] - T.fo - ge, S.hl[k] - goe);
+        if (MODE == MODE_GLOBAL && !GEN && r < 0) {
+            S.hl[k] = r == -1 ? 0 : kLow;  // H(-1, 0), else never taken
+            S.fp[k] = T.ht0 - T.hts;       // H(-1, 1)
+        }
+    }
+    S.diag = lrow0 == 0 ? 0 : T.hl0 - lrow0 * T.hls;
+    if (MODE == MODE_GLOBAL && !GEN && lrow0 < 0) S.diag = kLow;
+    S.hout = 0;
+    S.eout = 0;
+    S.bv = gbest;
+    S.bk = 0xffffffffu;
+    // The reverse sweep ends in the stripe whose H first reaches thresh, and
+    // with gap penalties >= 0 some cell does (the forward optimum read
+    // backwards), so nothing below thresh need be tracked.
+    S.thr = (MODE == MODE_LOCAL_REV && !GEN) ? thresh : gbest + 1;
+    if (lrow0 >= T.rows) S.thr = INT_MAX;  // padding only
+}
+
+// Boundary chunk registers at the start of a stripe, from the closed form or
+// from the previous stripe's last row.
+template <int R, int W>
+__device__ __forceinline__ void stripe_chunks(const Task& T, SweepState<R>& S, const int2* rb, bool first, int sl,
+                                              int ge, int goe) {
+    if (first) {
+        S.ch = T.ht0 - (1 + sl) * T.hts;
+        S.ce = first_row_e(T, S.ch, ge, goe);
+        S.nh = T.ht0 - (W + 1 + sl) * T.hts;
+        S.ne = first_row_e(T, S.nh, ge, goe);
+        return;
+    }
+    S.ch = S.ce = S.nh = S.ne = 0;
+    if (1 + sl <= T.cols) {
+        const int2 v = rb[1 + sl];
+        S.ch = v.x;
+        S.ce = __viaddmax_s32(v.y, -ge, v.x - goe);
+    }
+    if (W + 1 + sl <= T.cols) {
+        const int2 v = rb[W + 1 + sl];
+        S.nh = v.x;
+        S.ne = __viaddmax_s32(v.y, -ge, v.x - goe);
+    }
+}
+
+// Best of the stripe over the warp, folded into `best`.
+template <int R>
+__device__ __forceinline__ int stripe_best(const SweepState<R>& S, int lrow0, int gbest, Best& best) {
+    const unsigned lk = S.bv > gbest ? S.bk + ((unsigned)lrow0 << 16) : 0xffffffffu;
+    const int wv = __reduce_max_sync(kFull, S.bv);
+    const unsigned wk = __reduce_min_sync(kFull, S.bv == wv ? lk : 0xffffffffu);
+    if (wv > best.val) {  // later stripes hold later rows: strict keeps the first
+        best.val = wv;
+        best.key = wk;
+    }
+    return wv;
+}
+
+// Padding rows above the first row of a MODE_GLOBAL task.
+template <int R, int MODE, bool GEN>
+__device__ __forceinline__ int top_padding(int rows) {
+    return (MODE == MODE_GLOBAL && !GEN && rows > 0) ? (R - rows % R) % R : 0;
 }
 
 // The wavefront sweep. W = lanes per segment (32: one task per warp, 16: two
@@ -353,16 +492,16 @@ __device__ __forceinline__ void run_stripe(int nsteps, bool first, const Task& T
 // strict `hh > maxScore`); MODE_LOCAL_REV tracks the first cell, in the sweep's
 // row-major order, of the maximum of min(H, thresh) (reversePass's strict
 // `hh > cost` and its break at cost >= maxScore) and stops after the first
-// stripe that reached thresh. Tracking runs on the per-step maximum of the
-// lane's rows; only when it reaches the lane's running maximum are the rows
-// examined one by one.
-template <int R, int W, int MODE, bool NC = true>
+// stripe that reached thresh.
+template <int R, int W, int MODE, bool GEN, bool NC = true>
 __device__ void sweep(const Task& T, int go, int ge, int thresh, const Env& X, Best& best) {
     const int lane = threadIdx.x & 31;
     const int sl = lane & (W - 1);
     const int goe = go + ge;
     constexpr int RPS = W * R;
-    const int nstr = T.rows > 0 ? (T.rows + RPS - 1) / RPS : 0;
+    const int pad = top_padding<R, MODE, GEN>(T.rows);
+    const int prows = T.rows + pad;
+    const int nstr = prows > 0 ? (prows + RPS - 1) / RPS : 0;
     const int nstr_max = __reduce_max_sync(kFull, nstr);
     const uint16_t* prof_lane = X.region + lane * R;
     best.val = 0;
@@ -370,77 +509,21 @@ __device__ void sweep(const Task& T, int go, int ge, int thresh, const Env& X, B
     SweepState<R> S;
 
     for (int s = 0; s < nstr_max; ++s) {
-        const int srow0 = s * RPS;
-        const int seg_rows = min(T.rows - srow0, RPS);
-        const int lrow0 = srow0 + sl * R;
+        const int seg_rows = min(prows - s * RPS, RPS);
+        const int lrow0 = s * RPS + sl * R - pad;
         const int nvalid = max(0, min(R, T.rows - lrow0));
         const int lused = seg_rows > 0 ? (seg_rows + R - 1) / R : 0;
         const int nsteps = (seg_rows > 0 && T.cols > 0) ? T.cols + lused - 1 : 0;
         const int nsteps_max = __reduce_max_sync(kFull, nsteps);
         const bool last = (s == nstr - 1);
         const bool writer = (sl == lused - 1) && (MODE == MODE_GLOBAL || !last);
-        const bool full = __all_sync(kFull, seg_rows == RPS);
-
-        int a[R];
-#pragma unroll
-        for (int k = 0; k < R; ++k) a[k] = (k < nvalid) ? ldres<NC>(T.rseq + lrow0 + k) : 0;
-        __syncwarp();  // previous users of the shared region are done
-        build_profile<R>(X.region, X.smat, a, lane, X.K);
-        __syncwarp();  // previous stripe's buf writes visible to the whole segment
-
         const int gbest = best.val;
-#pragma unroll
-        for (int k = 0; k < R; ++k) {
-            S.hl[k] = T.hl0 - (lrow0 + k + 1) * T.hls;
-            S.fp[k] = S.hl[k] - T.fo + goe;
-            S.rm[k] = gbest;
-            S.rc[k] = 0;
-        }
-        S.diag = (lrow0 == 0) ? 0 : T.hl0 - lrow0 * T.hls;
-        S.hout = 0;
-        S.eout = 0;
-        S.thr = gbest + 1;
-        const bool first = (s == 0);
-        if (first) {
-            S.ch = T.ht0 - (1 + sl) * T.hts;
-            S.ce = S.ch - T.eo + goe;
-            S.nh = T.ht0 - (W + 1 + sl) * T.hts;
-            S.ne = S.nh - T.eo + goe;
-        } else {
-            S.ch = S.ce = S.nh = S.ne = 0;
-            if (1 + sl <= T.cols) {
-                const int2 v = T.buf[1 + sl];
-                S.ch = v.x;
-                S.ce = v.y;
-            }
-            if (W + 1 + sl <= T.cols) {
-                const int2 v = T.buf[W + 1 + sl];
-                S.nh = v.x;
-                S.ne = v.y;
-            }
-        }
-        if (full)
-            run_stripe<R, W, MODE, false, NC>(nsteps_max, first, T, S, sl, nvalid, writer, ge, goe, thresh, prof_lane);
-        else
-            run_stripe<R, W, MODE, true, NC>(nsteps_max, first, T, S, sl, nvalid, writer, ge, goe, thresh, prof_lane);
-
+        stripe_begin<R, MODE, GEN, NC>(T, S, lrow0, gbest, ge, goe, thresh, X, lane);
+        stripe_chunks<R, W>(T, S, T.buf, s == 0, sl, ge, goe);
+        run_stripe<R, W, MODE, GEN, NC>(nsteps_max, fill_steps(__reduce_max_sync(kFull, lused)), s == 0, T, S, sl, nvalid,
+                                        writer, ge, goe, thresh, prof_lane);
         if (MODE != MODE_GLOBAL) {
-            // Earliest row of this lane holding the lane's maximum (rows ascend with k).
-            int lv = gbest;
-            unsigned lk = 0xffffffffu;
-#pragma unroll
-            for (int k = 0; k < R; ++k) {
-                if (k < nvalid && S.rm[k] > lv) {
-                    lv = S.rm[k];
-                    lk = ((unsigned)(lrow0 + k) << 16) | (unsigned)S.rc[k];
-                }
-            }
-            const int wv = __reduce_max_sync(kFull, lv);
-            const unsigned wk = __reduce_min_sync(kFull, lv == wv ? lk : 0xffffffffu);
-            if (wv > best.val) {  // later stripes hold later rows: strict keeps the first
-                best.val = wv;
-                best.key = wk;
-            }
+            stripe_best<R>(S, lrow0, gbest, best);
             if (MODE == MODE_LOCAL_REV && best.val >= thresh) break;
         }
     }
@@ -458,10 +541,11 @@ __device__ void sweep(const Task& T, int go, int ge, int thresh, const Env& X, B
 // thresh; stripes above it are skipped (their progress is published as
 // complete so no successor waits), which leaves the result of the lowest
 // such stripe, reversePass's break cell. MODE_GLOBAL: the final row is in the
-// buffer of rank (stripes - 1) % nw (see mw_last_rank).
+// buffer of rank (stripes - 1) % nw (see mw_last_rank); padding rows above the
+// first do not change the number of stripes.
 __host__ __device__ inline int mw_stripes(int rows, int R) { return rows > 0 ? (rows + 32 * R - 1) / (32 * R) : 0; }
 
-template <int R, int MODE, bool NC = true>
+template <int R, int MODE, bool GEN, bool NC = true>
 __device__ void sweep_mw(const Task& T, int go, int ge, int thresh, const Env& X, Best& best, int2* bufs,
                          size_t stride, int slot0, int rank, int nw, const MwSync& mw, volatile int* stop) {
     constexpr int W = 32;
@@ -469,6 +553,8 @@ __device__ void sweep_mw(const Task& T, int go, int ge, int thresh, const Env& X
     const int sl = lane;
     const int goe = go + ge;
     constexpr int RPS = W * R;
+    const int pad = top_padding<R, MODE, GEN>(T.rows);
+    const int prows = T.rows + pad;
     const int nstr = mw_stripes(T.rows, R);
     const uint16_t* prof_lane = X.region + lane * R;
     best.val = 0;
@@ -487,78 +573,21 @@ __device__ void sweep_mw(const Task& T, int go, int ge, int thresh, const Env& X
             if (lane == 0) mw_publish(mw, io.own_slot, s, T.cols);
             continue;
         }
-        const int srow0 = s * RPS;
-        const int seg_rows = min(T.rows - srow0, RPS);
-        const int lrow0 = srow0 + sl * R;
+        const int seg_rows = min(prows - s * RPS, RPS);
+        const int lrow0 = s * RPS + sl * R - pad;
         const int nvalid = max(0, min(R, T.rows - lrow0));
         const int lused = (seg_rows + R - 1) / R;
-        const int nsteps = T.cols > 0 ? T.cols + lused - 1 : 0;
+        const int nsteps = T.cols + lused - 1;
         const bool last = (s == nstr - 1);
         const bool writer = (sl == lused - 1) && (MODE == MODE_GLOBAL || !last);
-        const bool full = seg_rows == RPS;
-
-        int a[R];
-#pragma unroll
-        for (int k = 0; k < R; ++k) a[k] = (k < nvalid) ? ldres<NC>(T.rseq + lrow0 + k) : 0;
-        __syncwarp();
-        build_profile<R>(X.region, X.smat, a, lane, X.K);
-        __syncwarp();
-
         const int gbest = best.val;
-#pragma unroll
-        for (int k = 0; k < R; ++k) {
-            S.hl[k] = T.hl0 - (lrow0 + k + 1) * T.hls;
-            S.fp[k] = S.hl[k] - T.fo + goe;
-            S.rm[k] = gbest;
-            S.rc[k] = 0;
-        }
-        S.diag = (lrow0 == 0) ? 0 : T.hl0 - lrow0 * T.hls;
-        S.hout = 0;
-        S.eout = 0;
-        S.thr = gbest + 1;
-        const bool first = (s == 0);
-        if (first) {
-            S.ch = T.ht0 - (1 + sl) * T.hts;
-            S.ce = S.ch - T.eo + goe;
-            S.nh = T.ht0 - (W + 1 + sl) * T.hts;
-            S.ne = S.nh - T.eo + goe;
-        } else {
-            mw_wait(mw, io.pred_slot, mw_word(mw, s - 1, min(T.cols, 2 * W)));
-            S.ch = S.ce = S.nh = S.ne = 0;
-            if (1 + sl <= T.cols) {
-                const int2 v = io.rbuf[1 + sl];
-                S.ch = v.x;
-                S.ce = v.y;
-            }
-            if (W + 1 + sl <= T.cols) {
-                const int2 v = io.rbuf[W + 1 + sl];
-                S.nh = v.x;
-                S.ne = v.y;
-            }
-        }
-        if (full)
-            run_stripe<R, W, MODE, false, NC, true>(nsteps, first, T, S, sl, nvalid, writer, ge, goe, thresh,
-                                                    prof_lane, io, &mw);
-        else
-            run_stripe<R, W, MODE, true, NC, true>(nsteps, first, T, S, sl, nvalid, writer, ge, goe, thresh,
-                                                   prof_lane, io, &mw);
-
+        stripe_begin<R, MODE, GEN, NC>(T, S, lrow0, gbest, ge, goe, thresh, X, lane);
+        if (s > 0) mw_wait(mw, io.pred_slot, mw_word(mw, s - 1, min(T.cols, 2 * W)));
+        stripe_chunks<R, W>(T, S, io.rbuf, s == 0, sl, ge, goe);
+        run_stripe<R, W, MODE, GEN, NC, true>(nsteps, fill_steps(lused), s == 0, T, S, sl, nvalid, writer, ge, goe,
+                                              thresh, prof_lane, io, &mw);
         if (MODE != MODE_GLOBAL) {
-            int lv = gbest;
-            unsigned lk = 0xffffffffu;
-#pragma unroll
-            for (int k = 0; k < R; ++k) {
-                if (k < nvalid && S.rm[k] > lv) {
-                    lv = S.rm[k];
-                    lk = ((unsigned)(lrow0 + k) << 16) | (unsigned)S.rc[k];
-                }
-            }
-            const int wv = __reduce_max_sync(kFull, lv);
-            const unsigned wk = __reduce_min_sync(kFull, lv == wv ? lk : 0xffffffffu);
-            if (wv > best.val) {
-                best.val = wv;
-                best.key = wk;
-            }
+            const int wv = stripe_best<R>(S, lrow0, gbest, best);
             if (MODE == MODE_LOCAL_REV && wv >= thresh && lane == 0) atomicMin((int*)stop, s);
         }
     }
@@ -746,8 +775,8 @@ __device__ __forceinline__ bool share_push(const FrameShare& fs, int4 f) {
 }
 
 // Midpoint scans of a Myers-Miller frame (FullPairwiseAlign.cpp:570-593), by
-// one warp. fwd[j] holds (HH, DD + goe) of row midi from the forward half,
-// rev[N - j] holds (RR, SS + goe) of the same row from the reverse half (j =
+// one warp. fwd[j] holds (HH, DD) of row midi from the forward half,
+// rev[N - j] holds (RR, SS) of the same row from the reverse half (j =
 // 1..N and 0..N-1; the other ends are closed-form). Scan 1 keeps the first j
 // reaching the maximum of HH+RR, replaced by the last tied j with HH!=DD &&
 // RR==SS; scan 2 switches to a type-2 midpoint at the largest j whose
@@ -755,7 +784,6 @@ __device__ __forceinline__ bool share_push(const FrameShare& fs, int4 f) {
 __device__ __forceinline__ void midpoint_scan(const int2* fwd, const int2* rev, int M, int N, int midi, int tb, int te,
                                               int go, int ge, int& midh, int& midj, bool& type2) {
     const int lane = threadIdx.x & 31;
-    const int goe = go + ge;
     const int HH0 = -tb - midi * ge;        // HH[0] = DD[0]
     const int RRN = -te - (M - midi) * ge;  // RR[N] = SS[N]
     int b1 = INT_MIN, j1 = 0x7fffffff, jc = -1, b2 = INT_MIN, j2 = -1;
@@ -766,14 +794,14 @@ __device__ __forceinline__ void midpoint_scan(const int2* fwd, const int2* rev, 
         } else {
             const int2 v = fwd[j];
             hh = v.x;
-            dd = v.y - goe;
+            dd = v.y;
         }
         if (j == N) {
             rr = ss = RRN;
         } else {
             const int2 v = rev[N - j];
             rr = v.x;
-            ss = v.y - goe;
+            ss = v.y;
         }
         const int v1 = hh + rr;
         const bool cond = (hh != dd) && (rr == ss);
@@ -820,7 +848,7 @@ __device__ __forceinline__ void midpoint_scan(const int2* fwd, const int2* rev, 
 // whole pair's frame has neither). SHARE: after each division the right child,
 // if it has at least fs->min_rows rows, goes to the CTA's shared stack (when
 // it has room) for any warp of the CTA to take, instead of this warp's own.
-template <int RS, bool NC = true, bool SHARE = false>
+template <int RS, bool GEN, bool NC = true, bool SHARE = false>
 static __device__ void mm_align(const int8_t* s1, const int8_t* s1r, int n, const int8_t* s2, const int8_t* s2r, int m,
                                 int A0, int B0, int M0, int N0, int go, int ge, int2* bufA, int2* bufB, const Env& X,
                                 int& mm_score, int& n_ident, int& n_match, long long& cells,
@@ -948,7 +976,7 @@ static __device__ void mm_align(const int8_t* s1, const int8_t* s1r, int n, cons
         t.hls = ge;
         t.fo = go;
         Best unused;
-        sweep<RS, 16, MODE_GLOBAL, NC>(t, go, ge, 0, X, unused);
+        sweep<RS, 16, MODE_GLOBAL, GEN, NC>(t, go, ge, 0, X, unused);
 
         int midh, midj;
         bool type2;
@@ -1013,6 +1041,11 @@ static __device__ void mm_align(const int8_t* s1, const int8_t* s1r, int n, cons
     cells = ncell;
 }
 
+// The block's shared copy of the matrix: 32x32 entries, then the padding row.
+__device__ __forceinline__ void stage_matrix(int* smat, const int32_t* matrix) {
+    for (int i = threadIdx.x; i < kSmatWords; i += blockDim.x) smat[i] = i < 32 * 32 ? matrix[i] : kPadScore;
+}
+
 struct PairArgs {
     const int8_t* codes;
     const int64_t* offs;
@@ -1034,6 +1067,7 @@ struct PairArgs {
     int gp1, gp2;  // remapped gap codes
     int K;         // remapped alphabet size
     int tiny_m, tiny_n;
+    int general;  // host: gap penalties outside padding_sound somewhere, take the GEN kernels
 };
 
 // forwardPass + reversePass + diff + distance for one pair, given its 0-based
@@ -1046,7 +1080,7 @@ struct PairArgs {
 // next 16-byte boundary (cwgpu_layout.h), and kGuard readable bytes surround both.
 __device__ __forceinline__ const int8_t* rev_of(const int8_t* s, int len) { return s + rev_offset(len); }
 
-template <int RS = kR, bool NC = true>
+template <int RS, bool GEN, bool NC = true>
 static __device__ float align_one(const int8_t* s1, int n, const int8_t* s2, int m, int len1, int len2, int go, int ge,
                            int2* bufA, int2* bufB, const Env& X, cwgpu_pair_stats& st, unsigned long long (&acc)[3]) {
     const int8_t* s1r = rev_of(s1, n);
@@ -1067,7 +1101,7 @@ static __device__ float align_one(const int8_t* s1, int n, const int8_t* s2, int
     t.fo = go;
     t.buf = bufA;
     Best fb;
-    sweep<RS, 32, MODE_LOCAL_FWD, NC>(t, go, ge, 0, X, fb);
+    sweep<RS, 32, MODE_LOCAL_FWD, GEN, NC>(t, go, ge, 0, X, fb);
     const int max_score = fb.val;
     const int se1 = max_score > 0 ? (int)(fb.key >> 16) + 1 : 0;
     const int se2 = max_score > 0 ? (int)(fb.key & 0xffffu) : 0;
@@ -1088,7 +1122,7 @@ static __device__ float align_one(const int8_t* s1, int n, const int8_t* s2, int
         r.fo = 0;
         r.buf = bufA;
         Best rb;
-        sweep<RS, 32, MODE_LOCAL_REV, NC>(r, go, ge, max_score, X, rb);
+        sweep<RS, 32, MODE_LOCAL_REV, GEN, NC>(r, go, ge, max_score, X, rb);
         if (rb.val > 0) {
             sb1 = se1 - (int)(rb.key >> 16);
             sb2 = se2 - (int)(rb.key & 0xffffu) + 1;
@@ -1104,7 +1138,7 @@ static __device__ float align_one(const int8_t* s1, int n, const int8_t* s2, int
     // diff + tracePath
     int mm = 0, ident = 0, matches = 0;
     long long dcells = 0;
-    mm_align<RS, NC>(s1, s1r, n, s2, s2r, m, sb1 - 1, sb2 - 1, se1 - sb1 + 1, se2 - sb2 + 1, go, ge, bufA, bufB, X, mm,
+    mm_align<RS, GEN, NC>(s1, s1r, n, s2, s2r, m, sb1 - 1, sb2 - 1, se1 - sb1 + 1, se2 - sb2 + 1, go, ge, bufA, bufB, X, mm,
                  ident, matches, dcells);
     acc[2] += (unsigned long long)dcells;
 
@@ -1126,14 +1160,14 @@ static __device__ float align_one(const int8_t* s1, int n, const int8_t* s2, int
 }
 
 // Aligns pair q: FullPairwiseAlign.cpp:112-183 for one (si, sj).
-template <int RS = kR>
+template <int RS, bool GEN>
 static __device__ void align_pair(const PairArgs& g, long long q, const Env& X, int2* bufA, int2* bufB,
                            unsigned long long (&acc)[3]) {
     const int lane = threadIdx.x & 31;
     const int si = g.pairs[2 * q], sj = g.pairs[2 * q + 1];
     const int n = g.lens[si], m = g.lens[sj];
     cwgpu_pair_stats st;
-    const float dist = align_one<RS>(g.codes + g.offs[si], n, g.codes + g.offs[sj], m, g.nres[si], g.nres[sj],
+    const float dist = align_one<RS, GEN>(g.codes + g.offs[si], n, g.codes + g.offs[sj], m, g.nres[si], g.nres[sj],
                                  g.go_table[min(n, m)], g.ge, bufA, bufB, X, st, acc);
     if (lane == 0) {
         g.dist[q] = dist;

@@ -27,6 +27,7 @@
 #include <mutex>
 
 #include "cwgpu.h"
+#include "cwgpu_context.h"
 #include "cwgpu_device.cuh"
 #include "cwgpu_layout.h"
 
@@ -79,6 +80,7 @@ __host__ __device__ inline size_t na_slot_bytes(int max_len) {
 // residue counts len1/len2 of :100-127 are counted here instead of being
 // uploaded. The two sequences are copied into the slot (forward and reversed)
 // and read back from there with plain loads, since the kernel wrote them.
+template <bool GEN>
 __device__ void na_align_pair(const NaArgs& a, long long q, const cwgpu::Env& X, int2* bufA, int2* bufB,
                               int8_t* slot_codes, unsigned long long (&acc)[3]) {
     const int lane = threadIdx.x & 31;
@@ -117,19 +119,21 @@ __device__ void na_align_pair(const NaArgs& a, long long q, const cwgpu::Env& X,
     int8_t* p2 = p1r + cwgpu::rev_offset(n);
     int8_t* p2r = p2 + cwgpu::rev_offset(m);
     __syncwarp();  // the previous pair's reads of the slot are done
-    for (int i = lane; i < n; i += 32) {
-        const int8_t c = s1[i];
+    const int pn = (int)cwgpu::rev_offset(n), pm = (int)cwgpu::rev_offset(m);
+    for (int i = lane; i < pn; i += 32) {
+        const int8_t c = i < n ? s1[i] : (int8_t)0;
         p1[i] = c;
-        p1r[n - 1 - i] = c;
+        p1r[i < n ? n - 1 - i : i] = c;
     }
-    for (int i = lane; i < m; i += 32) {
-        const int8_t c = s2[i];
+    for (int i = lane; i < pm; i += 32) {
+        const int8_t c = i < m ? s2[i] : (int8_t)0;
         p2[i] = c;
-        p2r[m - 1 - i] = c;
+        p2r[i < m ? m - 1 - i : i] = c;
     }
+    for (int i = lane; i < cwgpu::kGuard; i += 32) slot_codes[i] = p2r[pm + i] = 0;  // guards: any valid code
     __syncwarp();  // copies visible to the whole warp
     cwgpu_pair_stats st;
-    const float dist = cwgpu::align_one<cwgpu::kR, false>(p1, n, p2, m, len1, len2, go_table[min(n, m)], a.ge, bufA,
+    const float dist = cwgpu::align_one<cwgpu::kR, GEN, false>(p1, n, p2, m, len1, len2, go_table[min(n, m)], a.ge, bufA,
                                                           bufB, X, st, acc);
     if (lane == 0) {
         a.dist[q] = dist;
@@ -141,8 +145,9 @@ __device__ void na_align_pair(const NaArgs& a, long long q, const cwgpu::Env& X,
 // entries, so an entry outside [-32768, 32767] sets the matrix status word and
 // every block returns before aligning anything (cwgpu_set_matrix makes the same
 // check on the host for the allocating entry points).
+template <bool GEN>
 __global__ void __launch_bounds__(kNaWarpsPerBlock * 32) k_pairwise_noalloc(NaArgs a) {
-    __shared__ int smat[CWGPU_NUMRES * CWGPU_NUMRES];
+    __shared__ int smat[cwgpu::kSmatWords];
     extern __shared__ __align__(16) uint16_t na_region[];
     int bad_entry = 0;
     for (int i = threadIdx.x; i < CWGPU_NUMRES * CWGPU_NUMRES; i += blockDim.x) {
@@ -150,6 +155,7 @@ __global__ void __launch_bounds__(kNaWarpsPerBlock * 32) k_pairwise_noalloc(NaAr
         bad_entry |= (v < -32768 || v > 32767);
         smat[i] = v;
     }
+    if (threadIdx.x < 32) smat[CWGPU_NUMRES * CWGPU_NUMRES + threadIdx.x] = cwgpu::kPadScore;
     if (__syncthreads_or(bad_entry)) {
         if (threadIdx.x == 0) atomicExch(na_status(a.scratch, kNaStatusMatrix), 1);
         return;
@@ -176,7 +182,7 @@ __global__ void __launch_bounds__(kNaWarpsPerBlock * 32) k_pairwise_noalloc(NaAr
         if (lane == 0) k = atomicAdd(ctrl, 1ULL);
         k = __shfl_sync(cwgpu::kFull, k, 0);
         if (k >= (unsigned long long)a.npairs) break;
-        na_align_pair(a, (long long)k, X, bufA, bufB, slot_codes, acc);
+        na_align_pair<GEN>(a, (long long)k, X, bufA, bufB, slot_codes, acc);
     }
     if (lane == 0 && (acc[0] | acc[1] | acc[2])) {
         atomicAdd(ctrl + 1, acc[0]);
@@ -215,12 +221,16 @@ int na_setup(int dev, NaDevice** out) {
         }
         int sms = 0, per_sm = 0;
         e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-        if (e == cudaSuccess)
-            e = cudaFuncSetAttribute(k_pairwise_noalloc, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     (int)(kNaRegionBytes * kNaWarpsPerBlock));
-        if (e == cudaSuccess)
-            e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_pairwise_noalloc, kNaWarpsPerBlock * 32,
-                                                              kNaRegionBytes * kNaWarpsPerBlock);
+        int fit = 0;
+        for (auto* k : {k_pairwise_noalloc<true>, k_pairwise_noalloc<false>}) {
+            if (e == cudaSuccess)
+                e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         (int)(kNaRegionBytes * kNaWarpsPerBlock));
+            if (e == cudaSuccess)
+                e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&fit, k, kNaWarpsPerBlock * 32,
+                                                                  kNaRegionBytes * kNaWarpsPerBlock);
+            per_sm = per_sm ? (fit < per_sm ? fit : per_sm) : fit;
+        }
         if (e != cudaSuccess) {
             fprintf(stderr, "cwgpu_align_pairs_noalloc: set-up failed: %s\n", cudaGetErrorString(e));
             return CWGPU_ERR_CUDA;
@@ -262,6 +272,7 @@ extern "C" int cwgpu_align_pairs_noalloc(const int8_t* d_codes, const int64_t* d
         int32_t unused = 0;
         cwgpu_gap_penalties(params, L, L, &table[L], &unused);
     }
+    const bool general = cwgpu_general_gaps(table, max_len, ge);
 
     const long long slots = (long long)((kNaScratchBytes - kNaRowsOffset) / na_slot_bytes(max_len));
     long long grid = slots / kNaWarpsPerBlock;
@@ -292,7 +303,8 @@ extern "C" int cwgpu_align_pairs_noalloc(const int8_t* d_codes, const int64_t* d
         a.ge = ge;
         a.gp1 = params->gap_pos1;
         a.gp2 = params->gap_pos2;
-        k_pairwise_noalloc<<<(unsigned)grid, kNaWarpsPerBlock * 32, kNaRegionBytes * kNaWarpsPerBlock, s>>>(a);
+        auto* const k = general ? k_pairwise_noalloc<true> : k_pairwise_noalloc<false>;
+        k<<<(unsigned)grid, kNaWarpsPerBlock * 32, kNaRegionBytes * kNaWarpsPerBlock, s>>>(a);
         e = cudaGetLastError();
     }
     int status[3] = {0, 0, 0};

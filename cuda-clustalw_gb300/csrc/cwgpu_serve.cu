@@ -175,6 +175,7 @@ struct cwgpu_server {
     cwgpu_params params;
     int32_t matrix[CWGPU_NUMRES * CWGPU_NUMRES];
     int ge = 0;
+    bool general_gaps = false;  // cwgpu_general_gaps of the penalties up to max_seq_len
     // incremental dense alphabet shared by all jobs of the server
     int K = 0;
     int dense_of[CWGPU_NUMRES];
@@ -467,6 +468,7 @@ int launch_round(cwgpu_server* s, int ri, int64_t nitems) {
         gl.K = K;
         gl.tiny_m = 32;
         gl.tiny_n = cwgpu::kTinyMaxN;
+        gl.general = s->general_gaps;
         cwgpu::PairArgs gs = gl;
         gs.order = gl.order + r.nlong;
         gs.npairs = r.n - r.nlong;
@@ -637,6 +639,7 @@ int cwgpu_server_create(int device, const int32_t* matrix, const cwgpu_params* p
             int32_t ge = 0;
             cwgpu_gap_penalties(params, L, L, &got[(size_t)L], &ge);
         }
+        s->general_gaps = cwgpu_general_gaps(got.data(), opts->max_seq_len, s->ge);
         e = cudaMemcpy(s->d_go, got.data(), sizeof(int32_t) * got.size(), cudaMemcpyHostToDevice);
     }
     // Scratch rows per round: 5 CTAs per SM of each pair kernel (their launch bound).
