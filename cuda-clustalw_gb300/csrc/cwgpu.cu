@@ -56,8 +56,7 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32, 5)
     const int wpb = blockDim.x >> 5;
     const long long slot = (long long)blockIdx.x * wpb + warp;
     cwgpu::Env X;
-    X.smat = smat;
-    X.region = region_all + (size_t)warp * (cwgpu::warp_region_bytes(g.K) / sizeof(uint16_t));
+    X.set_shared(smat, region_all + (size_t)warp * (cwgpu::warp_region_bytes(g.K) / sizeof(uint16_t)));
     X.K = g.K;
     X.gp1 = g.gp1;
     X.gp2 = g.gp2;
@@ -83,6 +82,47 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32, 5)
         atomicAdd(g.cells + 1, acc[1]);
         atomicAdd(g.cells + 2, acc[2]);
     }
+}
+
+// The long-pair kernel: k_pairwise<kR, false> with the path of cwgpu_path.cuh in
+// place of diff()'s sweeps (1000 x 1523 protein family, 200 sequences: 80.8 ->
+// 51.4 ms; DNA 200 x 1002 35.2 -> 23.0).
+__global__ void __launch_bounds__(kWarpsPerBlock * 32, 5)
+    k_pairwise_long(const __grid_constant__ cwgpu::PairArgs g, long long single) {
+    __shared__ int smat[cwgpu::kSmatWords];
+    extern __shared__ __align__(16) uint16_t region_all[];
+    cwgpu::stage_matrix(smat, g.matrix);
+    __syncthreads();
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const long long slot = (long long)blockIdx.x * (blockDim.x >> 5) + warp;
+    cwgpu::Env X;
+    X.set_shared(smat, region_all + (size_t)warp * (cwgpu::warp_region_bytes(g.K) / sizeof(uint16_t)));
+    X.K = g.K;
+    X.gp1 = g.gp1;
+    X.gp2 = g.gp2;
+    X.tiny_m = g.tiny_m;
+    X.tiny_n = g.tiny_n;
+    X.err = g.err;
+    if (single >= 0) {
+        if (slot == 0) cwgpu::align_long(g, single, 0, X);
+        return;
+    }
+    for (;;) {
+        unsigned long long k = 0;
+        if (lane == 0) k = atomicAdd(g.counter, 1ULL);
+        k = __shfl_sync(cwgpu::kFull, k, 0);
+        if (k >= (unsigned long long)g.npairs) break;
+        cwgpu::align_long(g, (long long)g.order[k], slot, X);
+    }
+}
+
+// The kernel for pairs whose rows per lane are RS.
+template <int RS>
+auto pair_kernel(bool general) {
+    if constexpr (RS == cwgpu::kR)
+        return general ? k_pairwise<RS, true> : k_pairwise_long;
+    else
+        return general ? k_pairwise<RS, true> : k_pairwise<RS, false>;
 }
 
 // ---- one CTA per pair: the pair's stripes shared by the warps of a CTA ------
@@ -299,9 +339,11 @@ __device__ void cta_diff(CtaCtl& C, const int8_t* s1, const int8_t* s1r, int n, 
         t.eo = go;
         t.hls = ge;
         t.fo = go;
+        t.corner = 0;
+        t.pad = GEN ? 0 : cwgpu::lane_padding<RS>(t.rows);
         mw.epoch = (++epoch) << 32;
         cwgpu::Best unused;
-        cwgpu::sweep_mw<RS, cwgpu::MODE_GLOBAL, GEN>(t, go, ge, 0, X, unused, bufs, stride, slot0, warp - slot0, gw, mw,
+        cwgpu::sweep_mw<RS, cwgpu::MODE_GLOBAL, GEN>(t, go, ge, 0, 0, X, unused, bufs, stride, slot0, warp - slot0, gw, mw,
                                                 &C.stop);
         __syncthreads();
         if (warp == 0) {
@@ -380,59 +422,42 @@ __device__ void cta_pair(const cwgpu::PairArgs& g, long long q, CtaCtl& C, const
         mw.abort = &C.abort;
         mw.err = g.err;
         mw.limit_ns = ca.limit_ns;
-        // forwardPass
-        cwgpu::Task t;
-        t.rseq = s1;
-        t.cseq = s2;
-        t.rows = n;
-        t.cols = m;
-        t.ht0 = 0;
-        t.hts = 0;
-        t.eo = go;
-        t.hl0 = 0;
-        t.hls = 0;
-        t.fo = go;
-        t.buf = nullptr;
-        mw.epoch = (++epoch) << 32;
-        cwgpu::Best b;
-        cwgpu::sweep_mw<RS, cwgpu::MODE_LOCAL_FWD, GEN>(t, go, ge, 0, X, b, bufs, stride, 0, warp, nw, mw, &C.stop);
-        if (lane == 0) {
-            C.bval[warp] = b.val;
-            C.bkey[warp] = b.key;
-        }
-        __syncthreads();
-        const cwgpu::Best fb = cta_reduce(C, nw);
-        const int max_score = fb.val;
-        const int se1 = max_score > 0 ? (int)(fb.key >> 16) + 1 : 0;
-        const int se2 = max_score > 0 ? (int)(fb.key & 0xffffu) : 0;
-        __syncthreads();
-        if (threadIdx.x == 0) C.stop = INT_MAX;
-        __syncthreads();
-        // reversePass
-        int sb1 = 1, sb2 = 1;
-        if (se1 > 0) {
-            cwgpu::Task r;
-            r.rseq = s1r + (n - se1);
-            r.cseq = s2r + (m - se2);
-            r.rows = se1;
-            r.cols = se2;
-            r.ht0 = -1;
-            r.hts = 0;
-            r.eo = 0;
-            r.hl0 = -1;
-            r.hls = 0;
-            r.fo = 0;
-            r.buf = nullptr;
+        // forwardPass, then reversePass from its end cell.
+        int max_score = 0, se1 = 0, se2 = 0, sb1 = 1, sb2 = 1;
+        cwgpu::Best rb;
+        cwgpu::Task t = cwgpu::local_task(s1, n, s2, m, go, nullptr);
+#pragma unroll 1
+        for (int pass = 0; pass < 2; ++pass) {
+            __syncthreads();
+            if (threadIdx.x == 0) C.stop = INT_MAX;
+            __syncthreads();
             mw.epoch = (++epoch) << 32;
-            cwgpu::sweep_mw<RS, cwgpu::MODE_LOCAL_REV, GEN>(r, go, ge, max_score, X, b, bufs, stride, 0, warp, nw, mw,
-                                                            &C.stop);
+            cwgpu::Best b;
+            if (GEN && pass == 1)
+                cwgpu::sweep_mw<RS, GEN ? cwgpu::MODE_LOCAL_REV : cwgpu::MODE_LOCAL_FWD, GEN>(
+                    t, go, ge, 1, max_score, X, b, bufs, stride, 0, warp, nw, mw, &C.stop);
+            else
+                cwgpu::sweep_mw<RS, cwgpu::MODE_LOCAL_FWD, GEN>(t, go, ge, pass ? max_score + 1 : 1,
+                                                               pass ? max_score + 1 : INT_MAX, X, b, bufs, stride, 0,
+                                                               warp, nw, mw, &C.stop);
             if (lane == 0) {
                 C.bval[warp] = b.val;
                 C.bkey[warp] = b.key;
             }
             __syncthreads();
-            const cwgpu::Best rb = cta_reduce(C, nw);
-            __syncthreads();
+            rb = cta_reduce(C, nw);
+            if (pass == 0) {
+                max_score = rb.val;
+                if (max_score <= 0) break;
+                se1 = (int)(rb.key >> 16) + 1;
+                se2 = (int)(rb.key & 0xffffu);
+                t = cwgpu::reverse_task<RS, GEN>(s1r, n, se1, s2r, m, se2, go, nullptr);
+            } else if (!GEN) {
+                rb.val -= 1;
+            }
+        }
+        __syncthreads();
+        if (max_score > 0) {
             if (rb.val > 0) {
                 sb1 = se1 - (int)(rb.key >> 16);
                 sb2 = se2 - (int)(rb.key & 0xffffu) + 1;
@@ -486,8 +511,7 @@ __global__ void __launch_bounds__(kCtaMaxWarps * 32, 1) k_pairwise_cta(cwgpu::Pa
         C.stop = INT_MAX;
     }
     cwgpu::Env X;
-    X.smat = smat;
-    X.region = region_all + (size_t)warp * (cwgpu::warp_region_bytes(g.K) / sizeof(uint16_t));
+    X.set_shared(smat, region_all + (size_t)warp * (cwgpu::warp_region_bytes(g.K) / sizeof(uint16_t)));
     X.K = g.K;
     X.gp1 = g.gp1;
     X.gp2 = g.gp2;
@@ -705,7 +729,7 @@ size_t block_smem(int K, int warps) { return (size_t)cwgpu::warp_region_bytes(K)
 template <int RS>
 cudaError_t pair_grid(int K, int sm_count, int* grid) {
     int fit = INT_MAX;
-    for (auto* k : {k_pairwise<RS, false>, k_pairwise<RS, true>}) {
+    for (auto* k : {pair_kernel<RS>(false), pair_kernel<RS>(true)}) {
         int per_sm = 0;
         cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                              (int)block_smem(CWGPU_NUMRES, kWarpsPerBlock));
@@ -762,6 +786,34 @@ int cta_grid(cwgpu_context* ctx, int warps, int* grid) {
     return CWGPU_OK;
 }
 
+// Slices for cwgpu_path.cuh: as many as the kernel has warps and the set has
+// ordered pairs, each large enough for the finest row spacing at the longest
+// lengths, or for what kPathBudget leaves it (the kernel then picks a wider
+// spacing, or Myers-Miller for pairs that do not fit).
+constexpr size_t kPathBudget = (size_t)4 << 30;
+
+void path_sizes(int nseqs, int n, int m, int grid, size_t* bytes, long long* slots) {
+    *slots = std::min<long long>((long long)grid * kWarpsPerBlock, (long long)nseqs * nseqs);
+    *bytes = 0;
+    if (*slots < 1 || n < 1) return;
+    size_t want = cwgpu::path_bytes(n, m, 1);
+    want = std::min((want + 255) & ~(size_t)255, (kPathBudget / (size_t)*slots) & ~(size_t)255);
+    *bytes = want;
+}
+
+int ensure_path(cwgpu_context* ctx) {
+    path_sizes(ctx->nseqs, ctx->lmax, ctx->lmax, ctx->grid, &ctx->path_bytes, &ctx->path_slots);
+    const size_t need = ctx->lmax > ctx->short_rows ? ctx->path_bytes * (size_t)ctx->path_slots : 0;
+    if (need > ctx->path_cap) {
+        dfree(ctx->d_path);
+        ctx->path_cap = 0;
+        ctx->generation++;
+        CW_CUDA(ctx, cudaMalloc(&ctx->d_path, need));
+        ctx->path_cap = need;
+    }
+    return CWGPU_OK;
+}
+
 int ensure_scratch(cwgpu_context* ctx) {
     if (ctx->grid == 0 || ctx->grid_K != ctx->K) {
         int rc = persistent_grid<cwgpu::kR>(ctx, &ctx->grid);
@@ -781,7 +833,7 @@ int ensure_scratch(cwgpu_context* ctx) {
         ctx->scratch_bytes = need;
         ctx->generation++;
     }
-    return CWGPU_OK;
+    return ensure_path(ctx);
 }
 
 cwgpu::PairArgs make_args(cwgpu_context* ctx, const int32_t* d_pairs, const int32_t* d_order, int64_t npairs,
@@ -811,6 +863,9 @@ cwgpu::PairArgs make_args(cwgpu_context* ctx, const int32_t* d_pairs, const int3
     g.tiny_m = ctx->tiny_m;
     g.tiny_n = ctx->tiny_n;
     g.general = ctx->general_gaps;
+    g.path = ctx->d_path;
+    g.path_bytes = ctx->path_bytes;
+    g.path_slots = ctx->path_slots;
     return g;
 }
 
@@ -860,7 +915,7 @@ cudaError_t launch_persistent(const cwgpu::PairArgs& g, int max_grid, size_t sme
     attr[0].val.priority = priority;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, g.general ? k_pairwise<RS, true> : k_pairwise<RS, false>, g, -1LL);
+    return cudaLaunchKernelEx(&cfg, pair_kernel<RS>(g.general), g, -1LL);
 }
 
 // Warps per CTA for a launch of nlong long pairs: the knob, or, when it is 0,
@@ -944,6 +999,7 @@ void split_args(cwgpu_context* ctx, const int32_t* d_pairs, const int32_t* d_ord
     *gs = make_args(ctx, d_pairs, d_order + nlong, npairs - nlong, d_dist, d_stats);
     gs->counter = ctx->d_counter + 4;
     if (nlong > 0) gs->scratch += (size_t)ctx->grid * kWarpsPerBlock * 2 * (size_t)(ctx->lmax + 1);
+    gs->path = nullptr;
 }
 
 int status_error(cwgpu_context* ctx, int err) {
@@ -1086,6 +1142,7 @@ void cwgpu_destroy(cwgpu_context* ctx) {
     if (ctx->h_io) cudaFreeHost(ctx->h_io);
     if (ctx->ev_in) cudaEventDestroy(ctx->ev_in);
     dfree(ctx->d_scratch);
+    dfree(ctx->d_path);
     dfree(ctx->d_counter);
     dfree(ctx->d_err);
     dfree(ctx->d_call);
@@ -1387,9 +1444,8 @@ int cwgpu_align_pairs_plain(cwgpu_context* ctx, const int32_t* pairs, int64_t np
     if (e == cudaSuccess) {
         cwgpu::PairArgs g = make_args(ctx, d_pairs, nullptr, npairs, d_dist, d_stats);
         for (int64_t q = 0; q < npairs && e == cudaSuccess; ++q) {
-            auto* const k = short_pair(ctx, pairs, q)
-                                ? (g.general ? k_pairwise<cwgpu::kRShort, true> : k_pairwise<cwgpu::kRShort, false>)
-                                : (g.general ? k_pairwise<cwgpu::kR, true> : k_pairwise<cwgpu::kR, false>);
+            auto* const k = short_pair(ctx, pairs, q) ? pair_kernel<cwgpu::kRShort>(g.general)
+                                                      : pair_kernel<cwgpu::kR>(g.general);
             k<<<1, 32, block_smem(ctx->K, 1), ctx->stream>>>(g, (long long)q);
             e = cudaGetLastError();
         }

@@ -70,7 +70,7 @@ __host__ __device__ constexpr int warp_region_bytes(int K) {
 // Closed-form boundaries, which is what every sweep of the reference uses:
 //   H(-1, c) = ht0 - c*hts        E(-1, c) = H(-1, c) - eo      (c >= 1)
 //   H(r, 0)  = hl0 - (r+1)*hls    F(r, 0)  = H(r, 0) - fo
-//   H(-1, 0) = 0
+//   H(-1, 0) = corner
 // buf[c] (c = 1..cols) carries (H, E) of the last row of a stripe to the next
 // stripe, and in MODE_GLOBAL holds the final row on return.
 struct Task {
@@ -80,8 +80,19 @@ struct Task {
     int rows, cols;
     int ht0, hts, eo;
     int hl0, hls, fo;
+    int corner;
+    int pad;  // padding rows above the first (less than the rows of a lane)
 };
 
+// MODE_LOCAL_FWD: H floored at 0, the first maximum in row-major order tracked
+// (forwardPass's strict `hh > maxScore`). reversePass runs in the same loops,
+// on H + 1: the corner is 1, and its boundary of -1 becomes the floor. The
+// floor also holds inside the sweep there, which reversePass's does not; that
+// only adds paths that start at -1, whose remainder is a local alignment of at
+// most maxScore, so the first cell to reach maxScore is the same. The general
+// form (GEN, any penalties) cannot argue so and has MODE_LOCAL_REV: no floor,
+// and the first cell of the maximum of min(H, thresh) tracked (reversePass's
+// strict `hh > cost` and its break at cost >= maxScore).
 enum { MODE_LOCAL_FWD = 0, MODE_LOCAL_REV = 1, MODE_GLOBAL = 2 };
 
 struct Best {
@@ -96,12 +107,25 @@ constexpr int kPadScore = -32768;
 
 // Per-block constants the device functions read.
 struct Env {
-    const int* smat;     // shared matrix over remapped codes: 32x32, then the padding row
-    uint16_t* region;    // this warp's shared region (profile or tiny rows)
+    unsigned smat_at;    // shared matrix over remapped codes: 32x32, then the padding row
+    unsigned region_at;  // this warp's shared region (profile, tiny rows, box edges or frame stack)
     int K;               // number of remapped codes
     int gp1, gp2;        // remapped gapPos1 / gapPos2 (-1 if absent)
     int tiny_m, tiny_n;  // tiny-frame thresholds
     int* err;
+
+    // Kept as addresses in shared memory, so that functions that are not
+    // inlined still read them with shared-memory loads.
+    __device__ __forceinline__ void set_shared(const int* smat, uint16_t* region) {
+        smat_at = (unsigned)__cvta_generic_to_shared(smat);
+        region_at = (unsigned)__cvta_generic_to_shared(region);
+    }
+    __device__ __forceinline__ const int* smat() const {
+        return static_cast<const int*>(__cvta_shared_to_generic(smat_at));
+    }
+    __device__ __forceinline__ uint16_t* region() const {
+        return static_cast<uint16_t*>(__cvta_shared_to_generic(region_at));
+    }
 };
 
 template <int R>
@@ -234,16 +258,34 @@ __device__ __forceinline__ void mw_publish(const MwSync& m, int slot, int stripe
     m.prog[slot] = mw_word(m, stripe, cols);
 }
 
-// Where a stripe's boundary rows come from and go to. Single-warp sweeps read
-// and write one buffer; in a shared sweep the row above comes from the
-// predecessor warp's buffer and the stripe's last row goes to the own one.
+// A stripe's place in a shared sweep: the row above comes from the predecessor
+// warp's buffer and the stripe's last row goes to the own one.
 struct StripeIO {
-    const int2* rbuf;
-    int2* wbuf;
     int stripe;     // index of the stripe in the task
     int pred_slot;  // progress word of the warp with the previous stripe
     int own_slot;   // progress word of this warp
 };
+
+// The local sweeps of one warp keep rows that only they and the path read back,
+// much later: past L1, which at five CTAs per SM is small and holds the residues.
+template <int MODE, bool MW>
+__host__ __device__ constexpr bool rows_in_l2() {
+    return MODE != MODE_GLOBAL && !MW;
+}
+template <bool L2>
+__device__ __forceinline__ void row_store(int2* p, int2 v) {
+    if constexpr (L2)
+        __stcg(p, v);
+    else
+        *p = v;
+}
+template <bool L2>
+__device__ __forceinline__ int2 row_load(const int2* p) {
+    if constexpr (L2)
+        return __ldcg(p);
+    else
+        return *p;
+}
 
 // E of a task's first row, given H of the row above it.
 __device__ __forceinline__ int first_row_e(const Task& T, int h, int ge, int goe) {
@@ -281,16 +323,19 @@ __host__ __device__ inline bool padding_sound(int go, int ge) {
 // (padding_sound): rows of the stripe past the task's last row pass the row
 // above through, two selects per cell, so the segment's last used lane still
 // emits the last real row.
+// A lane with `writer` set stores its last row's (H, E) to `own`; the row above
+// the stripe is read from `above`.
 // MW: the stripe is one of a sweep shared by several warps (MwSync): before a
 // chunk of the row above is loaded the predecessor's progress is awaited, and
 // the writer publishes its progress every W columns and at the last one.
 template <int R, int W, int MODE, bool GEN, bool NC, bool MW = false>
 __device__ __forceinline__ void run_stripe(int nsteps, int fill, bool first, const Task& T, SweepState<R>& S, int sl,
-                                           int nvalid, bool writer, int ge, int goe, int thresh,
-                                           const uint16_t* prof_lane, const StripeIO& io = StripeIO{},
+                                           int nvalid, const int2* above, int2* own, bool writer, int ge, int goe,
+                                           int thresh, const uint16_t* prof_lane, const StripeIO& io = StripeIO{},
                                            const MwSync* mw = nullptr) {
+    constexpr bool kL2 = rows_in_l2<MODE, MW>();
     const int8_t* cp = T.cseq - sl;                 // residue of step t: cp[t]
-    int2* wp = (MW ? io.wbuf : T.buf) + 1 - sl;     // boundary-row entry of step t: wp[t]
+    int2* wp = own + 1 - sl;                        // the lane's row entry of step t: wp[t]
     const int wend = writer ? T.cols + sl : INT_MIN;  // the writer stores in steps below this
     int bnext = ldres<NC>(cp);
 
@@ -351,7 +396,7 @@ __device__ __forceinline__ void run_stripe(int nsteps, int fill, bool first, con
             }
         }
         if (t < wend) {
-            wp[t] = make_int2(hup, elast);
+            row_store<kL2>(wp + t, make_int2(hup, elast));
             if constexpr (MW) {
                 const int c = t - sl + 1;
                 if ((c & (W - 1)) == 0 || c == T.cols) mw_publish(*mw, io.own_slot, io.stripe, c);
@@ -372,7 +417,7 @@ __device__ __forceinline__ void run_stripe(int nsteps, int fill, bool first, con
                     mw_wait(*mw, io.pred_slot, mw_word(*mw, io.stripe - 1, min(T.cols, cfirst + W - 1)));
             }
             if (col <= T.cols) {
-                const int2 v = (MW ? io.rbuf : T.buf)[col];
+                const int2 v = row_load<kL2>(above + col);
                 S.nh = v.x;
                 S.ne = __viaddmax_s32(v.y, -ge, v.x - goe);
             }
@@ -403,12 +448,14 @@ __device__ __forceinline__ int fill_steps(int lused) { return lused & ~1; }
 // padding row r < 0 reproduces the top boundary in every column: its F starts
 // at H(-1, 1) and loses ge per column as the boundary does (hts == ge), and E
 // and the diagonal term stay below it as long as gapOpen >= 0 and 0 <= ge <=
-// -kPadScore. The local modes pad below the last row: such a row's H never
+// -kPadScore. The local mode pads below the last row: such a row's H never
 // exceeds one already seen above or to the left of it (gapOpen, ge >= 0), so
-// it is never the first maximum.
+// it is never the first maximum. Its reverse sweep pads above too, so that its
+// lanes end at the forward sweep's lane ends; those rows are at the floor, as
+// the boundary is.
 template <int R, int MODE, bool GEN, bool NC>
 __device__ __forceinline__ void stripe_begin(const Task& T, SweepState<R>& S, int lrow0, int gbest, int ge, int goe,
-                                             int thresh, const Env& X, int lane) {
+                                             int track, const Env& X, int lane) {
     int a[R];
 #pragma unroll
     for (int k = 0; k < R; ++k) {
@@ -416,7 +463,7 @@ __device__ __forceinline__ void stripe_begin(const Task& T, SweepState<R>& S, in
         a[k] = (r >= 0 && r < T.rows) ? ldres<NC>(T.rseq + r) : (GEN ? 0 : kPadRow);
     }
     __syncwarp();  // previous users of the shared region are done
-    build_profile<R>(X.region, X.smat, a, lane, X.K);
+    build_profile<R>(X.region(), X.smat(), a, lane, X.K);
     __syncwarp();  // previous stripe's buf writes visible to the whole segment
     constexpr int kLow = -(1 << 29);  // below every boundary value
 #pragma unroll
@@ -424,27 +471,24 @@ __device__ __forceinline__ void stripe_begin(const Task& T, SweepState<R>& S, in
         const int r = lrow0 + k;
         S.hl[k] = T.hl0 - (r + 1) * T.hls;
         S.fp[k] = max(S.hl[k] - T.fo - ge, S.hl[k] - goe);
-        if (MODE == MODE_GLOBAL && !GEN && r < 0) {
-            S.hl[k] = r == -1 ? 0 : kLow;  // H(-1, 0), else never taken
-            S.fp[k] = T.ht0 - T.hts;       // H(-1, 1)
+        if (!GEN && r < 0) {
+            S.hl[k] = r == -1 ? T.corner : kLow;  // H(-1, 0), else never taken
+            S.fp[k] = T.ht0 - T.hts;              // H(-1, 1)
         }
     }
-    S.diag = lrow0 == 0 ? 0 : T.hl0 - lrow0 * T.hls;
-    if (MODE == MODE_GLOBAL && !GEN && lrow0 < 0) S.diag = kLow;
+    S.diag = lrow0 == 0 ? T.corner : T.hl0 - lrow0 * T.hls;
+    if (!GEN && lrow0 < 0) S.diag = kLow;
     S.hout = 0;
     S.eout = 0;
     S.bv = gbest;
     S.bk = 0xffffffffu;
-    // The reverse sweep ends in the stripe whose H first reaches thresh, and
-    // with gap penalties >= 0 some cell does (the forward optimum read
-    // backwards), so nothing below thresh need be tracked.
-    S.thr = (MODE == MODE_LOCAL_REV && !GEN) ? thresh : gbest + 1;
+    S.thr = max(gbest + 1, track);
     if (lrow0 >= T.rows) S.thr = INT_MAX;  // padding only
 }
 
 // Boundary chunk registers at the start of a stripe, from the closed form or
 // from the previous stripe's last row.
-template <int R, int W>
+template <int R, int W, bool L2>
 __device__ __forceinline__ void stripe_chunks(const Task& T, SweepState<R>& S, const int2* rb, bool first, int sl,
                                               int ge, int goe) {
     if (first) {
@@ -456,12 +500,12 @@ __device__ __forceinline__ void stripe_chunks(const Task& T, SweepState<R>& S, c
     }
     S.ch = S.ce = S.nh = S.ne = 0;
     if (1 + sl <= T.cols) {
-        const int2 v = rb[1 + sl];
+        const int2 v = row_load<L2>(rb + 1 + sl);
         S.ch = v.x;
         S.ce = __viaddmax_s32(v.y, -ge, v.x - goe);
     }
     if (W + 1 + sl <= T.cols) {
-        const int2 v = rb[W + 1 + sl];
+        const int2 v = row_load<L2>(rb + W + 1 + sl);
         S.nh = v.x;
         S.ne = __viaddmax_s32(v.y, -ge, v.x - goe);
     }
@@ -480,33 +524,44 @@ __device__ __forceinline__ int stripe_best(const SweepState<R>& S, int lrow0, in
     return wv;
 }
 
-// Padding rows above the first row of a MODE_GLOBAL task.
-template <int R, int MODE, bool GEN>
-__device__ __forceinline__ int top_padding(int rows) {
-    return (MODE == MODE_GLOBAL && !GEN && rows > 0) ? (R - rows % R) % R : 0;
+// Padding rows that let a task of `rows` rows end with a lane's last row.
+template <int R>
+__device__ __forceinline__ int lane_padding(int rows) {
+    return rows > 0 ? (R - rows % R) % R : 0;
 }
+
+// Rows a local sweep keeps for the path (cwgpu_path.cuh). Node row i has the
+// first i residues of the forward sequence on one side; a lane whose last row
+// is the task's row r ends at i = start + dir * (r + 1) (the forward sweep: 0
+// and 1; the reverse: its first row and -1). Those with 0 < i < end and
+// i % every == 0 go to rows + (i / every - 1) * stride. rows == nullptr: none.
+struct RowSave {
+    int2* rows;
+    size_t stride;
+    int every;
+    int start, dir, end;
+};
 
 // The wavefront sweep. W = lanes per segment (32: one task per warp, 16: two
 // tasks, one per half-warp; the two tasks have the same column count).
-// MODE_LOCAL_FWD tracks the first maximum in row-major order (forwardPass's
-// strict `hh > maxScore`); MODE_LOCAL_REV tracks the first cell, in the sweep's
-// row-major order, of the maximum of min(H, thresh) (reversePass's strict
-// `hh > cost` and its break at cost >= maxScore) and stops after the first
-// stripe that reached thresh.
+// The local modes track the first cell of the maximum, of values from `track`
+// on, and stop after the first stripe that reached thresh.
 template <int R, int W, int MODE, bool GEN, bool NC = true>
-__device__ void sweep(const Task& T, int go, int ge, int thresh, const Env& X, Best& best) {
+__device__ __forceinline__ void sweep(const Task& T, int go, int ge, int track, int thresh, const Env& X, Best& best,
+                                      const RowSave& save = RowSave{}) {
     const int lane = threadIdx.x & 31;
     const int sl = lane & (W - 1);
     const int goe = go + ge;
     constexpr int RPS = W * R;
-    const int pad = top_padding<R, MODE, GEN>(T.rows);
+    const int pad = T.pad;
     const int prows = T.rows + pad;
     const int nstr = prows > 0 ? (prows + RPS - 1) / RPS : 0;
     const int nstr_max = __reduce_max_sync(kFull, nstr);
-    const uint16_t* prof_lane = X.region + lane * R;
+    const uint16_t* prof_lane = X.region() + lane * R;
     best.val = 0;
     best.key = 0xffffffffu;
     SweepState<R> S;
+    const int2* above = T.buf;
 
     for (int s = 0; s < nstr_max; ++s) {
         const int seg_rows = min(prows - s * RPS, RPS);
@@ -516,15 +571,25 @@ __device__ void sweep(const Task& T, int go, int ge, int thresh, const Env& X, B
         const int nsteps = (seg_rows > 0 && T.cols > 0) ? T.cols + lused - 1 : 0;
         const int nsteps_max = __reduce_max_sync(kFull, nsteps);
         const bool last = (s == nstr - 1);
-        const bool writer = (sl == lused - 1) && (MODE == MODE_GLOBAL || !last);
+        bool writer = (sl == lused - 1) && (MODE == MODE_GLOBAL || !last);
+        int2* own = T.buf;
+        if (R == kR && MODE != MODE_GLOBAL && !GEN && save.rows) {
+            const int i = save.start + save.dir * (lrow0 + R);
+            if (sl < lused && i > 0 && i < save.end && (i & (save.every - 1)) == 0) {
+                own = save.rows + (size_t)(i / save.every - 1) * save.stride;
+                writer = true;
+            }
+        }
         const int gbest = best.val;
-        stripe_begin<R, MODE, GEN, NC>(T, S, lrow0, gbest, ge, goe, thresh, X, lane);
-        stripe_chunks<R, W>(T, S, T.buf, s == 0, sl, ge, goe);
+        stripe_begin<R, MODE, GEN, NC>(T, S, lrow0, gbest, ge, goe, track, X, lane);
+        stripe_chunks<R, W, rows_in_l2<MODE, false>()>(T, S, above, s == 0, sl, ge, goe);
         run_stripe<R, W, MODE, GEN, NC>(nsteps_max, fill_steps(__reduce_max_sync(kFull, lused)), s == 0, T, S, sl, nvalid,
-                                        writer, ge, goe, thresh, prof_lane);
+                                        above, own, writer, ge, goe, thresh, prof_lane);
+        if (MODE != MODE_GLOBAL)
+            above = reinterpret_cast<const int2*>(__shfl_sync(kFull, reinterpret_cast<unsigned long long>(own), W - 1));
         if (MODE != MODE_GLOBAL) {
             stripe_best<R>(S, lrow0, gbest, best);
-            if (MODE == MODE_LOCAL_REV && best.val >= thresh) break;
+            if (best.val >= thresh) break;
         }
     }
     __syncwarp();
@@ -536,7 +601,7 @@ __device__ void sweep(const Task& T, int go, int ge, int thresh, const Env& X, B
 // bufs + (slot0 + rank) * stride, from which the warp with the next stripe
 // reads it (MwSync). Every warp tracks the best of its own stripes the way
 // sweep() does (strict, so the first in row-major order); the caller reduces
-// the ranks' results: maximum value, then lowest key. MODE_LOCAL_REV: *stop
+// the ranks' results: maximum value, then lowest key. Local modes: *stop
 // (shared, INT_MAX at the start) is lowered to every stripe that reached
 // thresh; stripes above it are skipped (their progress is published as
 // complete so no successor waits), which leaves the result of the lowest
@@ -546,30 +611,30 @@ __device__ void sweep(const Task& T, int go, int ge, int thresh, const Env& X, B
 __host__ __device__ inline int mw_stripes(int rows, int R) { return rows > 0 ? (rows + 32 * R - 1) / (32 * R) : 0; }
 
 template <int R, int MODE, bool GEN, bool NC = true>
-__device__ void sweep_mw(const Task& T, int go, int ge, int thresh, const Env& X, Best& best, int2* bufs,
+__device__ void sweep_mw(const Task& T, int go, int ge, int track, int thresh, const Env& X, Best& best, int2* bufs,
                          size_t stride, int slot0, int rank, int nw, const MwSync& mw, volatile int* stop) {
     constexpr int W = 32;
     const int lane = threadIdx.x & 31;
     const int sl = lane;
     const int goe = go + ge;
     constexpr int RPS = W * R;
-    const int pad = top_padding<R, MODE, GEN>(T.rows);
+    const int pad = T.pad;
     const int prows = T.rows + pad;
     const int nstr = mw_stripes(T.rows, R);
-    const uint16_t* prof_lane = X.region + lane * R;
+    const uint16_t* prof_lane = X.region() + lane * R;
     best.val = 0;
     best.key = 0xffffffffu;
     if (T.cols <= 0) return;  // no column: nothing to hand over (callers give columns)
     SweepState<R> S;
     StripeIO io;
-    io.wbuf = bufs + (size_t)(slot0 + rank) * stride;
+    int2* const own = bufs + (size_t)(slot0 + rank) * stride;
     io.own_slot = slot0 + rank;
 
     for (int s = rank; s < nstr; s += nw) {
         io.stripe = s;
         io.pred_slot = slot0 + (s + nw - 1) % nw;
-        io.rbuf = bufs + (size_t)io.pred_slot * stride;
-        if (MODE == MODE_LOCAL_REV && __shfl_sync(kFull, *stop, 0) < s) {  // one decision per warp
+        const int2* const above = bufs + (size_t)io.pred_slot * stride;
+        if (MODE != MODE_GLOBAL && __shfl_sync(kFull, *stop, 0) < s) {  // one decision per warp
             if (lane == 0) mw_publish(mw, io.own_slot, s, T.cols);
             continue;
         }
@@ -581,14 +646,14 @@ __device__ void sweep_mw(const Task& T, int go, int ge, int thresh, const Env& X
         const bool last = (s == nstr - 1);
         const bool writer = (sl == lused - 1) && (MODE == MODE_GLOBAL || !last);
         const int gbest = best.val;
-        stripe_begin<R, MODE, GEN, NC>(T, S, lrow0, gbest, ge, goe, thresh, X, lane);
+        stripe_begin<R, MODE, GEN, NC>(T, S, lrow0, gbest, ge, goe, track, X, lane);
         if (s > 0) mw_wait(mw, io.pred_slot, mw_word(mw, s - 1, min(T.cols, 2 * W)));
-        stripe_chunks<R, W>(T, S, io.rbuf, s == 0, sl, ge, goe);
-        run_stripe<R, W, MODE, GEN, NC, true>(nsteps, fill_steps(lused), s == 0, T, S, sl, nvalid, writer, ge, goe,
-                                              thresh, prof_lane, io, &mw);
+        stripe_chunks<R, W, rows_in_l2<MODE, true>()>(T, S, above, s == 0, sl, ge, goe);
+        run_stripe<R, W, MODE, GEN, NC, true>(nsteps, fill_steps(lused), s == 0, T, S, sl, nvalid, above, own, writer,
+                                              ge, goe, thresh, prof_lane, io, &mw);
         if (MODE != MODE_GLOBAL) {
             const int wv = stripe_best<R>(S, lrow0, gbest, best);
-            if (MODE == MODE_LOCAL_REV && wv >= thresh && lane == 0) atomicMin((int*)stop, s);
+            if (wv >= thresh && lane == 0) atomicMin((int*)stop, s);
         }
     }
     __syncwarp();
@@ -635,7 +700,7 @@ static __device__ int lane_mm(const int8_t* s1, const int8_t* s2, int A0, int B0
                 const int hh0 = -(te + ge) - (tb + ge * N);
                 if (hh0 > midh) midh = hh0;
                 int midj = 0;
-                const int* row = X.smat + 32 * ldres<NC>(s1 + A);
+                const int* row = X.smat() + 32 * ldres<NC>(s1 + A);
                 for (int j = 1; j <= N; ++j) {
                     const int hh = row[ldres<NC>(s2 + B + j - 1)] - (N - j > 0 ? te + ge * (N - j) : 0) -
                                    (j - 1 > 0 ? tb + ge * (j - 1) : 0);
@@ -662,7 +727,7 @@ static __device__ int lane_mm(const int8_t* s1, const int8_t* s2, int A0, int B0
             }
             t = -tb;
             for (int i = 1; i <= midi; ++i) {
-                const int* row = X.smat + 32 * ldres<NC>(s1 + A + i - 1);
+                const int* row = X.smat() + 32 * ldres<NC>(s1 + A + i - 1);
                 int s = TI(HH, 0);
                 int hh = t = t - ge;
                 TI(HH, 0) = hh;
@@ -686,7 +751,7 @@ static __device__ int lane_mm(const int8_t* s1, const int8_t* s2, int A0, int B0
             }
             t = -te;
             for (int i = M - 1; i >= midi; --i) {
-                const int* row = X.smat + 32 * ldres<NC>(s1 + A + i);
+                const int* row = X.smat() + 32 * ldres<NC>(s1 + A + i);
                 int s = TI(RR, N);
                 int hh = t = t - ge;
                 TI(RR, N) = hh;
@@ -845,14 +910,15 @@ __device__ __forceinline__ void midpoint_scan(const int2* fwd, const int2* rev, 
 // seq1[A + i] is s1[A + i - 1]. s1r/s2r are the reversed copies of the n- and
 // m-residue sequences (s1r[i] = s1[n - 1 - i]), which the reverse halves read.
 // N0 carries the top frame's flags: tb = gapOpen if bit 29, te if bit 30 (a
-// whole pair's frame has neither). SHARE: after each division the right child,
+// whole pair's frame has neither). list: its nlist frames (A, B, M, N and
+// flags) instead of that one, and no score. SHARE: after each division the right child,
 // if it has at least fs->min_rows rows, goes to the CTA's shared stack (when
 // it has room) for any warp of the CTA to take, instead of this warp's own.
 template <int RS, bool GEN, bool NC = true, bool SHARE = false>
-static __device__ void mm_align(const int8_t* s1, const int8_t* s1r, int n, const int8_t* s2, const int8_t* s2r, int m,
+static __device__ __forceinline__ void mm_align(const int8_t* s1, const int8_t* s1r, int n, const int8_t* s2, const int8_t* s2r, int m,
                                 int A0, int B0, int M0, int N0, int go, int ge, int2* bufA, int2* bufB, const Env& X,
                                 int& mm_score, int& n_ident, int& n_match, long long& cells,
-                                const FrameShare* fs = nullptr) {
+                                const FrameShare* fs = nullptr, const int4* list = nullptr, int nlist = 0) {
     const int lane = threadIdx.x & 31;
     constexpr int NMASK = (1 << 29) - 1;
     int stA = 0, stB = 0, stM = 0, stN = 0;  // stack entry `lane`
@@ -863,13 +929,24 @@ static __device__ void mm_align(const int8_t* s1, const int8_t* s1r, int n, cons
         stM = M0;
         stN = N0;
     }
-    int sp = 1, nq = 0;
-    bool top = true;
+    int sp = list ? 0 : 1, nq = 0;
+    int next = 0;  // of the list
+    bool top = !list;
     int ident = 0, matches = 0, mm = 0;
     long long ncell = 0;
     bool q_has_top = false;  // queue entry 0 is the top frame
 
-    while (sp > 0 || nq > 0) {
+    while (sp > 0 || nq > 0 || next < nlist) {
+        if (sp == 0 && next < nlist) {
+            const int4 f = list[next++];
+            if (lane == 0) {
+                stA = f.x;
+                stB = f.y;
+                stM = f.z;
+                stN = f.w;
+            }
+            sp = 1;
+        }
         if (sp == 0 || nq == 32) {
             // Solve the queued tiny frames, one per lane.
             __syncwarp();
@@ -877,7 +954,7 @@ static __device__ void mm_align(const int8_t* s1, const int8_t* s1r, int n, cons
             long long lc = 0;
             if (lane < nq) {
                 score = lane_mm<NC>(s1, s2, qA, qB, qM, qN & NMASK, (qN >> 29) & 1, (qN >> 30) & 1, go, ge, X,
-                                reinterpret_cast<int*>(X.region), li, lm, lc);
+                                reinterpret_cast<int*>(X.region()), li, lm, lc);
             }
             __syncwarp();
             ident += __reduce_add_sync(kFull, li);
@@ -929,7 +1006,7 @@ static __device__ void mm_align(const int8_t* s1, const int8_t* s1r, int n, cons
             int bv = INT_MIN, bj = 0x7fffffff;
             for (int j = lane + 1; j <= N; j += 32) {
                 const int rb = ldres<NC>(s2 + B + j - 1);
-                const int v = X.smat[ra * 32 + rb] - (N - j > 0 ? te + ge * (N - j) : 0) -
+                const int v = X.smat()[ra * 32 + rb] - (N - j > 0 ? te + ge * (N - j) : 0) -
                               (j - 1 > 0 ? tb + ge * (j - 1) : 0);
                 if (v > bv) {
                     bv = v;
@@ -975,8 +1052,10 @@ static __device__ void mm_align(const int8_t* s1, const int8_t* s1r, int n, cons
         t.eo = go;
         t.hls = ge;
         t.fo = go;
+        t.corner = 0;
+        t.pad = GEN ? 0 : lane_padding<RS>(t.rows);
         Best unused;
-        sweep<RS, 16, MODE_GLOBAL, GEN, NC>(t, go, ge, 0, X, unused);
+        sweep<RS, 16, MODE_GLOBAL, GEN, NC>(t, go, ge, 0, 0, X, unused);
 
         int midh, midj;
         bool type2;
@@ -1046,6 +1125,12 @@ __device__ __forceinline__ void stage_matrix(int* smat, const int32_t* matrix) {
     for (int i = threadIdx.x; i < kSmatWords; i += blockDim.x) smat[i] = i < 32 * 32 ? matrix[i] : kPadScore;
 }
 
+}  // namespace cwgpu
+
+#include "cwgpu_path.cuh"
+
+namespace cwgpu {
+
 struct PairArgs {
     const int8_t* codes;
     const int64_t* offs;
@@ -1067,8 +1152,117 @@ struct PairArgs {
     int gp1, gp2;  // remapped gap codes
     int K;         // remapped alphabet size
     int tiny_m, tiny_n;
+    unsigned char* path;  // the warps' slices for cwgpu_path.cuh, path_bytes each; nullptr: none
+    size_t path_bytes;
+    long long path_slots;  // warps that have a slice
     int general;  // host: gap penalties outside padding_sound somewhere, take the GEN kernels
 };
+
+// A sequence's reversed copy (cwgpu_layout.h).
+__device__ __forceinline__ const int8_t* rev_of(const int8_t* s, int len) { return s + rev_offset(len); }
+
+// forwardPass over all of s1 x s2.
+__device__ __forceinline__ Task local_task(const int8_t* s1, int n, const int8_t* s2, int m, int go, int2* buf) {
+    Task t;
+    t.rseq = s1;
+    t.cseq = s2;
+    t.rows = n;
+    t.cols = m;
+    t.ht0 = t.hts = 0;
+    t.eo = go;
+    t.hl0 = t.hls = 0;
+    t.fo = go;
+    t.corner = t.pad = 0;
+    t.buf = buf;
+    return t;
+}
+
+// reversePass from the end cell (se1, se2): rows se1-1 .. 0 of s1, columns
+// se2 .. 1. GEN: the reference's -1 boundaries; else H + 1 over the floor
+// (MODE_LOCAL_FWD).
+template <int RS, bool GEN>
+__device__ __forceinline__ Task reverse_task(const int8_t* s1r, int n, int se1, const int8_t* s2r, int m, int se2,
+                                             int go, int2* buf) {
+    Task t = local_task(s1r + (n - se1), se1, s2r + (m - se2), se2, GEN ? 0 : go, buf);
+    if (GEN) {
+        t.ht0 = t.hl0 = -1;
+    } else {
+        t.corner = 1;
+        t.pad = lane_padding<RS>(se1);
+    }
+    return t;
+}
+
+// What the local sweeps of a pair find: maxScore, its cell (1-based) and the
+// start cell; whether reversePass reached maxScore (else it ran to its end).
+struct PairEnds {
+    int max_score, se1, se2, sb1, sb2;
+    bool reached;
+};
+
+// forwardPass, then reversePass from its end cell: one copy of the sweep's code
+// for both, which at this size the instruction cache rewards. fwd/rev: rows to
+// keep for the path (nullptr: none).
+template <int RS, bool GEN, bool NC>
+__device__ __forceinline__ PairEnds pair_ends(const int8_t* s1, int n, const int8_t* s2, int m, int go, int ge,
+                                              int2* buf, int2* fwd, int2* rev, size_t stride, int every,
+                                              const Env& X) {
+    PairEnds e{0, 0, 0, 1, 1, false};
+    RowSave save{fwd, stride, every, 0, 1, n};
+    Task t = local_task(s1, n, s2, m, go, buf);
+#pragma unroll 1
+    for (int pass = 0; pass < 2; ++pass) {
+        Best b;
+        if (GEN && pass == 1)
+            sweep<RS, 32, GEN ? MODE_LOCAL_REV : MODE_LOCAL_FWD, GEN, NC>(t, go, ge, 1, e.max_score, X, b);
+        else
+            sweep<RS, 32, MODE_LOCAL_FWD, GEN, NC>(t, go, ge, pass ? e.max_score + 1 : 1,
+                                                   pass ? e.max_score + 1 : INT_MAX, X, b, save);
+        if (pass == 0) {
+            e.max_score = b.val;
+            if (b.val <= 0) break;
+            e.se1 = (int)(b.key >> 16) + 1;
+            e.se2 = (int)(b.key & 0xffffu);
+            t = reverse_task<RS, GEN>(rev_of(s1, n), n, e.se1, rev_of(s2, m), m, e.se2, go, buf);
+            save = RowSave{rev, stride, every, e.se1, -1, e.se1};
+        } else {
+            if (!GEN) b.val -= 1;
+            if (b.val > 0) {
+                e.sb1 = e.se1 - (int)(b.key >> 16);
+                e.sb2 = e.se2 - (int)(b.key & 0xffffu) + 1;
+            }
+            e.reached = b.val >= e.max_score;
+        }
+    }
+    return e;
+}
+
+// The inner-loop iterations the reference executes in the two local sweeps;
+// reversePass stops at the first cell reaching maxScore (:404-413).
+__device__ __forceinline__ unsigned long long reverse_cells(const PairEnds& e) {
+    if (e.max_score <= 0) return 0;
+    return e.reached ? (unsigned long long)(e.se1 - e.sb1) * e.se2 + (unsigned long long)(e.se2 - e.sb2 + 1)
+                     : (unsigned long long)e.se1 * e.se2;
+}
+
+// Distance (:170-181), float arithmetic with IEEE rounding, and the statistics.
+__device__ __forceinline__ float pair_result(const PairEnds& e, int mm, int ident, int matches, int len1, int len2,
+                                             cwgpu_pair_stats& st) {
+    float mmv = (float)(100 * ident);
+    if (len1 == 0 || len2 == 0)
+        mmv = 0.0f;
+    else
+        mmv = __fdiv_rn(mmv, (float)min(len1, len2));
+    st.fwd_score = e.max_score;
+    st.se1 = e.se1;
+    st.se2 = e.se2;
+    st.sb1 = e.sb1;
+    st.sb2 = e.sb2;
+    st.mm_score = mm;
+    st.n_ident = ident;
+    st.n_match = matches;
+    return __fdiv_rn(__fsub_rn(100.0f, mmv), 100.0f);
+}
 
 // forwardPass + reversePass + diff + distance for one pair, given its 0-based
 // code pointers, lengths, non-gap residue counts and gap penalties. Returns
@@ -1078,85 +1272,20 @@ struct PairArgs {
 // warp steps when n <= 128 (one stripe, lanes of 4 rows instead of
 // half-empty lanes of 8). Each sequence's reversed copy follows it at the
 // next 16-byte boundary (cwgpu_layout.h), and kGuard readable bytes surround both.
-__device__ __forceinline__ const int8_t* rev_of(const int8_t* s, int len) { return s + rev_offset(len); }
-
 template <int RS, bool GEN, bool NC = true>
 static __device__ float align_one(const int8_t* s1, int n, const int8_t* s2, int m, int len1, int len2, int go, int ge,
                            int2* bufA, int2* bufB, const Env& X, cwgpu_pair_stats& st, unsigned long long (&acc)[3]) {
-    const int8_t* s1r = rev_of(s1, n);
-    const int8_t* s2r = rev_of(s2, m);
     st = cwgpu_pair_stats{0, 0, 0, 0, 0, 0, 0, 0};
     if (n <= 0 || m <= 0) return 1.0f;
-    // forwardPass
-    Task t;
-    t.rseq = s1;
-    t.cseq = s2;
-    t.rows = n;
-    t.cols = m;
-    t.ht0 = 0;
-    t.hts = 0;
-    t.eo = go;
-    t.hl0 = 0;
-    t.hls = 0;
-    t.fo = go;
-    t.buf = bufA;
-    Best fb;
-    sweep<RS, 32, MODE_LOCAL_FWD, GEN, NC>(t, go, ge, 0, X, fb);
-    const int max_score = fb.val;
-    const int se1 = max_score > 0 ? (int)(fb.key >> 16) + 1 : 0;
-    const int se2 = max_score > 0 ? (int)(fb.key & 0xffffu) : 0;
-
-    // reversePass
-    int sb1 = 1, sb2 = 1;
-    if (se1 > 0) {
-        Task r;
-        r.rseq = s1r + (n - se1);  // rows se1-1 .. 0 of s1
-        r.cseq = s2r + (m - se2);  // columns se2 .. 1
-        r.rows = se1;
-        r.cols = se2;
-        r.ht0 = -1;
-        r.hts = 0;
-        r.eo = 0;
-        r.hl0 = -1;
-        r.hls = 0;
-        r.fo = 0;
-        r.buf = bufA;
-        Best rb;
-        sweep<RS, 32, MODE_LOCAL_REV, GEN, NC>(r, go, ge, max_score, X, rb);
-        if (rb.val > 0) {
-            sb1 = se1 - (int)(rb.key >> 16);
-            sb2 = se2 - (int)(rb.key & 0xffffu) + 1;
-        }
-        // reversePass stops at the first cell reaching maxScore (:404-413).
-        if (rb.val >= max_score)
-            acc[1] += (unsigned long long)(se1 - sb1) * se2 + (unsigned long long)(se2 - sb2 + 1);
-        else
-            acc[1] += (unsigned long long)se1 * se2;
-    }
-    acc[0] += (unsigned long long)n * m;
-
-    // diff + tracePath
+    const PairEnds e = pair_ends<RS, GEN, NC>(s1, n, s2, m, go, ge, bufA, nullptr, nullptr, 0, 1, X);
     int mm = 0, ident = 0, matches = 0;
     long long dcells = 0;
-    mm_align<RS, GEN, NC>(s1, s1r, n, s2, s2r, m, sb1 - 1, sb2 - 1, se1 - sb1 + 1, se2 - sb2 + 1, go, ge, bufA, bufB, X, mm,
-                 ident, matches, dcells);
+    mm_align<RS, GEN, NC>(s1, rev_of(s1, n), n, s2, rev_of(s2, m), m, e.sb1 - 1, e.sb2 - 1, e.se1 - e.sb1 + 1,
+                          e.se2 - e.sb2 + 1, go, ge, bufA, bufB, X, mm, ident, matches, dcells);
+    acc[0] += (unsigned long long)n * m;
+    acc[1] += reverse_cells(e);
     acc[2] += (unsigned long long)dcells;
-
-    // distance (:170-181), float arithmetic with IEEE rounding.
-    float mmv = (float)(100 * ident);
-    if (len1 == 0 || len2 == 0)
-        mmv = 0.0f;
-    else
-        mmv = __fdiv_rn(mmv, (float)min(len1, len2));
-    st.fwd_score = max_score;
-    st.se1 = se1;
-    st.se2 = se2;
-    st.sb1 = sb1;
-    st.sb2 = sb2;
-    st.mm_score = mm;
-    st.n_ident = ident;
-    st.n_match = matches;
-    return __fdiv_rn(__fsub_rn(100.0f, mmv), 100.0f);
+    return pair_result(e, mm, ident, matches, len1, len2, st);
 }
 
 // Aligns pair q: FullPairwiseAlign.cpp:112-183 for one (si, sj).
@@ -1173,6 +1302,91 @@ static __device__ void align_pair(const PairArgs& g, long long q, const Env& X, 
         g.dist[q] = dist;
         if (g.stats) g.stats[q] = st;
     }
+}
+
+// The same for the long-pair kernel, with the path of cwgpu_path.cuh where the
+// warp has a slice for it. In two parts: everything after the sweeps is a call
+// that finds its arguments again by itself, so that the sweeps' loops have the
+// registers (with it inlined the compiler computed lane numbers and addresses
+// anew in every step).
+struct LongPair {
+    const int8_t *s1, *s2;
+    int n, m, si, sj, go;
+    int2* buf;
+    PathMem pm;
+    bool path;
+};
+
+__device__ __forceinline__ LongPair long_pair(const PairArgs& g, long long q, long long slot) {
+    LongPair p;
+    p.si = g.pairs[2 * q];
+    p.sj = g.pairs[2 * q + 1];
+    p.n = g.lens[p.si];
+    p.m = g.lens[p.sj];
+    p.s1 = g.codes + g.offs[p.si];
+    p.s2 = g.codes + g.offs[p.sj];
+    p.go = g.go_table[min(p.n, p.m)];
+    p.buf = g.scratch + (size_t)slot * 2 * (g.lmax + 1);
+    p.path = g.path && slot < g.path_slots && g.ge >= 1 && p.go <= kMaxPathOpen &&
+             path_mem(p.n, p.m, g.path + (size_t)slot * g.path_bytes, g.path_bytes, p.pm);
+    return p;
+}
+
+static __device__ __noinline__ void finish_long(const PairArgs& g, long long q, long long slot, PairEnds e,
+                                                const Env& env) {
+    const Env X = env;
+    const LongPair p = long_pair(g, q, slot);
+    int2* const bufA = p.buf;
+    int2* const bufB = bufA + (g.lmax + 1);
+    const int A0 = e.sb1 - 1, B0 = e.sb2 - 1;
+    int mm = 0, ident = 0, matches = 0;
+    long long dcells = 0;
+    int rest = -1;  // frames for mm_align; -1: the pair's own
+    if (p.path && e.max_score > 0 &&
+        path_band<true>(p.s1, p.n, p.s2, p.pm, bufB, A0, B0, e.se1, e.se2, e.max_score, p.go, g.ge, X)) {
+        rest = path_walk<true>(p.s1, p.n, p.s2, p.m, p.pm, bufB, A0, B0, e.se1, e.se2, p.go, g.ge, X, ident, matches,
+                               dcells);
+        mm = e.max_score;  // the box's best path is the local optimum
+    }
+    if (rest != 0) {
+        int id = 0, mt = 0, score = 0;
+        long long ce = 0;
+        mm_align<kR, false, true>(p.s1, rev_of(p.s1, p.n), p.n, p.s2, rev_of(p.s2, p.m), p.m, A0, B0, e.se1 - A0,
+                                  e.se2 - B0, p.go, g.ge, bufA, bufB, X, score, id, mt, ce, nullptr,
+                                  rest > 0 ? p.pm.list : nullptr, max(rest, 0));
+        if (rest < 0) mm = score;
+        ident += id;
+        matches += mt;
+        dcells += ce;
+    }
+    if ((threadIdx.x & 31) == 0) {
+        cwgpu_pair_stats st;
+        g.dist[q] = pair_result(e, mm, ident, matches, g.nres[p.si], g.nres[p.sj], st);
+        if (g.stats) g.stats[q] = st;
+        if (g.cells) {
+            atomicAdd(g.cells + 0, (unsigned long long)p.n * p.m);
+            atomicAdd(g.cells + 1, reverse_cells(e));
+            atomicAdd(g.cells + 2, (unsigned long long)dcells);
+        }
+    }
+    __syncwarp();
+}
+
+__device__ __forceinline__ void align_long(const PairArgs& g, long long q, long long slot, const Env& X) {
+    PairEnds e;
+    {
+        const LongPair p = long_pair(g, q, slot);
+        if (p.n <= 0 || p.m <= 0) {
+            if ((threadIdx.x & 31) == 0) {
+                g.dist[q] = 1.0f;
+                if (g.stats) g.stats[q] = cwgpu_pair_stats{0, 0, 0, 0, 0, 0, 0, 0};
+            }
+            return;
+        }
+        e = pair_ends<kR, false, true>(p.s1, p.n, p.s2, p.m, p.go, g.ge, p.buf, p.path ? p.pm.fwd : nullptr,
+                                       p.path ? p.pm.rev : nullptr, p.pm.stride, p.pm.every, X);
+    }
+    finish_long(g, q, slot, e, X);
 }
 
 }  // namespace cwgpu

@@ -163,8 +163,7 @@ __global__ void __launch_bounds__(kNaWarpsPerBlock * 32) k_pairwise_noalloc(NaAr
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const long long slot = (long long)blockIdx.x * kNaWarpsPerBlock + warp;
     cwgpu::Env X;
-    X.smat = smat;
-    X.region = na_region + (size_t)warp * (kNaRegionBytes / sizeof(uint16_t));
+    X.set_shared(smat, na_region + (size_t)warp * (kNaRegionBytes / sizeof(uint16_t)));
     X.K = CWGPU_NUMRES;
     X.gp1 = (a.gp1 >= 0 && a.gp1 < CWGPU_NUMRES) ? a.gp1 : -1;
     X.gp2 = (a.gp2 >= 0 && a.gp2 < CWGPU_NUMRES) ? a.gp2 : -1;

@@ -1,0 +1,804 @@
+// The path diff() chooses, from the rows the local sweeps saved.
+//
+// Myers-Miller divides a pair's box [sb1..se1] x [sb2..se2] recursively, about
+// two more sweeps' worth of cells, but what it decides at a row depends only on
+// the cells that lie on some optimal path: the midpoint scan takes the columns
+// whose forward and reverse values add up to the frame's optimum, and its tie
+// rule compares values of those columns. forwardPass and reversePass have
+// already computed both values for every row. So:
+//
+// 1. Every G rows (G a multiple of 32) the two sweeps keep their row (H, E).
+//    Adding them up gives, at such a row, exactly the columns optimal paths
+//    cross it in (path_row). Local starts other than (sb1, sb2) and the -1
+//    boundaries of reversePass can only add columns or values below the
+//    optimum: a path from such a boundary scores at most maxScore - 1.
+// 2. Between two such rows optimal paths stay inside the box of their first
+//    and last columns, about G x G cells, whose forward and reverse values are
+//    recomputed (path_boxes). Every row gets the first and last column of its
+//    cells on an optimal path, whether through H (type 1 of the midpoint scan)
+//    or inside a vertical gap (type 2).
+// 3. The frames of the recursion are then walked 32 at a time, one per lane
+//    (path_walk). Where a frame's middle row has a single column and type the
+//    midpoint is that column. Elsewhere the lane runs diff()'s own two halves
+//    over the rows' column ranges, from the nearest rows above and below where
+//    every path goes through H of one cell.
+// 4. A type 2 midpoint leaves children with a free gap opening at one corner
+//    (tb or te 0), which diff() also grants to a horizontal gap there. Such a
+//    path gains gapOpen over its true score, so it can only matter if it is
+//    within gapOpen of the optimum; the rows between the corner and the next
+//    saved row are computed over the columns of all paths that near, which tells
+//    whether one would tie or win (path_ask). A path that uses both of a frame's
+//    free corners gains twice, but parts from the optimal paths all the way
+//    between: not past a saved row where every path within 2 gapOpen goes
+//    through H of one cell (kPathTight). The few frames that are left, and those
+//    in boxes too wide for the slice, go to mm_align.
+//
+// Needs 0 <= gapOpen <= kMaxPathOpen and gapExtend >= 1: with a free extension
+// a gap at the box's corner would tie with the local optimum.
+#pragma once
+
+namespace cwgpu {
+
+constexpr int kMaxPathOpen = 1 << 26;
+constexpr int kPathLow = -(1 << 28);  // below every value of a cell on an optimal path
+constexpr int kPathRows = 4;          // rows per lane in the boxes
+constexpr int kMaxPathG = 4;          // rows between saved rows: 32 * 1, 2 or 4
+constexpr int kPathRing = 4;          // steps of forward values in flight
+
+// A row's cells on optimal paths: through H, inside a vertical gap (no kind at
+// all: the row's box was too wide).
+enum { kPathH = 1, kPathD = 2, kPathTight = 4 };
+
+// A warp's slice of the saved rows and of the working arrays below, for a pair
+// of n x m residues; fwd == nullptr when there is none.
+struct PathMem {
+    int every = 0;        // G
+    int2* fwd = nullptr;  // row i (i % G == 0, 0 < i < n): fwd + (i / G - 1) * stride, column j at [j]
+    int2* rev = nullptr;  // the same rows from reversePass, one above its values: column j at [se2 - j]
+    size_t stride = 0;
+    int2* cells = nullptr;  // forward values of the boxes in work
+    int cell_cap = 0;
+    int2* half = nullptr;  // two rows of n + m + 2 for the lanes' own halves
+    int4* span = nullptr;  // the saved rows' columns: of optimal paths (x, y), near (z, w)
+    int4* list = nullptr;  // frames left to mm_align, from the front; to ask for, from the back
+    int list_cap = 0;
+};
+
+// Bytes of a slice with rows every 32 * g, and its parts. The cells hold the
+// boxes a warp works on at a time, 64 columns wider than high: a wider box is
+// taken alone.
+__host__ __device__ inline size_t path_bytes(int n, int m, int g, PathMem* p = nullptr, unsigned char* base = nullptr) {
+    const int every = 32 * g;
+    const size_t saved = n > 0 ? (size_t)((n - 1) / every) * (size_t)(m + 1) : 0;
+    const size_t cells = (size_t)128 * ((m + 1 < every + 64 ? m + 1 : every + 64) + 8 * g);
+    const size_t half = 2 * (size_t)(n + m + 2), spans = (size_t)(n / every + 1);
+    if (p) {
+        p->every = every;
+        p->stride = (size_t)(m + 1);
+        p->cell_cap = (int)cells;
+        p->cells = reinterpret_cast<int2*>(base);
+        p->span = reinterpret_cast<int4*>(p->cells + cells);
+        p->list = p->span + spans;
+        p->list_cap = n + 1;
+        p->fwd = reinterpret_cast<int2*>(p->list + n + 1);
+        p->rev = p->fwd + saved;
+        p->half = p->rev + saved;
+    }
+    return 8 * (cells + 2 * spans + 2 * (size_t)(n + 1) + 2 * saved + half);
+}
+
+// The finest spacing whose slice fits `cap` bytes.
+__device__ __forceinline__ bool path_mem(int n, int m, unsigned char* base, size_t cap, PathMem& p) {
+    for (int g = 1; g <= kMaxPathG; g *= 2) {
+        if (path_bytes(n, m, g) <= cap) {
+            path_bytes(n, m, g, &p, base);
+            return true;
+        }
+    }
+    return false;
+}
+
+// A row's columns on optimal paths, relative to the box: first | last << 16,
+// and the kinds of its cells.
+__device__ __forceinline__ int2 path_entry(int lo, int hi, int kinds) { return make_int2(lo | (hi << 16), kinds); }
+__device__ __forceinline__ int path_lo(int2 v) { return v.x & 0xffff; }
+__device__ __forceinline__ int path_hi(int2 v) { return (int)((unsigned)v.x >> 16); }
+// Every optimal path goes through H of the row's one cell.
+__device__ __forceinline__ bool path_single(int2 v) {
+    return (v.y & (kPathH | kPathD)) == kPathH && path_lo(v) == path_hi(v);
+}
+
+// Columns of saved row i that optimal paths cross it in (lo..hi, kinds), and
+// those of paths within gapOpen of the optimum (near_lo..near_hi). kinds has
+// kPathTight if that is one cell, in H, also within 2 gapOpen. jl: the first
+// column any path within 2 gapOpen crosses the saved row above in, replaced by
+// this row's. At the pair's edges (column 0, column se2) a path has just started
+// or just ended: H 0 and, one above reversePass's -1, 0.
+__device__ __forceinline__ bool path_row(const PathMem& p, int i, int& jl, int se2, int best, int go, int& lo, int& hi,
+                                         int& kinds, int& near_lo, int& near_hi) {
+    const int lane = threadIdx.x & 31;
+    const int2* f = p.fwd + (size_t)(i / p.every - 1) * p.stride;
+    const int2* r = p.rev + (size_t)(i / p.every - 1) * p.stride + se2;
+    unsigned first = 0xffffffffu, nfirst = 0xffffffffu, wfirst = 0xffffffffu;
+    int last = -1, nlast = -1, k = 0, within = 0;
+    constexpr int U = 4;  // the rows come from DRAM: several loads in flight
+    for (int j0 = jl + lane; j0 <= se2; j0 += 32 * U) {
+        int2 a[U], b[U];
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            const int j = min(j0 + 32 * u, se2);
+            a[u] = __ldcg(f + max(j, 1));
+            b[u] = __ldcg(r - min(j, se2 - 1));
+            if (j == 0) a[u] = make_int2(0, kPathLow);
+            if (j == se2) b[u] = make_int2(0, kPathLow);
+        }
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            const int j = j0 + 32 * u;
+            const int vh = a[u].x + b[u].x - 1, vd = a[u].y + b[u].y - 1 + go;
+            if (max(vh, vd) < best - 2 * go || j > se2) continue;
+            within += 1 + (vd >= best - 2 * go);
+            wfirst = min(wfirst, (unsigned)j);
+            if (max(vh, vd) >= best - go) {
+                nfirst = min(nfirst, (unsigned)j);
+                nlast = j;
+                const int hit = (vh == best ? kPathH : 0) | (vd == best ? kPathD : 0);
+                if (hit) {
+                    first = min(first, (unsigned)j);
+                    last = j;
+                    k |= hit;
+                }
+            }
+        }
+    }
+    jl = (int)__reduce_min_sync(kFull, wfirst);
+    lo = (int)__reduce_min_sync(kFull, first);
+    hi = __reduce_max_sync(kFull, last);
+    near_lo = (int)__reduce_min_sync(kFull, nfirst);
+    near_hi = __reduce_max_sync(kFull, nlast);
+    kinds = (int)__reduce_or_sync(kFull, (unsigned)k);
+    if (kinds == kPathH && __reduce_add_sync(kFull, within) == 1) kinds |= kPathTight;
+    return hi >= 0;
+}
+
+// Shared memory of the boxes in work: the ring, the edge rows, the residues.
+constexpr int kPathRingWords = kPathRing * 64 * (int)sizeof(int4) / (int)sizeof(uint16_t);
+__device__ __forceinline__ int path_code_bytes(int width, int W) { return (width + 4 * W + 7) & ~7; }
+__device__ __forceinline__ int path_edge_bytes(int width, int W) { return 8 * width + path_code_bytes(width, W); }
+// Whether `used` boxes of W lanes and at most `width` columns fit the slice and
+// the warp's shared region.
+__device__ __forceinline__ bool path_fits(const PathMem& p, int used, int width, int W, int K) {
+    const int shared = kPathRingWords * (int)sizeof(uint16_t) + used * path_edge_bytes(width, W);
+    return used * (width + W) <= p.cell_cap / (W * kPathRows) && shared <= warp_region_bytes(K);
+}
+
+// 16 bytes from global to shared memory without passing through registers;
+// the lane that copied them reads them after the wait.
+__device__ __forceinline__ void copy_async16(int4* to, const int4* from) {
+#ifdef __CUDA_ARCH__
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((unsigned)__cvta_generic_to_shared(to)), "l"(from)
+                 : "memory");
+#else
+    *to = *from;
+#endif
+}
+__device__ __forceinline__ void copy_async_commit() {
+#ifdef __CUDA_ARCH__
+    asm volatile("cp.async.commit_group;" ::: "memory");
+#endif
+}
+template <int LEFT>
+__device__ __forceinline__ void copy_async_wait() {
+#ifdef __CUDA_ARCH__
+    asm volatile("cp.async.wait_group %0;" ::"n"(LEFT) : "memory");
+#endif
+}
+
+// Box b lies strictly between node rows i0 = max(A0, saved row) and i1 =
+// min(se1, next saved row): rows i0 + 1 .. i1 - 1, columns jl..jh of the optimal
+// paths.
+struct PathBox {
+    int i0, i1, jl, jh;
+};
+
+__device__ __forceinline__ PathBox path_box(const PathMem& p, int b, int nboxes, int A0, int B0, int se1, int se2) {
+    PathBox x;
+    const int base = A0 / p.every * p.every;
+    x.i0 = b == 0 ? A0 : base + b * p.every;
+    x.i1 = b == nboxes - 1 ? se1 : base + (b + 1) * p.every;
+    x.jl = b == 0 ? B0 : p.span[b - 1].x;
+    x.jh = b == nboxes - 1 ? se2 : p.span[b].y;
+    return x;
+}
+
+// Forward and reverse values of up to 32 / (p.every / 4) boxes at once, a
+// segment of p.every / 4 lanes each (box `mine`, -1: none), four rows per lane,
+// columns as a wavefront like the sweeps'. The row above (below) a box comes from the saved
+// forward (reverse) row, or is the box's own start (end) corner. Lane rows are
+// numbered so that a box's last row ends a lane: the first `pad` ones pass the
+// row above through, and a reverse lane's four rows are one forward lane's in
+// reverse order, two 16-byte words. Writes the rows' entries to band[i - A0];
+// false if a row has no cell on an optimal path. Bound by latency (one warp's
+// chain of steps), so the residues and the edge rows are in shared memory, and
+// the forward values come from L2 through a ring there, kPathRing - 1 steps
+// ahead.
+template <bool NC>
+__device__ __noinline__ bool path_boxes(const int8_t* s1, int n, const int8_t* s2, const PathMem& mem, int2* band, int A0, int B0,
+                           int se1, int se2, int mine, int width, int nboxes, int best, int go, int ge,
+                           const Env& env) {
+    const Env X = env;  // copies stay in registers across the stores below
+    const PathMem p = mem;
+    constexpr int R = kPathRows;
+    const int lane = threadIdx.x & 31, W = p.every / R, seg = lane / W, sl = lane & (W - 1);
+    const int goe = go + ge;
+    const PathBox x = path_box(p, max(mine, 0), nboxes, A0, B0, se1, se2);
+    const int ncols = mine >= 0 ? x.jh - x.jl + 1 : 1, nrows = mine >= 0 ? x.i1 - x.i0 - 1 : 0;
+    const int lanes = (nrows + R - 1) / R, pad = lanes * R - nrows;
+    const int nsteps = __reduce_max_sync(kFull, ncols + lanes - 1);
+    const int row_quads = R * W / 2;  // int4 words of one step: rows 0, 1 of every lane, then rows 2, 3
+    int4* const cells = reinterpret_cast<int4*>(p.cells) + seg * row_quads * (width + W);
+    const int* const smat = X.smat();
+    int4* const ring = reinterpret_cast<int4*>(X.region()) + lane;  // slot q: [64 q] and [64 q + 32]
+    int8_t* const own = reinterpret_cast<int8_t*>(X.region() + kPathRingWords) +
+                        (mine >= 0 ? seg : 0) * path_edge_bytes(width, W);
+    int2* const edge = reinterpret_cast<int2*>(own);
+    // Residues of columns jl - 1 .. jh, with 2 W more on either side.
+    int8_t* const codes = own + 8 * width + 2 * W;
+    const bool on = sl < lanes;
+    int hl[R], fp[R], mrow[R];
+    int diag = kPathLow, hout = kPathLow, eout = kPathLow;
+
+    // Forward: lane row r is node row i0 + 1 + r - pad, which consumes residue i0 + r - pad.
+    __syncwarp();
+    if (nrows > 0) {
+        const int2* top = p.fwd + (x.i0 == A0 ? 0 : (size_t)(x.i0 / p.every - 1) * p.stride);
+        for (int c = sl; c < ncols; c += W) {
+            int2 v = make_int2(x.i0 == A0 && x.jl + c == B0 ? 0 : kPathLow, kPathLow);
+            if (x.i0 != A0 && x.jl + c >= 1) v = __ldcg(top + x.jl + c);
+            edge[c] = v;
+        }
+        for (int c = sl - 2 * W; c < width + 2 * W; c += W)
+            codes[c] = c >= 0 && c <= ncols && x.jl - 1 + c >= 0 ? (int8_t)ldres<NC>(s2 + x.jl - 1 + c) : (int8_t)0;
+    }
+    __syncwarp();
+    const int own_pad = sl == 0 ? pad : 0;
+#pragma unroll
+    for (int k = 0; k < R; ++k) {
+        mrow[k] = 32 * ldres<NC>(s1 + max(0, min(x.i0 + R * sl + k - pad, n - 1)));
+        hl[k] = fp[k] = kPathLow;
+    }
+    int res = codes[-sl];  // of step t: codes[t - sl]
+    int4* out = cells + sl;
+    for (int t = 0; t < nsteps; ++t, out += row_quads) {
+        int hin = __shfl_up_sync(kFull, hout, 1, W);
+        int e = __shfl_up_sync(kFull, eout, 1, W);
+        const int2 above = edge[min(t, ncols - 1)];
+        if (sl == 0) {
+            hin = above.x;
+            e = __viaddmax_s32(above.y, -ge, above.x - goe);
+        }
+        const int b = res;
+        res = codes[t + 1 - sl];
+        if ((unsigned)(t - sl) < (unsigned)ncols && on) {
+            int d = diag, hup = hin, v[2 * R];
+#pragma unroll
+            for (int k = 0; k < R; ++k) {
+                int h = __vimax3_s32(e, fp[k], d + smat[mrow[k] + b]);
+                const int g = h - goe;
+                const bool real = k >= own_pad;
+                v[2 * k + 1] = e;
+                fp[k] = __viaddmax_s32(fp[k], -ge, g);
+                const int en = __viaddmax_s32(e, -ge, g);
+                e = real ? en : e;
+                h = real ? h : hup;
+                d = hl[k];
+                hl[k] = hup = h;
+                v[2 * k] = h;
+            }
+            diag = hin;
+            hout = hup;
+            eout = e;
+            __stcg(out, make_int4(v[0], v[1], v[2], v[3]));
+            __stcg(out + W, make_int4(v[4], v[5], v[6], v[7]));
+        }
+    }
+
+    // Reverse: lane row r is node row i1 - 1 - r, which consumes residue i1 - 1 - r.
+    __syncwarp();
+    if (nrows > 0) {
+        const int2* bottom = p.rev + (x.i1 == se1 ? 0 : (size_t)(x.i1 / p.every - 1) * p.stride) + se2;
+        for (int c = sl; c < ncols; c += W) {
+            int2 v = make_int2(x.i1 == se1 && x.jl + c == se2 ? 0 : kPathLow, kPathLow);
+            if (x.i1 != se1 && x.jl + c < se2) {
+                v = __ldcg(bottom - (x.jl + c));
+                v.x -= 1;
+                v.y -= 1;
+            }
+            edge[c] = v;
+        }
+    }
+    __syncwarp();
+    int span[R];  // columns with a cell on an optimal path, from jl: first | last << 16; 0xffff: none
+    unsigned kinds = 0;  // four bits per row
+#pragma unroll
+    for (int k = 0; k < R; ++k) {
+        mrow[k] = 32 * ldres<NC>(s1 + max(x.i1 - 1 - (R * sl + k), 0));
+        hl[k] = fp[k] = kPathLow;
+        span[k] = 0xffff;
+    }
+    diag = hout = eout = kPathLow;
+    const int8_t* const back = codes + ncols + sl;  // residue of step t: back[-t]
+    res = back[0];
+    // Column jh - (t - sl) of forward lane lanes - 1 - sl: step ncols - 1 - (t - sl) + that lane's delay.
+    const int4* in = cells + (size_t)(on ? ncols + lanes - 2 : 0) * row_quads + (on ? lanes - 1 - sl : 0);
+    // Step t's words go to slot t % kPathRing; every step starts one copy
+    // (maybe of nothing), so step t's has landed when all but the last
+    // kPathRing - 1 have.
+    auto fetch = [&](int t) {
+        if ((unsigned)(t - sl) < (unsigned)ncols && on) {
+            int4* slot = ring + 64 * (t & (kPathRing - 1));
+            const int4* from = in - (ptrdiff_t)t * row_quads;
+            copy_async16(slot, from);
+            copy_async16(slot + 32, from + W);
+        }
+        copy_async_commit();
+    };
+#pragma unroll
+    for (int t = 0; t < kPathRing - 1; ++t) fetch(t);
+    for (int t = 0; t < nsteps; ++t) {
+        int hin = __shfl_up_sync(kFull, hout, 1, W);
+        int e = __shfl_up_sync(kFull, eout, 1, W);
+        const int2 below = edge[max(ncols - 1 - t, 0)];
+        if (sl == 0) {
+            hin = below.x;
+            e = __viaddmax_s32(below.y, -ge, below.x - goe);
+        }
+        const int b = res;
+        res = back[-t - 1];
+        const int c = t - sl;
+        fetch(t + kPathRing - 1);
+        copy_async_wait<kPathRing - 1>();
+        if ((unsigned)c < (unsigned)ncols && on) {
+            const int4 nlo = ring[64 * (t & (kPathRing - 1))], nhi = ring[64 * (t & (kPathRing - 1)) + 32];
+            const int fh[R] = {nhi.z, nhi.x, nlo.z, nlo.x}, fe[R] = {nhi.w, nhi.y, nlo.w, nlo.y};
+            int d = diag;
+#pragma unroll
+            for (int k = 0; k < R; ++k) {
+                const int f = fp[k];
+                const int h = __vimax3_s32(e, f, d + smat[mrow[k] + b]);
+                const int g = h - goe;
+                d = hl[k];
+                hl[k] = h;
+                const int vh = fh[k] + h, vd = fe[k] + e + go;
+                if (max(vh, vd) == best && R * sl + k < nrows) {
+                    const int col = ncols - 1 - c;
+                    span[k] = col | (span[k] == 0xffff ? col << 16 : span[k] & 0xffff0000);
+                    kinds |= ((vh == best ? kPathH : 0) | (vd == best ? kPathD : 0)) << (4 * k);
+                }
+                fp[k] = __viaddmax_s32(f, -ge, g);
+                e = __viaddmax_s32(e, -ge, g);
+            }
+            diag = hin;
+            hout = hl[R - 1];
+            eout = e;
+        }
+    }
+    bool ok = true;
+#pragma unroll
+    for (int k = 0; k < R; ++k) {
+        const int r = R * sl + k;
+        if (r >= nrows) continue;
+        const int lo = span[k] & 0xffff, hi = (int)((unsigned)span[k] >> 16);
+        ok = ok && lo != 0xffff;
+        band[x.i1 - 1 - r - A0] =
+            path_entry(lo + x.jl - B0, hi + x.jl - B0, (kinds >> (4 * k)) & 15);
+    }
+    __syncwarp();
+    return __all_sync(kFull, ok);
+}
+
+// The entries of all rows of the pair's box; false if some row has no cell on
+// an optimal path, or the boxes cost more than they save, and the caller runs
+// mm_align.
+template <bool NC>
+__device__ __noinline__ bool path_band(const int8_t* s1, int n, const int8_t* s2, const PathMem& mem, int2* band, int A0, int B0,
+                          int se1, int se2, int best, int go, int ge, const Env& env) {
+    const Env X = env;  // copies stay in registers across the stores below
+    const PathMem p = mem;
+    const int lane = threadIdx.x & 31;
+    if (lane == 0) {
+        band[0] = path_entry(0, 0, kPathH);
+        band[se1 - A0] = path_entry(se2 - B0, se2 - B0, kPathH);
+    }
+    const int base = A0 / p.every;
+    const int nboxes = (se1 - 1) / p.every - base + 1;
+    for (int b = 0, jl = B0; b + 1 < nboxes; ++b) {
+        const int i = (base + b + 1) * p.every;
+        int lo, hi, kinds, near_lo, near_hi;
+        if (!path_row(p, i, jl, se2, best, go, lo, hi, kinds, near_lo, near_hi)) return false;
+        if (lane == 0) {
+            band[i - A0] = path_entry(lo - B0, hi - B0, kinds);
+            p.span[b] = make_int4(lo, hi, near_lo, near_hi);
+        }
+    }
+    __syncwarp();
+    // A column of boxes costs about four steps of a sweep; mm_align's steps are
+    // about a 96th of the pair's box, and a few per row for the small frames.
+    const int W = p.every / kPathRows, seg = lane / W;
+    int left = (int)min((long long)(se1 - A0) * (se2 - B0) / 384 + (se1 - A0), (long long)INT_MAX);
+    for (int b = 0; b < nboxes;) {
+        // As many boxes as the slice and the shared edge rows hold.
+        int used = 0, width = 0, mine = -1;
+        while (used * W < 32 && b + used < nboxes) {
+            const PathBox x = path_box(p, b + used, nboxes, A0, B0, se1, se2);
+            const int w = max(width, x.jh - x.jl + 1);
+            if (!path_fits(p, used + 1, w, W, X.K)) break;
+            if (seg == used) mine = b + used;
+            width = w;
+            ++used;
+        }
+        left -= width + W;
+        if (left < 0) return false;
+        if (used == 0) {
+            const PathBox x = path_box(p, b, nboxes, A0, B0, se1, se2);
+            for (int i = x.i0 + 1 + lane; i < x.i1; i += 32) band[i - A0] = path_entry(0, 0, 0);
+            ++b;
+            continue;
+        }
+        if (!path_boxes<NC>(s1, n, s2, p, band, A0, B0, se1, se2, mine, width, nboxes, best, go, ge, X))
+            return false;
+        b += used;
+    }
+    __syncwarp();
+    return true;
+}
+
+// One lane: diff()'s two halves of frame (A, B, M, N) at row r = A + M / 2 over
+// the rows' column ranges, and its midpoint scans (:570-593). All coordinates
+// are relative to the box; s1/s2 point at its first residues. Cells outside the
+// ranges are on no optimal path and only ever lose to those inside.
+template <bool NC>
+__device__ void path_midpoint(const int8_t* s1, const int8_t* s2, const int2* band, int2* half, size_t half_stride,
+                              int A, int B, int M, int N, int tb, int te, int go, int ge, const Env& X, int& midj,
+                              bool& type2) {
+    const int goe = go + ge, r = A + M / 2;
+    int2* F = half + A;  // column j at F[j], j = B..B + N: words no other frame of the walk uses
+    int2* Rv = F + half_stride;
+    // forward half, from the last single row above r
+    int q = r - 1;
+    while (q > A && !path_single(band[q])) --q;
+    int lo, hi;
+    if (q > A) {
+        lo = hi = path_lo(band[q]);
+        F[lo] = make_int2(0, -go);
+    } else {
+        q = A;
+        lo = B;
+        hi = min(path_hi(band[A]), B + N);
+        F[B] = make_int2(0, -tb);
+        for (int j = B + 1; j <= hi; ++j) F[j] = make_int2(-tb - ge * (j - B), -tb - ge * (j - B) - go);
+    }
+    const int first = lo;
+    for (; q < r; ++q) {
+        const int2 v = band[q + 1];
+        const int nlo = max(path_lo(v), first), nhi = min(path_hi(v), B + N);
+        const int* row = X.smat() + 32 * ldres<NC>(s1 + q);
+        int diag = nlo - 1 >= lo && nlo - 1 <= hi ? F[nlo - 1].x : kPathLow;
+        int f = kPathLow;
+        for (int j = nlo; j <= nhi; ++j) {
+            const int2 up = j >= lo && j <= hi ? F[j] : make_int2(kPathLow, kPathLow);
+            const int e = __viaddmax_s32(up.y, -ge, up.x - goe);
+            const int s = j > 0 ? row[ldres<NC>(s2 + j - 1)] : kPadScore;
+            const int h = __vimax3_s32(e, f, diag + s);
+            f = __viaddmax_s32(f, -ge, h - goe);
+            diag = up.x;
+            F[j] = make_int2(h, e);
+        }
+        lo = nlo;
+        hi = nhi;
+    }
+    const int flo = lo, fhi = hi;
+    // reverse half, from the first single row below r
+    q = r + 1;
+    while (q < A + M && !path_single(band[q])) ++q;
+    if (q < A + M) {
+        lo = hi = path_lo(band[q]);
+        Rv[lo] = make_int2(0, -go);
+    } else {
+        q = A + M;
+        hi = B + N;
+        lo = max(path_lo(band[q]), B);
+        Rv[hi] = make_int2(0, -te);
+        for (int j = hi - 1; j >= lo; --j) Rv[j] = make_int2(-te - ge * (hi - j), -te - ge * (hi - j) - go);
+    }
+    const int lastc = hi;
+    for (; q > r; --q) {
+        const int2 v = band[q - 1];
+        const int nlo = max(path_lo(v), B), nhi = min(path_hi(v), lastc);
+        const int* row = X.smat() + 32 * ldres<NC>(s1 + q - 1);
+        int diag = nhi + 1 >= lo && nhi + 1 <= hi ? Rv[nhi + 1].x : kPathLow;
+        int f = kPathLow;
+        for (int j = nhi; j >= nlo; --j) {
+            const int2 dn = j >= lo && j <= hi ? Rv[j] : make_int2(kPathLow, kPathLow);
+            const int e = __viaddmax_s32(dn.y, -ge, dn.x - goe);
+            const int h = __vimax3_s32(e, f, diag + row[ldres<NC>(s2 + j)]);
+            f = __viaddmax_s32(f, -ge, h - goe);
+            diag = dn.x;
+            Rv[j] = make_int2(h, e);
+        }
+        lo = nlo;
+        hi = nhi;
+    }
+    lo = max(lo, flo);
+    hi = min(hi, fhi);
+    int midh = INT_MIN;
+    midj = lo;
+    type2 = false;
+    for (int j = lo; j <= hi; ++j) {
+        const int2 a = F[j], b = Rv[j];
+        const int hh = a.x + b.x;
+        if (hh >= midh && (hh > midh || (a.x != a.y && b.x == b.y))) {
+            midh = hh;
+            midj = j;
+        }
+    }
+    for (int j = hi; j >= lo; --j) {
+        const int hh = F[j].y + Rv[j].y + go;
+        if (hh > midh) {
+            midh = hh;
+            midj = j;
+            type2 = true;
+        }
+    }
+    midj -= B;
+}
+
+// Whether a tight row lies strictly inside rows A .. A + M of the box.
+__device__ __forceinline__ bool path_tight(const int2* band, int A, int M, int A0, int every) {
+    for (int i = ((A0 + A) / every + 1) * every - A0; i < A + M; i += every)
+        if (band[i].y & kPathTight) return true;
+    return false;
+}
+
+// Up to 32 / (p.every / 4) of the last frames asked for, a segment of lanes each
+// like the boxes': those whose free corner no horizontal gap can use go to the
+// stack, the others to the list. For a frame that starts at its free corner
+// (r, c): the rows between the next saved row and r, over the columns from c to
+// the last a path within gapOpen of the optimum crosses that row in; the gap
+// can be used if the best value right of c, less its extension, reaches the
+// corner's own. A frame that ends at its free corner: the same mirrored, from
+// the saved row above. Lane row t is t + 1 rows from the saved row.
+template <bool NC>
+__device__ void path_ask(const int8_t* s1, int n, const int8_t* s2, int m, const PathMem& p, int A0, int B0, int se1,
+                         int se2, int go, int ge, const Env& X, int4* stack, int& sp, int& nlist, int& nask) {
+    constexpr int R = kPathRows;
+    const int lane = threadIdx.x & 31, W = p.every / R, seg = lane / W, sl = lane & (W - 1);
+    const int goe = go + ge;
+    const int* const smat = X.smat();
+    const int take = min(32 / W, nask);
+    const int base = A0 / p.every;
+    int4 f = p.list[p.list_cap - nask + min(seg, take - 1)];
+    const bool end = (f.z >> 30) & 1;
+    f.z &= (1 << 30) - 1;
+    const int dir = end ? -1 : 1;  // from the corner to the saved row
+    const int r = end ? f.x + f.z : f.x, c = end ? f.y + (f.w & ((1 << 29) - 1)) : f.y;
+    const int i = end ? max(A0, (r - 1) / p.every * p.every) : min(se1, (r / p.every + 1) * p.every);
+    const bool corner = end ? i == A0 : i == se1;
+    const int4 span = corner ? make_int4(0, 0, B0, se2) : p.span[i / p.every - base - 1];
+    // The frame's other corner may be the pair's own, where diff() opens gaps
+    // free as well: a path may then run along the box's edge before it reaches
+    // the saved row, in any column, which is no better than ending (starting)
+    // where it does, at reversePass's -1 (forwardPass's 0).
+    const bool loose = end ? f.x == A0 && !((f.w >> 29) & 1) : f.x + f.z == se1 && !((f.w >> 30) & 1);
+    const int floor = !loose ? 2 * kPathLow : end ? 0 : -1;
+    const int far = loose ? (end ? B0 : se2) : (end ? span.z : span.w);
+    const int nrows = dir * (i - r), ncols = dir * (far - c) + 1, lanes = (nrows + R - 1) / R;
+    const int nsteps = __reduce_max_sync(kFull, seg < take ? ncols + lanes - 1 : 0);
+    const bool on = seg < take && sl < lanes;
+    const int2* saved = corner ? p.fwd : (end ? p.fwd : p.rev + se2) + (size_t)(i / p.every - 1) * p.stride;
+    int hl[R], fp[R], mrow[R];
+#pragma unroll
+    for (int k = 0; k < R; ++k) {
+        // Lane row t lies across residue i - 1 - t (below the corner's row: i + t).
+        const int at = end ? i + R * sl + k : i - 1 - (R * sl + k);
+        mrow[k] = 32 * ldres<NC>(s1 + max(0, min(at, n - 1)));
+        hl[k] = fp[k] = kPathLow;
+    }
+    int diag = kPathLow, hout = kPathLow, eout = kPathLow, v = kPathLow;
+    bool bad = false;
+    for (int t = 0; t < nsteps; ++t) {
+        int hin = __shfl_up_sync(kFull, hout, 1, W);
+        int e = __shfl_up_sync(kFull, eout, 1, W);
+        const int q = t - sl, j = far - dir * q;  // node column
+        const bool in = (unsigned)q < (unsigned)ncols && on;
+        if (in) {
+            if (sl == 0) {
+                int2 a = make_int2(kPathLow, kPathLow);
+                if (corner) {
+                    if (q == 0) a.x = 0;
+                } else if (end ? j >= 1 : j < se2) {
+                    a = __ldcg(end ? saved + j : saved - j);
+                    if (!end) a = make_int2(a.x - 1, a.y - 1);
+                }
+                hin = max(a.x, floor);
+                e = __viaddmax_s32(a.y, -ge, hin - goe);
+            }
+            const int b = ldres<NC>(s2 + max(0, min(end ? j - 1 : j, m - 1)));
+            int d = diag;
+#pragma unroll
+            for (int k = 0; k < R; ++k) {
+                const int before = hl[k];
+                const int h = max(__vimax3_s32(e, fp[k], d + smat[mrow[k] + b]), floor);
+                const int g = h - goe;
+                if (R * sl + k == nrows - 1) {
+                    v = max(v, before) - ge;
+                    if (q == ncols - 1) bad = v >= max(e + go, h);
+                }
+                d = before;
+                hl[k] = h;
+                fp[k] = __viaddmax_s32(fp[k], -ge, g);
+                e = __viaddmax_s32(e, -ge, g);
+            }
+            diag = hin;
+            hout = hl[R - 1];
+            eout = e;
+        }
+    }
+    const unsigned hits = __ballot_sync(kFull, bad);
+    const bool head = sl == 0 && seg < take, listed = (hits >> (seg * W)) & (W == 32 ? kFull : (1u << W) - 1);
+    const unsigned below = (1u << lane) - 1;
+    const unsigned to_stack = __ballot_sync(kFull, head && !listed), to_list = __ballot_sync(kFull, head && listed);
+    if (head && !listed) stack[sp + __popc(to_stack & below)] = make_int4(f.x - A0, f.y - B0, f.z, f.w);
+    if (head && listed) p.list[nlist + __popc(to_list & below)] = f;
+    sp += __popc(to_stack);
+    nlist += __popc(to_list);
+    nask -= take;
+    __syncwarp();
+}
+
+// Whether one lane's halves of frame (A, M) would visit a row of a box left
+// out, or more cells than mm_align's steps are worth (a 53rd of the frame, and
+// some).
+__device__ inline bool path_too_wide(const int2* band, int A, int M, int N) {
+    const int r = A + M / 2;
+    int cells = path_hi(band[r]) - path_lo(band[r]) + 1;
+    bool known = band[r].y != 0;
+    const int most = (int)min((long long)M * N / 53 + 400, (long long)INT_MAX);
+    for (int q = r - 1; q > A && !path_single(band[q]) && cells <= most && known; --q) {
+        cells += path_hi(band[q]) - path_lo(band[q]) + 1;
+        known = band[q].y != 0;
+    }
+    for (int q = r + 1; q < A + M && !path_single(band[q]) && cells <= most && known; ++q) {
+        cells += path_hi(band[q]) - path_lo(band[q]) + 1;
+        known = band[q].y != 0;
+    }
+    return cells > most || !known;
+}
+
+// Walks diff()'s frames from the box's own, 32 at a time. Adds identities,
+// matches and inner-loop iterations; frames left to mm_align go to p.list
+// (count returned).
+template <bool NC>
+__device__ __noinline__ int path_walk(const int8_t* s1, int n, const int8_t* s2, int m, const PathMem& mem, const int2* band,
+                                      int A0, int B0, int se1, int se2, int go, int ge, const Env& env,
+                                      int& n_ident, int& n_match, long long& n_cells) {
+    const Env X = env;  // copies stay in registers across the stores below
+    const PathMem p = mem;
+    const int M0 = se1 - A0, N0 = se2 - B0;
+    const int8_t* const seq1 = s1;
+    const int8_t* const seq2 = s2;
+    s1 += A0;
+    s2 += B0;
+    const int lane = threadIdx.x & 31;
+    constexpr int NMASK = (1 << 29) - 1;
+    int4* stack = reinterpret_cast<int4*>(X.region());
+    const int cap = warp_region_bytes(X.K) / (int)sizeof(int4);
+    const size_t half_stride = (size_t)(n + m + 2);
+    int ident = 0, match = 0, nlist = 0, nask = 0;
+    long long cells = 0;
+    __syncwarp();
+    if (lane == 0) stack[0] = make_int4(0, 0, M0, N0);
+    __syncwarp();
+    int sp = 1;
+    for (;;) {
+        if (sp == 0) {
+            if (nask == 0) break;
+            while (nask > 0) path_ask<NC>(seq1, n, seq2, m, p, A0, B0, se1, se2, go, ge, X, stack, sp, nlist, nask);
+            continue;
+        }
+        // Taking one frame at a time grows the stack by at most the depth of
+        // the recursion (17), so near its end the walk goes depth first.
+        const int take = sp > cap - 96 ? 1 : min(32, sp);
+        int4 fr = make_int4(0, 0, 0, 0);
+        if (lane < take) fr = stack[sp - 1 - lane];
+        sp -= take;
+        __syncwarp();
+        int4 kid[2];
+        int kind[2] = {0, 0};  // 0: nothing to do, 1: to the stack, 2: to the list, 3: to ask for
+        const int A = fr.x, B = fr.y, M = fr.z, N = fr.w & NMASK;
+        const int tbf = (fr.w >> 29) & 1, tef = (fr.w >> 30) & 1;
+        const int tb = tbf ? go : 0, te = tef ? go : 0;
+        if (lane < take && M == 1) {
+            cells += N;
+            int midh = -(tb + ge) - (te + ge * N);
+            const int hh0 = -(te + ge) - (tb + ge * N);
+            midh = max(midh, hh0);
+            const int2 u = band[A], v = band[A + 1];
+            const int ra = ldres<NC>(s1 + A);
+            const int* row = X.smat() + 32 * ra;
+            int at = 0, rb = 0;
+            const int j1 = min(N, min(path_hi(u) + 1, path_hi(v)) - B);
+            for (int j = max(1, max(path_lo(u) + 1, path_lo(v)) - B); j <= j1; ++j) {
+                const int b = ldres<NC>(s2 + B + j - 1);
+                const int hh = row[b] - (N - j > 0 ? te + ge * (N - j) : 0) - (j - 1 > 0 ? tb + ge * (j - 1) : 0);
+                if (hh > midh) {
+                    midh = hh;
+                    at = j;
+                    rb = b;
+                }
+            }
+            if (at > 0) {
+                ++match;
+                if (ra != X.gp1 && rb != X.gp2 && ra == rb) ++ident;
+            }
+        } else if (lane < take) {
+            const int midi = M / 2;
+            const int2 v = band[A + midi];
+            int midj = path_lo(v) - B;
+            const int kinds = v.y & (kPathH | kPathD);
+            bool type2 = kinds == kPathD;
+            const bool open = kinds == 0 || kinds == (kPathH | kPathD) || path_lo(v) != path_hi(v);
+            if (open && path_too_wide(band, A, M, N)) {
+                kid[0] = fr;
+                kind[0] = 2;
+            } else {
+                cells += (long long)M * N;
+                if (open)
+                    path_midpoint<NC>(s1, s2, band, p.half, half_stride, A, B, M, N, tb, te, go, ge, X, midj, type2);
+                if (!type2) {
+                    kid[0] = make_int4(A + midi, B + midj, M - midi, (N - midj) | (1 << 29) | (tef << 30));
+                    kid[1] = make_int4(A, B, midi, midj | (tbf << 29) | (1 << 30));
+                } else {
+                    kid[0] = make_int4(A + midi + 1, B + midj, M - midi - 1, (N - midj) | (tef << 30));
+                    kid[1] = make_int4(A, B, midi - 1, midj | (tbf << 29));
+                }
+#pragma unroll
+                for (int c = 0; c < 2; ++c) {
+                    if (kid[c].z > 0 && (kid[c].w & NMASK) > 0) kind[c] = 1;
+                }
+                if (type2) {
+                    // Free openings inside the box: at kid 0's start and kid 1's end,
+                    // and maybe already at their other corners.
+                    if (kind[0])
+                        kind[0] = tef == 0 && A + M < M0 && !path_tight(band, kid[0].x, kid[0].z, A0, p.every) ? 2 : 3;
+                    if (kind[1])
+                        kind[1] = tbf == 0 && A > 0 && !path_tight(band, kid[1].x, kid[1].z, A0, p.every) ? 2 : 3;
+                }
+            }
+        }
+#pragma unroll
+        for (int c = 0; c < 2; ++c) {
+            const unsigned below = (1u << lane) - 1;
+            const unsigned on = __ballot_sync(kFull, kind[c] == 1), off = __ballot_sync(kFull, kind[c] == 2);
+            const unsigned ask = __ballot_sync(kFull, kind[c] == 3);
+            if (kind[c] == 1) stack[sp + __popc(on & below)] = kid[c];
+            if (kind[c] == 2)
+                p.list[nlist + __popc(off & below)] = make_int4(kid[c].x + A0, kid[c].y + B0, kid[c].z, kid[c].w);
+            // Absolute rows and columns in both, the kid's number with the ones to ask for.
+            if (kind[c] == 3)
+                p.list[p.list_cap - 1 - nask - __popc(ask & below)] =
+                    make_int4(kid[c].x + A0, kid[c].y + B0, kid[c].z | c << 30, kid[c].w);
+            sp += __popc(on);
+            nlist += __popc(off);
+            nask += __popc(ask);
+        }
+        __syncwarp();
+    }
+    n_ident += __reduce_add_sync(kFull, ident);
+    n_match += __reduce_add_sync(kFull, match);
+    for (int d = 16; d; d >>= 1) cells += __shfl_xor_sync(kFull, cells, d);
+    n_cells += cells;
+    return nlist;
+}
+
+}  // namespace cwgpu

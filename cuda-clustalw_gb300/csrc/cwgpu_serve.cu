@@ -469,6 +469,9 @@ int launch_round(cwgpu_server* s, int ri, int64_t nitems) {
         gl.tiny_m = 32;
         gl.tiny_n = cwgpu::kTinyMaxN;
         gl.general = s->general_gaps;
+        gl.path = nullptr;
+        gl.path_bytes = 0;
+        gl.path_slots = 0;
         cwgpu::PairArgs gs = gl;
         gs.order = gl.order + r.nlong;
         gs.npairs = r.n - r.nlong;
