@@ -155,6 +155,8 @@ struct CtaCtl {
     int ident[kCtaMaxWarps], match[kCtaMaxWarps];
     int mm;  // diff()'s score of the pair
     int nstack, nsmall, small_next;
+    int path_bad;                  // a warp found the path cannot be had from the kept rows
+    int path_rest[kCtaMaxWarps];   // frames each warp leaves to diff()'s divisions
     int lock, active;  // the shared frame stack `small`: its lock, warps holding a frame from it
     int4 stack[kCtaStack];  // large frames: (A, B, M | root, N | tb << 29 | te << 30)
     int4 small[kCtaSmall];  // frames for one warp each
@@ -163,6 +165,7 @@ struct CtaCtl {
 struct CtaArgs {
     int large_rows;
     unsigned long long limit_ns;
+    size_t path_bytes;  // of a CTA's slice of PairArgs::path
 };
 
 // Maximum value, then lowest key, over the warps' results in C.
@@ -273,12 +276,13 @@ __device__ void cta_small_frames(CtaCtl& C, const int8_t* s1, const int8_t* s1r,
     __syncthreads();
 }
 
-// diff() + tracePath of one pair by the whole CTA (every thread calls).
+// diff() + tracePath of one pair by the whole CTA (every thread calls), or, if
+// `list` is given, of its nlist frames only (no score).
 template <int RS, bool GEN>
 __device__ void cta_diff(CtaCtl& C, const int8_t* s1, const int8_t* s1r, int n, const int8_t* s2, const int8_t* s2r,
                          int m, int A0, int B0, int M0, int N0, int go, int ge, int2* bufs, size_t stride, int nw,
                          const cwgpu::Env& X, cwgpu::MwSync& mw, unsigned long long& epoch, const CtaArgs& ca,
-                         int& mm_score, int& n_ident, int& n_match, long long& cells) {
+                         int& mm_score, int& n_ident, int& n_match, long long& cells, const int4* list, int nlist) {
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     int2* bufA = bufs + (size_t)warp * stride;
     int2* bufB = bufA + stride / 2;
@@ -292,16 +296,36 @@ __device__ void cta_diff(CtaCtl& C, const int8_t* s1, const int8_t* s1r, int n, 
         C.nstack = 0;
         C.nsmall = 0;
         C.mm = 0;
-        const int4 root = make_int4(A0, B0, M0 | kRootBit, N0);
-        if (cta_large(M0, N0, large_rows))
-            C.stack[C.nstack++] = root;
-        else
-            C.small[C.nsmall++] = root;
+        if (!list) {
+            const int4 root = make_int4(A0, B0, M0 | kRootBit, N0);
+            if (cta_large(M0, N0, large_rows))
+                C.stack[C.nstack++] = root;
+            else
+                C.small[C.nsmall++] = root;
+        }
     }
     __syncthreads();
-    for (;;) {
+    for (int next = 0;;) {
         const int ns = C.nstack;
-        if (ns == 0) break;
+        if (ns == 0) {
+            if (!list || next >= nlist) break;
+            __syncthreads();  // every thread has seen the empty stack before it is filled
+            const int upto = min(nlist, next + kCtaStack / 2);
+            if (threadIdx.x == 0) {
+                for (int k = next; k < upto; ++k) {
+                    if (cta_large(list[k].z, list[k].w & ((1 << 29) - 1), large_rows))
+                        C.stack[C.nstack++] = list[k];
+                    else
+                        C.small[C.nsmall++] = list[k];
+                }
+            }
+            next = upto;
+            __syncthreads();
+            if (C.nsmall > kCtaSmall - kCtaStack)
+                cta_small_frames<RS, GEN>(C, s1, s1r, n, s2, s2r, m, go, ge, bufA, bufB, X, ca, ident, match, ncell);
+            __syncthreads();
+            continue;
+        }
         // One large frame by the whole CTA, or, when two are waiting, both at
         // once: frame f on warps [f * nw / 2, (f + 1) * nw / 2), forward half
         // on the first half of those warps, reverse half on the second.
@@ -426,6 +450,10 @@ __device__ void cta_pair(const cwgpu::PairArgs& g, long long q, CtaCtl& C, const
         int max_score = 0, se1 = 0, se2 = 0, sb1 = 1, sb2 = 1;
         cwgpu::Best rb;
         cwgpu::Task t = cwgpu::local_task(s1, n, s2, m, go, nullptr);
+        cwgpu::PathMem pm;
+        const bool path = !GEN && g.path && ge >= 1 && go <= cwgpu::kMaxPathOpen &&
+                          cwgpu::path_mem(n, m, nw, g.path + (size_t)blockIdx.x * ca.path_bytes, ca.path_bytes, pm);
+        cwgpu::RowSave save{path ? pm.fwd : nullptr, pm.stride, pm.every, 0, 1, n};
 #pragma unroll 1
         for (int pass = 0; pass < 2; ++pass) {
             __syncthreads();
@@ -439,7 +467,7 @@ __device__ void cta_pair(const cwgpu::PairArgs& g, long long q, CtaCtl& C, const
             else
                 cwgpu::sweep_mw<RS, cwgpu::MODE_LOCAL_FWD, GEN>(t, go, ge, pass ? max_score + 1 : 1,
                                                                pass ? max_score + 1 : INT_MAX, X, b, bufs, stride, 0,
-                                                               warp, nw, mw, &C.stop);
+                                                               warp, nw, mw, &C.stop, save);
             if (lane == 0) {
                 C.bval[warp] = b.val;
                 C.bkey[warp] = b.key;
@@ -452,6 +480,7 @@ __device__ void cta_pair(const cwgpu::PairArgs& g, long long q, CtaCtl& C, const
                 se1 = (int)(rb.key >> 16) + 1;
                 se2 = (int)(rb.key & 0xffffu);
                 t = cwgpu::reverse_task<RS, GEN>(s1r, n, se1, s2r, m, se2, go, nullptr);
+                save = cwgpu::RowSave{path ? pm.rev : nullptr, pm.stride, pm.every, se1, -1, se1};
             } else if (!GEN) {
                 rb.val -= 1;
             }
@@ -471,8 +500,63 @@ __device__ void cta_pair(const cwgpu::PairArgs& g, long long q, CtaCtl& C, const
         // diff + tracePath
         int mm = 0, ident = 0, matches = 0;
         long long dcells = 0;
-        cta_diff<RS, GEN>(C, s1, s1r, n, s2, s2r, m, sb1 - 1, sb2 - 1, se1 - sb1 + 1, se2 - sb2 + 1, go, ge, bufs, stride,
-                     nw, X, mw, epoch, ca, mm, ident, matches, dcells);
+        const int A0 = sb1 - 1, B0 = sb2 - 1;
+        int rest = -1;  // frames left to diff()'s divisions; -1: the pair's own
+        if constexpr (!GEN) {
+            // The path from the kept rows (cwgpu_path.cuh): rows, boxes and the
+            // walk's frames dealt over the warps. Against diff()'s divisions by
+            // the whole CTA: one column of 100 DNA sequences of 1523 residues
+            // 1.95 to 1.6 ms, the 15 pairs of six proteins of 3000 3.9 to 2.8
+            // to 3.5 ms (by family).
+            if (path && max_score > 0) {
+                int2* const band = bufs + stride / 2;  // of warp 0: no sweep uses it
+                const cwgpu::PathMem own = cwgpu::path_of_warp(pm, warp);
+                if (threadIdx.x == 0) C.path_bad = 0;
+                __syncthreads();
+                if (!cwgpu::path_rows(pm, band, A0, B0, se1, se2, max_score, go, warp, nw)) C.path_bad = 1;
+                __syncthreads();
+                if (!C.path_bad && !cwgpu::path_fill<true, true>(s1, n, s2, own, band, A0, B0, se1, se2, max_score, go, ge, X,
+                                                           warp, nw))
+                    C.path_bad = 1;
+                __syncthreads();
+                if (!C.path_bad) {
+                    int id = 0, mt = 0;
+                    long long ce = 0;
+                    const int r = cwgpu::path_walk<true, true>(s1, n, s2, m, own, band, A0, B0, se1, se2, go, ge, X, id, mt, ce,
+                                                         warp, nw);
+                    if (lane == 0) {
+                        C.ident[warp] = id;
+                        C.match[warp] = mt;
+                        C.dcells[warp] = ce;
+                        C.path_rest[warp] = r;
+                    }
+                    __syncthreads();
+                    // The warps' lists behind one another: no more frames than rows.
+                    rest = 0;
+                    for (int w = 0; w < nw; ++w) {
+                        const int4* from = pm.list + (size_t)w * pm.list_cap;
+                        if (w > 0 && threadIdx.x == 0)
+                            for (int k = 0; k < C.path_rest[w]; ++k) pm.list[rest + k] = from[k];
+                        rest += C.path_rest[w];
+                        ident += C.ident[w];
+                        matches += C.match[w];
+                        dcells += C.dcells[w];
+                    }
+                    mm = max_score;
+                    __syncthreads();
+                }
+            }
+        }
+        if (rest != 0) {
+            int id = 0, mt = 0, score = 0;
+            long long ce = 0;
+            cta_diff<RS, GEN>(C, s1, s1r, n, s2, s2r, m, A0, B0, se1 - A0, se2 - B0, go, ge, bufs, stride, nw, X, mw, epoch,
+                              ca, score, id, mt, ce, rest > 0 ? pm.list : nullptr, max(rest, 0));
+            if (rest < 0) mm = score;
+            ident += id;
+            matches += mt;
+            dcells += ce;
+        }
         acc[2] += (unsigned long long)dcells;
         // distance (:170-181), float arithmetic with IEEE rounding.
         const int len1 = g.nres[si], len2 = g.nres[sj];
@@ -939,6 +1023,7 @@ cudaError_t launch_cta(const cwgpu_context* ctx, const cwgpu::PairArgs& g, int p
     CtaArgs ca;
     ca.large_rows = ctx->cta_large_rows;
     ca.limit_ns = 4000000000ULL;  // no legitimate hand-over waits this long
+    ca.path_bytes = (ctx->path_cap / (size_t)grid) & ~(size_t)255;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)grid);
     cfg.blockDim = dim3(warps * 32);

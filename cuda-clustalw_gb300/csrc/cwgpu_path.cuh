@@ -49,8 +49,9 @@ constexpr int kPathRing = 4;          // steps of forward values in flight
 // all: the row's box was too wide).
 enum { kPathH = 1, kPathD = 2, kPathTight = 4 };
 
-// A warp's slice of the saved rows and of the working arrays below, for a pair
-// of n x m residues; fwd == nullptr when there is none.
+// A pair's slice of the saved rows and of the working arrays below, for n x m
+// residues and `warps` warps that share it, each with cells and list of
+// its own (path_of_warp); fwd == nullptr when there is none.
 struct PathMem {
     int every = 0;        // G
     int2* fwd = nullptr;  // row i (i % G == 0, 0 < i < n): fwd + (i / G - 1) * stride, column j at [j]
@@ -58,7 +59,6 @@ struct PathMem {
     size_t stride = 0;
     int2* cells = nullptr;  // forward values of the boxes in work
     int cell_cap = 0;
-    int2* half = nullptr;  // two rows of n + m + 2 for the lanes' own halves
     int4* span = nullptr;  // the saved rows' columns: of optimal paths (x, y), near (z, w)
     int4* list = nullptr;  // frames left to mm_align, from the front; to ask for, from the back
     int list_cap = 0;
@@ -67,31 +67,37 @@ struct PathMem {
 // Bytes of a slice with rows every 32 * g, and its parts. The cells hold the
 // boxes a warp works on at a time, 64 columns wider than high: a wider box is
 // taken alone.
-__host__ __device__ inline size_t path_bytes(int n, int m, int g, PathMem* p = nullptr, unsigned char* base = nullptr) {
+__host__ __device__ inline size_t path_bytes(int n, int m, int g, int warps = 1, PathMem* p = nullptr,
+                                             unsigned char* base = nullptr) {
     const int every = 32 * g;
     const size_t saved = n > 0 ? (size_t)((n - 1) / every) * (size_t)(m + 1) : 0;
     const size_t cells = (size_t)128 * ((m + 1 < every + 64 ? m + 1 : every + 64) + 8 * g);
-    const size_t half = 2 * (size_t)(n + m + 2), spans = (size_t)(n / every + 1);
+    const size_t spans = (size_t)(n / every + 1);
     if (p) {
         p->every = every;
         p->stride = (size_t)(m + 1);
         p->cell_cap = (int)cells;
         p->cells = reinterpret_cast<int2*>(base);
-        p->span = reinterpret_cast<int4*>(p->cells + cells);
+        p->span = reinterpret_cast<int4*>(p->cells + warps * cells);
         p->list = p->span + spans;
         p->list_cap = n + 1;
-        p->fwd = reinterpret_cast<int2*>(p->list + n + 1);
+        p->fwd = reinterpret_cast<int2*>(p->list + warps * (size_t)(n + 1));
         p->rev = p->fwd + saved;
-        p->half = p->rev + saved;
     }
-    return 8 * (cells + 2 * spans + 2 * (size_t)(n + 1) + 2 * saved + half);
+    return 8 * (warps * (cells + 2 * (size_t)(n + 1)) + 2 * spans + 2 * saved);
+}
+
+__device__ __forceinline__ PathMem path_of_warp(PathMem p, int w) {
+    p.cells += (size_t)w * p.cell_cap;
+    p.list += (size_t)w * p.list_cap;
+    return p;
 }
 
 // The finest spacing whose slice fits `cap` bytes.
-__device__ __forceinline__ bool path_mem(int n, int m, unsigned char* base, size_t cap, PathMem& p) {
+__device__ __forceinline__ bool path_mem(int n, int m, int warps, unsigned char* base, size_t cap, PathMem& p) {
     for (int g = 1; g <= kMaxPathG; g *= 2) {
-        if (path_bytes(n, m, g) <= cap) {
-            path_bytes(n, m, g, &p, base);
+        if (path_bytes(n, m, g, warps) <= cap) {
+            path_bytes(n, m, g, warps, &p, base);
             return true;
         }
     }
@@ -397,24 +403,25 @@ __device__ __noinline__ bool path_boxes(const int8_t* s1, int n, const int8_t* s
     return __all_sync(kFull, ok);
 }
 
-// The entries of all rows of the pair's box; false if some row has no cell on
-// an optimal path, or the boxes cost more than they save, and the caller runs
-// mm_align.
-template <bool NC>
-__device__ __noinline__ bool path_band(const int8_t* s1, int n, const int8_t* s2, const PathMem& mem, int2* band, int A0, int B0,
-                          int se1, int se2, int best, int go, int ge, const Env& env) {
-    const Env X = env;  // copies stay in registers across the stores below
-    const PathMem p = mem;
+__device__ __forceinline__ int path_box_count(const PathMem& p, int A0, int se1) {
+    return (se1 - 1) / p.every - A0 / p.every + 1;
+}
+
+// The entries of the saved rows, and the box's own first and last row; warp w
+// of nw. One warp follows the columns down; several start every row at the
+// box's first. False if a row has no cell on an optimal path.
+__device__ inline bool path_rows(const PathMem& p, int2* band, int A0, int B0, int se1, int se2, int best, int go, int w,
+                                 int nw) {
     const int lane = threadIdx.x & 31;
-    if (lane == 0) {
+    if (lane == 0 && w == 0) {
         band[0] = path_entry(0, 0, kPathH);
         band[se1 - A0] = path_entry(se2 - B0, se2 - B0, kPathH);
     }
-    const int base = A0 / p.every;
-    const int nboxes = (se1 - 1) / p.every - base + 1;
-    for (int b = 0, jl = B0; b + 1 < nboxes; ++b) {
+    const int base = A0 / p.every, nboxes = path_box_count(p, A0, se1);
+    for (int b = w, jl = B0; b + 1 < nboxes; b += nw) {
         const int i = (base + b + 1) * p.every;
         int lo, hi, kinds, near_lo, near_hi;
+        if (nw > 1) jl = B0;
         if (!path_row(p, i, jl, se2, best, go, lo, hi, kinds, near_lo, near_hi)) return false;
         if (lane == 0) {
             band[i - A0] = path_entry(lo - B0, hi - B0, kinds);
@@ -422,48 +429,75 @@ __device__ __noinline__ bool path_band(const int8_t* s1, int n, const int8_t* s2
         }
     }
     __syncwarp();
-    // A column of boxes costs about four steps of a sweep; mm_align's steps are
+    return true;
+}
+
+// The entries of the rows between them; warp w of nw, boxes dealt in runs of
+// as many as a warp takes at a time. False if some row has no cell on an
+// optimal path, or (one warp) the boxes cost more than they save.
+template <bool NC, bool CTA>
+__device__ __noinline__ bool path_fill(const int8_t* s1, int n, const int8_t* s2, const PathMem& mem, int2* band, int A0,
+                                       int B0, int se1, int se2, int best, int go, int ge, const Env& env, int w,
+                                       int nw) {
+    if (!CTA) w = 0, nw = 1;
+    const Env X = env;  // copies stay in registers across the stores below
+    const PathMem p = mem;
+    const int lane = threadIdx.x & 31;
+    const int nboxes = path_box_count(p, A0, se1);
+    // A column of boxes costs about five steps of a sweep; mm_align's steps are
     // about a 96th of the pair's box, and a few per row for the small frames.
-    const int W = p.every / kPathRows, seg = lane / W;
-    int left = (int)min((long long)(se1 - A0) * (se2 - B0) / 384 + (se1 - A0), (long long)INT_MAX);
-    for (int b = 0; b < nboxes;) {
-        // As many boxes as the slice and the shared edge rows hold.
-        int used = 0, width = 0, mine = -1;
-        while (used * W < 32 && b + used < nboxes) {
-            const PathBox x = path_box(p, b + used, nboxes, A0, B0, se1, se2);
-            const int w = max(width, x.jh - x.jl + 1);
-            if (!path_fits(p, used + 1, w, W, X.K)) break;
-            if (seg == used) mine = b + used;
-            width = w;
-            ++used;
+    // (A CTA's warps share the boxes, but not the small frames' divisions.)
+    const int W = p.every / kPathRows, seg = lane / W, run = nw > 1 ? 32 / W : nboxes;
+    int left = nw > 1 ? INT_MAX : (int)min((long long)(se1 - A0) * (se2 - B0) / 384 + (se1 - A0), (long long)INT_MAX);
+    for (int first = w * run; first < nboxes; first += nw * run) {
+        const int stop = min(first + run, nboxes);
+        for (int b = first; b < stop;) {
+            // As many boxes as the slice and the shared edge rows hold.
+            int used = 0, width = 0, mine = -1;
+            while (used * W < 32 && b + used < stop) {
+                const PathBox x = path_box(p, b + used, nboxes, A0, B0, se1, se2);
+                const int wide = max(width, x.jh - x.jl + 1);
+                if (!path_fits(p, used + 1, wide, W, X.K)) break;
+                if (seg == used) mine = b + used;
+                width = wide;
+                ++used;
+            }
+            if (nw == 1) left -= width + W;
+            if (left < 0) return false;
+            if (used == 0) {
+                const PathBox x = path_box(p, b, nboxes, A0, B0, se1, se2);
+                for (int i = x.i0 + 1 + lane; i < x.i1; i += 32) band[i - A0] = path_entry(0, 0, 0);
+                ++b;
+                continue;
+            }
+            if (!path_boxes<NC>(s1, n, s2, p, band, A0, B0, se1, se2, mine, width, nboxes, best, go, ge, X)) return false;
+            b += used;
         }
-        left -= width + W;
-        if (left < 0) return false;
-        if (used == 0) {
-            const PathBox x = path_box(p, b, nboxes, A0, B0, se1, se2);
-            for (int i = x.i0 + 1 + lane; i < x.i1; i += 32) band[i - A0] = path_entry(0, 0, 0);
-            ++b;
-            continue;
-        }
-        if (!path_boxes<NC>(s1, n, s2, p, band, A0, B0, se1, se2, mine, width, nboxes, best, go, ge, X))
-            return false;
-        b += used;
     }
     __syncwarp();
     return true;
 }
+
+// The walk's rows of diff()'s halves, at the end of the warp's region: of a lane
+// kPathLaneCols columns (enough if two rows in succession never span more), or
+// of the whole warp kPathWarpCols; column j at j modulo that.
+constexpr int kPathLaneCols = 8;
+constexpr int kPathWarpCols = 32 * kPathLaneCols;
+constexpr int kPathRowBytes = 2 * kPathWarpCols * (int)sizeof(int2);  // of a warp, both halves
+struct PathRow {
+    int2* at;  // of this lane
+    __device__ __forceinline__ int2& operator[](int j) const { return at[(j & (kPathLaneCols - 1)) * 32]; }
+};
 
 // One lane: diff()'s two halves of frame (A, B, M, N) at row r = A + M / 2 over
 // the rows' column ranges, and its midpoint scans (:570-593). All coordinates
 // are relative to the box; s1/s2 point at its first residues. Cells outside the
 // ranges are on no optimal path and only ever lose to those inside.
 template <bool NC>
-__device__ void path_midpoint(const int8_t* s1, const int8_t* s2, const int2* band, int2* half, size_t half_stride,
+__device__ void path_midpoint(const int8_t* s1, const int8_t* s2, const int2* band, const PathRow F, const PathRow Rv,
                               int A, int B, int M, int N, int tb, int te, int go, int ge, const Env& X, int& midj,
                               bool& type2) {
     const int goe = go + ge, r = A + M / 2;
-    int2* F = half + A;  // column j at F[j], j = B..B + N: words no other frame of the walk uses
-    int2* Rv = F + half_stride;
     // forward half, from the last single row above r
     int q = r - 1;
     while (q > A && !path_single(band[q])) --q;
@@ -560,6 +594,41 @@ __device__ __forceinline__ bool path_tight(const int2* band, int A, int M, int A
     return false;
 }
 
+// The free corner (r, c) of frame f (absolute rows and columns; end: its last,
+// else its first), the saved row i (or the pair's own edge) the rows there are
+// computed from, and the farthest column they are computed over.
+struct PathCorner {
+    int r, c, i, far;
+    bool edge, loose;
+};
+
+__device__ __forceinline__ PathCorner path_corner(const PathMem& p, int4 f, bool end, int A0, int B0, int se1, int se2) {
+    PathCorner x;
+    x.r = end ? f.x + f.z : f.x;
+    x.c = end ? f.y + (f.w & ((1 << 29) - 1)) : f.y;
+    x.i = end ? max(A0, (x.r - 1) / p.every * p.every) : min(se1, (x.r / p.every + 1) * p.every);
+    x.edge = end ? x.i == A0 : x.i == se1;
+    const int4 span = x.edge ? make_int4(0, 0, B0, se2) : p.span[x.i / p.every - A0 / p.every - 1];
+    // The frame's other corner may be the pair's own, where diff() opens gaps
+    // free as well: a path may then run along the box's edge before it reaches
+    // the saved row, in any column, which is no better than ending (starting)
+    // where it does, at reversePass's -1 (forwardPass's 0).
+    x.loose = end ? f.x == A0 && !((f.w >> 29) & 1) : f.x + f.z == se1 && !((f.w >> 30) & 1);
+    x.far = x.loose ? (end ? B0 : se2) : (end ? span.z : span.w);
+    return x;
+}
+
+// Whether mm_align divides frame f in fewer steps than path_ask takes to tell
+// that it need not: each level takes its columns and some 40 steps, down to the
+// frames one lane does; a quarter of the corner's columns, of 1.5 steps each.
+// (Asked for all frames, pairs of weak alignments of 1600 residues spent 20 of
+// 47 million cycles there: paths within gapOpen are a thousand columns apart.)
+__device__ __forceinline__ bool path_ask_dear(const PathMem& p, int4 f, bool end, int A0, int B0, int se1, int se2) {
+    const PathCorner x = path_corner(p, f, end, A0, B0, se1, se2);
+    const int levels = 32 - __clz(f.z >> 5);
+    return 3 * (abs(x.far - x.c) + 8) / 8 > ((f.w & ((1 << 29) - 1)) + 40) * levels + 20;
+}
+
 // Up to 32 / (p.every / 4) of the last frames asked for, a segment of lanes each
 // like the boxes': those whose free corner no horizontal gap can use go to the
 // stack, the others to the list. For a frame that starts at its free corner
@@ -570,28 +639,21 @@ __device__ __forceinline__ bool path_tight(const int2* band, int A, int M, int A
 // the saved row above. Lane row t is t + 1 rows from the saved row.
 template <bool NC>
 __device__ void path_ask(const int8_t* s1, int n, const int8_t* s2, int m, const PathMem& p, int A0, int B0, int se1,
-                         int se2, int go, int ge, const Env& X, int4* stack, int& sp, int& nlist, int& nask) {
+                         int se2, int go, int ge, const Env& X, int4* stack, int& sp, int& nlist, int& nask,
+                         bool keep) {
     constexpr int R = kPathRows;
     const int lane = threadIdx.x & 31, W = p.every / R, seg = lane / W, sl = lane & (W - 1);
     const int goe = go + ge;
     const int* const smat = X.smat();
     const int take = min(32 / W, nask);
-    const int base = A0 / p.every;
     int4 f = p.list[p.list_cap - nask + min(seg, take - 1)];
     const bool end = (f.z >> 30) & 1;
     f.z &= (1 << 30) - 1;
     const int dir = end ? -1 : 1;  // from the corner to the saved row
-    const int r = end ? f.x + f.z : f.x, c = end ? f.y + (f.w & ((1 << 29) - 1)) : f.y;
-    const int i = end ? max(A0, (r - 1) / p.every * p.every) : min(se1, (r / p.every + 1) * p.every);
-    const bool corner = end ? i == A0 : i == se1;
-    const int4 span = corner ? make_int4(0, 0, B0, se2) : p.span[i / p.every - base - 1];
-    // The frame's other corner may be the pair's own, where diff() opens gaps
-    // free as well: a path may then run along the box's edge before it reaches
-    // the saved row, in any column, which is no better than ending (starting)
-    // where it does, at reversePass's -1 (forwardPass's 0).
-    const bool loose = end ? f.x == A0 && !((f.w >> 29) & 1) : f.x + f.z == se1 && !((f.w >> 30) & 1);
+    const PathCorner at = path_corner(p, f, end, A0, B0, se1, se2);
+    const int r = at.r, c = at.c, i = at.i, far = at.far;
+    const bool corner = at.edge, loose = at.loose;
     const int floor = !loose ? 2 * kPathLow : end ? 0 : -1;
-    const int far = loose ? (end ? B0 : se2) : (end ? span.z : span.w);
     const int nrows = dir * (i - r), ncols = dir * (far - c) + 1, lanes = (nrows + R - 1) / R;
     const int nsteps = __reduce_max_sync(kFull, seg < take ? ncols + lanes - 1 : 0);
     const bool on = seg < take && sl < lanes;
@@ -649,39 +711,185 @@ __device__ void path_ask(const int8_t* s1, int n, const int8_t* s2, int m, const
     const unsigned below = (1u << lane) - 1;
     const unsigned to_stack = __ballot_sync(kFull, head && !listed), to_list = __ballot_sync(kFull, head && listed);
     if (head && !listed) stack[sp + __popc(to_stack & below)] = make_int4(f.x - A0, f.y - B0, f.z, f.w);
-    if (head && listed) p.list[nlist + __popc(to_list & below)] = f;
+    if (head && listed && keep) p.list[nlist + __popc(to_list & below)] = f;
     sp += __popc(to_stack);
-    nlist += __popc(to_list);
+    if (keep) nlist += __popc(to_list);
     nask -= take;
     __syncwarp();
 }
 
-// Whether one lane's halves of frame (A, M) would visit a row of a box left
-// out, or more cells than mm_align's steps are worth (a 53rd of the frame, and
-// some).
-__device__ inline bool path_too_wide(const int2* band, int A, int M, int N) {
+// What one lane's halves of frame (A, M) would visit: 0 at most `most` cells,
+// two rows in succession never over more than kPathLaneCols columns; 1 more; 2
+// a row of a box left out.
+__device__ inline int path_extent(const int2* band, int A, int M, int most) {
     const int r = A + M / 2;
-    int cells = path_hi(band[r]) - path_lo(band[r]) + 1;
-    bool known = band[r].y != 0;
-    const int most = (int)min((long long)M * N / 53 + 400, (long long)INT_MAX);
-    for (int q = r - 1; q > A && !path_single(band[q]) && cells <= most && known; --q) {
-        cells += path_hi(band[q]) - path_lo(band[q]) + 1;
-        known = band[q].y != 0;
+    const int2 mid = band[r];
+    int cells = path_hi(mid) - path_lo(mid) + 1, span = cells;
+    if (mid.y == 0) return 2;
+    for (int dir = -1; dir <= 1; dir += 2) {
+        int2 last = mid;
+        const int end = dir < 0 ? A : A + M;
+        for (int q = r + dir;; q += dir) {
+            const int2 v = band[q];
+            if (v.y == 0) return 2;
+            span = max(span, dir < 0 ? path_hi(last) - path_lo(v) + 1 : path_hi(v) - path_lo(last) + 1);
+            cells += path_hi(v) - path_lo(v) + 1;
+            if (cells > most || span > kPathLaneCols) return 1;
+            if (q == end || path_single(v)) break;
+            last = v;
+        }
     }
-    for (int q = r + 1; q < A + M && !path_single(band[q]) && cells <= most && known; ++q) {
-        cells += path_hi(band[q]) - path_lo(band[q]) + 1;
-        known = band[q].y != 0;
+    return 0;
+}
+
+// The same frame's midpoint by the whole warp, a row of up to 32 columns at a
+// time: the gap along a row is a prefix maximum over the lanes. False if a row
+// of a box left out is in the way, or mm_align's steps cost less (a row or 32
+// columns here about as much as three cells of the frame there). A lane alone
+// spent 150 to 300 cycles per cell on frames this wide, up to 27 million per
+// pair of weak alignments of 1600 residues (of 46 in all); row by row 250.
+template <bool NC>
+__device__ bool path_midpoint_warp(const int8_t* s1, const int8_t* s2, const int2* band, int2* rows, int A, int B,
+                                   int M, int N, int tb, int te, int go, int ge, int nw, const Env& X, int& midj,
+                                   bool& type2) {
+    const int lane = threadIdx.x & 31, r = A + M / 2, goe = go + ge;
+    const int2 mid = band[r];
+    // Both ways to the nearest single row, or the frame's end.
+    int start[2], cells = 0, span = path_hi(mid) - path_lo(mid) + 1, unknown = mid.y == 0;
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+        const int dir = h ? 1 : -1, end = h ? A + M : A;
+        for (int q0 = r + dir;; q0 += 32 * dir) {
+            const int q = q0 + dir * lane;
+            const bool in = h ? q <= end : q >= end;
+            const int2 v = in ? band[q] : make_int2(0, 0), last = in ? band[q - dir] : v;
+            const unsigned stops = __ballot_sync(kFull, in && (q == end || path_single(v)));
+            if (in && lane <= __ffs(stops) - 1u) {
+                unknown |= v.y == 0;
+                span = max(span, h ? path_hi(v) - path_lo(last) + 1 : path_hi(last) - path_lo(v) + 1);
+                cells += path_hi(v) - path_lo(v) + 1;
+            }
+            if (stops) {
+                start[h] = q0 + dir * (__ffs(stops) - 1);
+                break;
+            }
+        }
     }
-    return cells > most || !known;
+    span = __reduce_max_sync(kFull, span);
+    cells = __reduce_add_sync(kFull, cells);
+    if (__any_sync(kFull, unknown) || span > kPathWarpCols ||
+        cells + 32ll * (start[1] - start[0]) > (long long)M * N / (3 * nw) + 2000)
+        return false;
+
+    int lo[2], hi[2];
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+        const int dir = h ? -1 : 1;  // from the start row to r
+        const int open = h ? te : tb;
+        int2* const row = rows + h * kPathWarpCols;  // column j at [j & (kPathWarpCols - 1)]
+        int q = start[h];
+        const int2 v0 = band[q];
+        const bool edge = q == (h ? A + M : A);
+        // Columns from..to of the row so far, in the half's own direction.
+        const int c0 = !edge ? path_lo(v0) : h ? B + N : B;
+        int from = c0, to = c0;
+        if (edge) to = h ? max(path_lo(v0), B) : min(path_hi(v0), B + N);
+        __syncwarp();
+        for (int k = lane; k <= dir * (to - from); k += 32) {
+            const int left = edge ? -open - ge * k : 0;
+            row[(from + dir * k) & (kPathWarpCols - 1)] =
+                k ? make_int2(left, left - go) : make_int2(0, edge ? -open : -go);
+        }
+        __syncwarp();
+        int2 v32 = make_int2(0, 0);
+        int res32 = 0;
+        for (int k = 0; q != r; ++k, q += dir) {
+            if ((k & 31) == 0) {  // the next 32 rows' entries and residues
+                const int qq = q + dir * lane;
+                const bool in = h ? qq > r : qq < r;
+                v32 = in ? band[qq + dir] : make_int2(0, 0);
+                res32 = in ? (int)ldres<NC>(s1 + (h ? qq - 1 : qq)) : 0;
+            }
+            const int ends = __shfl_sync(kFull, v32.x, k & 31);
+            const int* const sub = X.smat() + 32 * __shfl_sync(kFull, res32, k & 31);
+            const int2 v = make_int2(ends, 0);
+            const int nfrom = h ? min(path_hi(v), c0) : max(path_lo(v), c0);
+            const int nto = h ? max(path_lo(v), B) : min(path_hi(v), B + N);
+            int carry = kPathLow, behind = kPathLow;  // the gap along the row, H above the column before
+            for (int t = 0; t <= dir * (nto - nfrom); t += 32) {
+                const int j = nfrom + dir * (t + lane);
+                const bool in = dir * (nto - j) >= 0;
+                const bool above = dir * (j - from) >= 0 && dir * (to - j) >= 0;
+                const int2 up = above ? row[j & (kPathWarpCols - 1)] : make_int2(kPathLow, kPathLow);
+                int diag = __shfl_up_sync(kFull, up.x, 1);
+                if (lane == 0) {
+                    const int jb = j - dir;
+                    diag = t ? behind
+                             : (dir * (jb - from) >= 0 && dir * (to - jb) >= 0 ? row[jb & (kPathWarpCols - 1)].x : kPathLow);
+                }
+                behind = __shfl_sync(kFull, up.x, 31);
+                const int e = __viaddmax_s32(up.y, -ge, up.x - goe);
+                const int jr = h ? j : j - 1;  // the column's residue
+                const int sc = in && jr >= 0 ? sub[ldres<NC>(s2 + jr)] : kPadScore;
+                const int he = max(e, diag + sc);
+                int best = in ? he - goe : kPathLow;  // of a gap from a column up to here, at the next
+                const int count = min(32, dir * (nto - nfrom) + 1 - t);
+                for (int d = 1; d < count; d *= 2) {
+                    const int o = __shfl_up_sync(kFull, best, d);
+                    if (lane >= d) best = max(best, o - ge * d);
+                }
+                int f = __shfl_up_sync(kFull, best, 1);
+                f = lane ? max(f, carry - ge * lane) : carry;
+                carry = max(__shfl_sync(kFull, best, 31), carry - ge * 32);
+                __syncwarp();  // every lane has read the row above
+                if (in) row[j & (kPathWarpCols - 1)] = make_int2(max(he, f), e);
+            }
+            __syncwarp();
+            from = nfrom;
+            to = nto;
+        }
+        lo[h] = h ? to : from;
+        hi[h] = h ? from : to;
+    }
+    // Type 1: the last of the best columns that has (F.x != F.y, R.x == R.y),
+    // else the first; type 2, if better: the last.
+    const int l = max(lo[0], lo[1]), u = min(hi[0], hi[1]);
+    int h1 = INT_MIN, first = INT_MAX, tied = -1, h2 = INT_MIN, at2 = -1;
+    for (int j = l + lane; j <= u; j += 32) {
+        const int2 a = rows[j & (kPathWarpCols - 1)], b = rows[kPathWarpCols + (j & (kPathWarpCols - 1))];
+        const int hh = a.x + b.x, vv = a.y + b.y + go;
+        const bool keep = a.x != a.y && b.x == b.y;
+        if (hh > h1) {
+            h1 = hh;
+            first = j;
+            tied = keep ? j : -1;
+        } else if (hh == h1 && keep) {
+            tied = j;
+        }
+        if (vv >= h2) {
+            h2 = vv;
+            at2 = j;
+        }
+    }
+    const int b1 = __reduce_max_sync(kFull, h1), b2 = __reduce_max_sync(kFull, h2);
+    first = __reduce_min_sync(kFull, h1 == b1 ? first : INT_MAX);
+    tied = __reduce_max_sync(kFull, h1 == b1 ? tied : -1);
+    at2 = __reduce_max_sync(kFull, h2 == b2 ? at2 : -1);
+    type2 = b2 > b1;
+    midj = (type2 ? at2 : tied >= 0 ? tied : first) - B;
+    __syncwarp();
+    return true;
 }
 
 // Walks diff()'s frames from the box's own, 32 at a time. Adds identities,
 // matches and inner-loop iterations; frames left to mm_align go to p.list
-// (count returned).
-template <bool NC>
+// (count returned). With nw warps (w: this one's number) all walk the first
+// levels, which only warp 0 accounts for, and then a share of the frames each.
+template <bool NC, bool CTA>
 __device__ __noinline__ int path_walk(const int8_t* s1, int n, const int8_t* s2, int m, const PathMem& mem, const int2* band,
                                       int A0, int B0, int se1, int se2, int go, int ge, const Env& env,
-                                      int& n_ident, int& n_match, long long& n_cells) {
+                                      int& n_ident, int& n_match, long long& n_cells, int w, int nw) {
+    if (!CTA) w = 0, nw = 1;
     const Env X = env;  // copies stay in registers across the stores below
     const PathMem p = mem;
     const int M0 = se1 - A0, N0 = se2 - B0;
@@ -692,8 +900,9 @@ __device__ __noinline__ int path_walk(const int8_t* s1, int n, const int8_t* s2,
     const int lane = threadIdx.x & 31;
     constexpr int NMASK = (1 << 29) - 1;
     int4* stack = reinterpret_cast<int4*>(X.region());
-    const int cap = warp_region_bytes(X.K) / (int)sizeof(int4);
-    const size_t half_stride = (size_t)(n + m + 2);
+    const int cap = (warp_region_bytes(X.K) - kPathRowBytes) / (int)sizeof(int4);
+    int2* const rows = reinterpret_cast<int2*>(stack + cap);
+    bool dealt = nw == 1;  // this warp's frames are its own
     int ident = 0, match = 0, nlist = 0, nask = 0;
     long long cells = 0;
     __syncwarp();
@@ -701,14 +910,28 @@ __device__ __noinline__ int path_walk(const int8_t* s1, int n, const int8_t* s2,
     __syncwarp();
     int sp = 1;
     for (;;) {
-        if (sp == 0) {
-            if (nask == 0) break;
-            while (nask > 0) path_ask<NC>(seq1, n, seq2, m, p, A0, B0, se1, se2, go, ge, X, stack, sp, nlist, nask);
+        if (sp == 0 && nask == 0) break;
+        if (nask > 0 && (sp == 0 || !dealt)) {
+            while (nask > 0 && sp + 32 < cap - 96)
+                path_ask<NC>(seq1, n, seq2, m, p, A0, B0, se1, se2, go, ge, X, stack, sp, nlist, nask, dealt || w == 0);
             continue;
         }
-        // Taking one frame at a time grows the stack by at most the depth of
-        // the recursion (17), so near its end the walk goes depth first.
-        const int take = sp > cap - 96 ? 1 : min(32, sp);
+        if (!dealt && sp >= 2 * nw) {  // every warp has the same frames: warp w keeps those at w, w + nw, ...
+            int kept = 0;
+            for (int k = w; k < sp; k += nw, ++kept) {
+                const int4 f = stack[k];
+                __syncwarp();
+                if (lane == 0) stack[kept] = f;
+                __syncwarp();
+            }
+            sp = kept;
+            dealt = true;
+            continue;
+        }
+        const bool mine = dealt || w == 0;
+        // Taking t frames grows the stack by at most t, one at a time by at
+        // most the depth of the recursion (17): near the stack's end fewer.
+        const int take = max(1, min(min(32, sp), cap - 40 - sp));
         int4 fr = make_int4(0, 0, 0, 0);
         if (lane < take) fr = stack[sp - 1 - lane];
         sp -= take;
@@ -718,8 +941,36 @@ __device__ __noinline__ int path_walk(const int8_t* s1, int n, const int8_t* s2,
         const int A = fr.x, B = fr.y, M = fr.z, N = fr.w & NMASK;
         const int tbf = (fr.w >> 29) & 1, tef = (fr.w >> 30) & 1;
         const int tb = tbf ? go : 0, te = tef ? go : 0;
+        // Where the middle row leaves a choice: by 0 this lane, 1 the warp, 2 mm_align.
+        const int midi = M / 2;
+        int by = 3, midj = 0;
+        bool type2 = false;
+        if (lane < take && M > 1) {
+            const int2 v = band[A + midi];
+            const int kinds = v.y & (kPathH | kPathD);
+            midj = path_lo(v) - B;
+            type2 = kinds == kPathD;
+            // The fewer frames there are, the sooner the whole warp is faster.
+            if (kinds == 0 || kinds == (kPathH | kPathD) || path_lo(v) != path_hi(v))
+                by = path_extent(band, A, M, 32 + 16 * take);
+        }
+        for (unsigned wide = __ballot_sync(kFull, by == 1); wide; wide &= wide - 1) {
+            const int l = __ffs(wide) - 1;
+            int mj;
+            bool t2;
+            const bool done = path_midpoint_warp<NC>(
+                s1, s2, band, rows, __shfl_sync(kFull, A, l), __shfl_sync(kFull, B, l), __shfl_sync(kFull, M, l),
+                __shfl_sync(kFull, N, l), __shfl_sync(kFull, tb, l), __shfl_sync(kFull, te, l), go, ge, nw, X, mj, t2);
+            if (lane == l) {
+                by = done ? 3 : 2;
+                if (done) {
+                    midj = mj;
+                    type2 = t2;
+                }
+            }
+        }
         if (lane < take && M == 1) {
-            cells += N;
+            if (mine) cells += N;
             int midh = -(tb + ge) - (te + ge * N);
             const int hh0 = -(te + ge) - (tb + ge * N);
             midh = max(midh, hh0);
@@ -737,24 +988,19 @@ __device__ __noinline__ int path_walk(const int8_t* s1, int n, const int8_t* s2,
                     rb = b;
                 }
             }
-            if (at > 0) {
+            if (at > 0 && mine) {
                 ++match;
                 if (ra != X.gp1 && rb != X.gp2 && ra == rb) ++ident;
             }
         } else if (lane < take) {
-            const int midi = M / 2;
-            const int2 v = band[A + midi];
-            int midj = path_lo(v) - B;
-            const int kinds = v.y & (kPathH | kPathD);
-            bool type2 = kinds == kPathD;
-            const bool open = kinds == 0 || kinds == (kPathH | kPathD) || path_lo(v) != path_hi(v);
-            if (open && path_too_wide(band, A, M, N)) {
+            if (by == 2) {
                 kid[0] = fr;
                 kind[0] = 2;
             } else {
-                cells += (long long)M * N;
-                if (open)
-                    path_midpoint<NC>(s1, s2, band, p.half, half_stride, A, B, M, N, tb, te, go, ge, X, midj, type2);
+                if (mine) cells += (long long)M * N;
+                if (by == 0)
+                    path_midpoint<NC>(s1, s2, band, PathRow{rows + lane}, PathRow{rows + kPathWarpCols + lane}, A, B, M, N,
+                                      tb, te, go, ge, X, midj, type2);
                 if (!type2) {
                     kid[0] = make_int4(A + midi, B + midj, M - midi, (N - midj) | (1 << 29) | (tef << 30));
                     kid[1] = make_int4(A, B, midi, midj | (tbf << 29) | (1 << 30));
@@ -773,6 +1019,11 @@ __device__ __noinline__ int path_walk(const int8_t* s1, int n, const int8_t* s2,
                         kind[0] = tef == 0 && A + M < M0 && !path_tight(band, kid[0].x, kid[0].z, A0, p.every) ? 2 : 3;
                     if (kind[1])
                         kind[1] = tbf == 0 && A > 0 && !path_tight(band, kid[1].x, kid[1].z, A0, p.every) ? 2 : 3;
+#pragma unroll
+                    for (int c = 0; c < 2; ++c) {
+                        const int4 f = make_int4(kid[c].x + A0, kid[c].y + B0, kid[c].z, kid[c].w);
+                        if (kind[c] == 3 && path_ask_dear(p, f, c == 1, A0, B0, se1, se2)) kind[c] = 2;
+                    }
                 }
             }
         }
@@ -782,14 +1033,14 @@ __device__ __noinline__ int path_walk(const int8_t* s1, int n, const int8_t* s2,
             const unsigned on = __ballot_sync(kFull, kind[c] == 1), off = __ballot_sync(kFull, kind[c] == 2);
             const unsigned ask = __ballot_sync(kFull, kind[c] == 3);
             if (kind[c] == 1) stack[sp + __popc(on & below)] = kid[c];
-            if (kind[c] == 2)
+            if (kind[c] == 2 && mine)
                 p.list[nlist + __popc(off & below)] = make_int4(kid[c].x + A0, kid[c].y + B0, kid[c].z, kid[c].w);
             // Absolute rows and columns in both, the kid's number with the ones to ask for.
             if (kind[c] == 3)
                 p.list[p.list_cap - 1 - nask - __popc(ask & below)] =
                     make_int4(kid[c].x + A0, kid[c].y + B0, kid[c].z | c << 30, kid[c].w);
             sp += __popc(on);
-            nlist += __popc(off);
+            if (mine) nlist += __popc(off);
             nask += __popc(ask);
         }
         __syncwarp();

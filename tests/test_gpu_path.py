@@ -48,12 +48,15 @@ def sequences(kind, seed):
     raise ValueError(kind)
 
 
-def check(ctx, oracle_mod, seqs, matrix, params, pairs):
+def check(ctx, oracle_mod, seqs, matrix, params, pairs, cta_warps=0):
     want = oracle_mod.align_pairs(seqs, matrix, params, pairs)
     ctx.set_matrix(matrix)
     ctx.set_params(params)
     ctx.upload_seqs(seqs)
-    ctx.set_cta_tuning(max_pairs=0)  # one warp per pair
+    if cta_warps:
+        ctx.set_cta_tuning(1 << 30, cta_warps)  # one CTA of that many warps per pair
+    else:
+        ctx.set_cta_tuning(max_pairs=0)  # one warp per pair
     plan = ctx.plan(pairs)
     plan.launch()
     dist, stats = plan.results(stats=True)
@@ -117,3 +120,16 @@ def test_path_free_corners_near_the_ends(oracle_mod):
         params["pw_gap_open"], params["pw_gap_extend"] = 4.0, 0.2
         i, j = synth.all_pairs(600)[54841]
         check(ctx, oracle_mod, [family[i], family[j]], matrix, params, np.array([[0, 1], [1, 0]], dtype=np.int32))
+
+
+@pytest.mark.parametrize("warps", [2, 8, 16])
+@pytest.mark.parametrize("kind", ["gaps", "close gaps", "wide gaps", "ties", "weak", "edges"])
+def test_path_shared_by_a_cta(oracle_mod, kind, warps):
+    """The rows, the boxes and the walk's frames dealt over a CTA's warps."""
+    from clustalw_gb300 import load_matrix, native, synth
+
+    seqs = sequences(kind, 200 + len(kind))
+    matrix, params = load_matrix("protein")
+    up = synth.all_pairs(len(seqs))
+    with native.Context(0) as ctx:
+        check(ctx, oracle_mod, seqs, matrix, params, np.concatenate([up, up[:, ::-1]]), cta_warps=warps)
