@@ -46,6 +46,7 @@
 
 namespace {
 
+constexpr size_t kServePathLimit = (size_t)2 << 30;  // bytes of the pair kernels' path slices, both rounds
 constexpr int kShortRows = 128;  // pairs whose first sequence is this short: the 4-row kernel
 
 // A job's block in the budget arena.
@@ -190,6 +191,8 @@ struct cwgpu_server {
     cudaStream_t upload = nullptr;  // job uploads, waited for before the job's first round
     unsigned long long* d_counter[2] = {nullptr, nullptr};
     int2* d_scratch[2] = {nullptr, nullptr};
+    unsigned char* d_path[2] = {nullptr, nullptr};  // the long-pair kernel's slices (PairArgs::path)
+    size_t path_bytes = 0;
     int32_t* d_go = nullptr;  // gap-open penalty by min(n, m), 0..max_seq_len
     int grid = 0, grid_short = 0, grid_K = -1;
     int prio_low = 0, prio_high = 0;
@@ -469,12 +472,13 @@ int launch_round(cwgpu_server* s, int ri, int64_t nitems) {
         gl.tiny_m = 32;
         gl.tiny_n = cwgpu::kTinyMaxN;
         gl.general = s->general_gaps;
-        gl.path = nullptr;
-        gl.path_bytes = 0;
-        gl.path_slots = 0;
+        gl.path = s->d_path[ri];
+        gl.path_bytes = s->path_bytes;
+        gl.path_slots = 5LL * s->sm_count * wpc;
         cwgpu::PairArgs gs = gl;
         gs.order = gl.order + r.nlong;
         gs.npairs = r.n - r.nlong;
+        gs.path = nullptr;
         gs.counter = s->d_counter[ri] + 4;
         if (r.nlong > 0) gs.scratch += (size_t)5 * s->sm_count * wpc * 2 * (size_t)(s->opts.max_seq_len + 1);
         e = cwgpu_enqueue_pair_kernels(gl, gs, s->grid, s->grid_short, s->prio_high, s->prio_low, st, r.s2, r.fork,
@@ -647,12 +651,17 @@ int cwgpu_server_create(int device, const int32_t* matrix, const cwgpu_params* p
     }
     // Scratch rows per round: 5 CTAs per SM of each pair kernel (their launch bound).
     const size_t slots = (size_t)2 * 5 * s->sm_count * cwgpu_pair_kernel_warps_per_cta();
+    // Slices of the long-pair kernel: for the longest pairs, or what the limit
+    // leaves each (longer pairs then keep rows further apart, or none).
+    s->path_bytes = std::min((cwgpu::path_bytes(opts->max_seq_len, opts->max_seq_len, 1) + 255) & ~(size_t)255,
+                             kServePathLimit / slots & ~(size_t)255);
     if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&s->upload, cudaStreamNonBlocking);
     for (int i = 0; i < 2 && e == cudaSuccess; ++i) {
         e = cudaStreamCreateWithFlags(&s->streams[i], cudaStreamNonBlocking);
         if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&s->rounds[i].s2, cudaStreamNonBlocking);
         if (e == cudaSuccess) e = cudaMalloc(&s->d_counter[i], 8 * sizeof(unsigned long long));
         if (e == cudaSuccess) e = cudaMalloc(&s->d_scratch[i], slots * 2 * (opts->max_seq_len + 1) * sizeof(int2));
+        if (e == cudaSuccess) e = cudaMalloc(&s->d_path[i], slots / 2 * s->path_bytes);
         if (e == cudaSuccess) e = cudaEventCreateWithFlags(&s->rounds[i].ev, cudaEventDisableTiming);
         if (e == cudaSuccess) e = cudaEventCreateWithFlags(&s->rounds[i].fork, cudaEventDisableTiming);
         if (e == cudaSuccess) e = cudaEventCreateWithFlags(&s->rounds[i].join, cudaEventDisableTiming);
@@ -695,6 +704,7 @@ void cwgpu_server_destroy(cwgpu_server* s) {
         if (r.d) cudaFree(r.d);
         if (s->d_counter[i]) cudaFree(s->d_counter[i]);
         if (s->d_scratch[i]) cudaFree(s->d_scratch[i]);
+        if (s->d_path[i]) cudaFree(s->d_path[i]);
         if (s->streams[i]) cudaStreamDestroy(s->streams[i]);
     }
     if (s->upload) cudaStreamDestroy(s->upload);
