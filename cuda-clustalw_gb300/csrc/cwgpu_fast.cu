@@ -644,7 +644,7 @@ struct cwgpu_fast_state {
     int32_t* d_start = nullptr;
     int limit = 0;
     unsigned long long* d_counter = nullptr;
-    size_t smem_set = 0;
+    bool smem_set = false;
     uint2* d_ovf = nullptr;  // list overflow, ovf_records per warp of the grid
     size_t ovf_bytes = 0;
     uint16_t* d_sort = nullptr;  // sort copies, 2 * sort_stride per warp of the grid
@@ -750,15 +750,17 @@ int ensure_tables(cwgpu_context* ctx, const Params& P) {
     return CWGPU_OK;
 }
 
+constexpr size_t kMaxShared = 227 * 1024;
+
 // Runs the pairs (device pointers) in `d_order` order on `st`; synchronous.
 int run_fast(cwgpu_context* ctx, const Params& P, const int32_t* d_pairs, const int32_t* d_order, long long npairs,
              double* d_dist, cwgpu_fast_stats* d_stats, cudaStream_t st) {
     cwgpu_fast_state* F = ctx->fast;
     const size_t sm = smem_bytes(ctx->lmax, max_flagged(ctx->lmax, P.signif, P.window));
-    if (sm > 227 * 1024) return ffail(ctx, CWGPU_ERR_ARG, "sequences too long for the quick path's shared memory");
-    if (sm > F->smem_set) {
-        FAST_CUDA(ctx, cudaFuncSetAttribute(k_fast, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
-        F->smem_set = sm;
+    if (sm > kMaxShared) return ffail(ctx, CWGPU_ERR_ARG, "sequences too long for the quick path's shared memory");
+    if (!F->smem_set) {  // one value for the process: contexts need different amounts at the same time
+        FAST_CUDA(ctx, cudaFuncSetAttribute(k_fast, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMaxShared));
+        F->smem_set = true;
     }
     int per_sm = 0;
     FAST_CUDA(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_fast, 32, sm));

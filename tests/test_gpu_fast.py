@@ -188,3 +188,14 @@ def test_gpu_fast_range_and_errors(ctx, oracle_mod):
         ctx.fast_pairwise_align(native.FastParams.from_dict(fp), 5, 2, 0, n, el, n + 1)
     with pytest.raises(CwgpuError):  # too many k-tuple codes
         ctx.fast_align_pairs([[0, 1]], native.FastParams.from_dict(dict(fp, ktup=4)))
+
+
+def test_gpu_fast_two_contexts_of_different_lengths(ctx, oracle_mod):
+    """A context of long sequences, one of short ones, the first again: what one
+    allows itself of shared memory leaves the other's launches as they were."""
+    from clustalw_gb300 import native, synth
+
+    long_set, short_set = synth.protein_family(4, 1500, 1), synth.protein_family(4, 40, 2)
+    with native.Context(0) as other:
+        for c, seqs in ((ctx, long_set), (other, short_set), (ctx, long_set)):
+            check(c, oracle_mod, seqs, params(seqs=seqs))
