@@ -743,15 +743,17 @@ __device__ inline int path_extent(const int2* band, int A, int M, int most) {
 }
 
 // The same frame's midpoint by the whole warp, a row of up to 32 columns at a
-// time: the gap along a row is a prefix maximum over the lanes. False if a row
-// of a box left out is in the way, or mm_align's steps cost less (a row or 32
-// columns here about as much as three cells of the frame there). A lane alone
-// spent 150 to 300 cycles per cell on frames this wide, up to 27 million per
-// pair of weak alignments of 1600 residues (of 46 in all); row by row 250.
+// time: the gap along a row is a prefix maximum over the lanes. Returns 2 * midj
+// + (type 2), or -1 if a row of a box left out is in the way, or mm_align's
+// steps cost less (a row or 32 columns here about as much as three cells of the
+// frame there). A lane alone spent 150 to 300 cycles per cell on frames this
+// wide, up to 27 million per pair of weak alignments of 1600 residues (of 46 in
+// all); row by row 250. A call of its own: inlined it took registers from the
+// walk (200 x 1523: 52.1 against 51.4 ms).
 template <bool NC>
-__device__ bool path_midpoint_warp(const int8_t* s1, const int8_t* s2, const int2* band, int2* rows, int A, int B,
-                                   int M, int N, int tb, int te, int go, int ge, int nw, const Env& X, int& midj,
-                                   bool& type2) {
+__device__ __noinline__ int path_midpoint_warp(const int8_t* s1, const int8_t* s2, const int2* band, int2* rows, int A,
+                                               int B, int M, int N, int tb, int te, int go, int ge, int nw,
+                                               const int* smat) {
     const int lane = threadIdx.x & 31, r = A + M / 2, goe = go + ge;
     const int2 mid = band[r];
     // Both ways to the nearest single row, or the frame's end.
@@ -779,7 +781,7 @@ __device__ bool path_midpoint_warp(const int8_t* s1, const int8_t* s2, const int
     cells = __reduce_add_sync(kFull, cells);
     if (__any_sync(kFull, unknown) || span > kPathWarpCols ||
         cells + 32ll * (start[1] - start[0]) > (long long)M * N / (3 * nw) + 2000)
-        return false;
+        return -1;
 
     int lo[2], hi[2];
 #pragma unroll
@@ -811,7 +813,7 @@ __device__ bool path_midpoint_warp(const int8_t* s1, const int8_t* s2, const int
                 res32 = in ? (int)ldres<NC>(s1 + (h ? qq - 1 : qq)) : 0;
             }
             const int ends = __shfl_sync(kFull, v32.x, k & 31);
-            const int* const sub = X.smat() + 32 * __shfl_sync(kFull, res32, k & 31);
+            const int* const sub = smat + 32 * __shfl_sync(kFull, res32, k & 31);
             const int2 v = make_int2(ends, 0);
             const int nfrom = h ? min(path_hi(v), c0) : max(path_lo(v), c0);
             const int nto = h ? max(path_lo(v), B) : min(path_hi(v), B + N);
@@ -875,10 +877,8 @@ __device__ bool path_midpoint_warp(const int8_t* s1, const int8_t* s2, const int
     first = __reduce_min_sync(kFull, h1 == b1 ? first : INT_MAX);
     tied = __reduce_max_sync(kFull, h1 == b1 ? tied : -1);
     at2 = __reduce_max_sync(kFull, h2 == b2 ? at2 : -1);
-    type2 = b2 > b1;
-    midj = (type2 ? at2 : tied >= 0 ? tied : first) - B;
     __syncwarp();
-    return true;
+    return 2 * ((b2 > b1 ? at2 : tied >= 0 ? tied : first) - B) + (b2 > b1);
 }
 
 // Walks diff()'s frames from the box's own, 32 at a time. Adds identities,
@@ -956,17 +956,13 @@ __device__ __noinline__ int path_walk(const int8_t* s1, int n, const int8_t* s2,
         }
         for (unsigned wide = __ballot_sync(kFull, by == 1); wide; wide &= wide - 1) {
             const int l = __ffs(wide) - 1;
-            int mj;
-            bool t2;
-            const bool done = path_midpoint_warp<NC>(
+            const int mid = path_midpoint_warp<NC>(
                 s1, s2, band, rows, __shfl_sync(kFull, A, l), __shfl_sync(kFull, B, l), __shfl_sync(kFull, M, l),
-                __shfl_sync(kFull, N, l), __shfl_sync(kFull, tb, l), __shfl_sync(kFull, te, l), go, ge, nw, X, mj, t2);
+                __shfl_sync(kFull, N, l), __shfl_sync(kFull, tb, l), __shfl_sync(kFull, te, l), go, ge, nw, X.smat());
             if (lane == l) {
-                by = done ? 3 : 2;
-                if (done) {
-                    midj = mj;
-                    type2 = t2;
-                }
+                by = mid < 0 ? 2 : 3;
+                midj = mid >> 1;
+                type2 = mid & 1;
             }
         }
         if (lane < take && M == 1) {
