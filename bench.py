@@ -49,7 +49,7 @@ for _p in (REPO, os.path.join(REPO, "cuda-clustalw_gb300")):
         sys.path.insert(0, _p)
 
 FP64_NOMINAL_TFLOPS = 1.25  # GB300 nominal dense fp64 (an FMA counts 2; the join's criterion has none)
-OPS_PER_CELL = 8  # E, F via __viaddmax (2), H-gap term (1), diag add + 3-way max (2), max tracking (2), score (1)
+OPS_PER_CELL = 5  # score and diagonal add (1), 3-way max (1), H-gap term (1), E and F via __viaddmax (2)
 INT32_LANES_PER_SM = 128
 ALU_PIPE_LANES_PER_SM = 64  # integer ALU pipe (IMNMX, IADD3, DPX): half the INT32 lane rate
 
@@ -866,7 +866,9 @@ def ours_arm(args):
     sm_max = float(peaks.get("sm_max_mhz", 2070.0))
     peak_tops = props.multi_processor_count * INT32_LANES_PER_SM * sm_max * 1e6 / 1e12
     cells_alg = fwd + rev + dif
-    achieved = cells_alg * OPS_PER_CELL / (ms / 1e3) / 1e12
+    # The two local sweeps compute every cell; of diff()'s cells, only those near
+    # the optimal paths (its path comes from rows the sweeps keep).
+    achieved = (fwd + rev) * OPS_PER_CELL / (ms / 1e3) / 1e12
     tpc, tsrc = traffic_per_cell()
     roofline = {
         "bound": "int32",

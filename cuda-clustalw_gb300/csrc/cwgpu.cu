@@ -1003,14 +1003,15 @@ cudaError_t launch_persistent(const cwgpu::PairArgs& g, int max_grid, size_t sme
 }
 
 // Warps per CTA for a launch of nlong long pairs: the knob, or, when it is 0,
-// 16 for at most half a pair per SM, 8 up to 2.5 pairs per SM, else 4
-// (measured on 3000- and 1523-residue families: 15 pairs 21.4 / 18.6 / 14.3
-// GCUPS with 16 / 8 / 4 warps; 190 pairs 137 / 171 / 151; 1,770 pairs 117 /
-// 187 / 248).
+// 16 for at most half a pair per SM, 8 up to 2 pairs per SM, else 4. Measured
+// on families of 1523 residues with 16 / 8 / 4 warps: 91 pairs 1.49 / 1.49 /
+// 1.84 ms, 231 pairs 3.10 / 2.64 / 3.00, 325 pairs 3.13 / 2.53 / 2.16; of 3000
+// residues: 91 pairs 4.4 / 4.7 / 6.1, 231 pairs 5.2 / 6.0 / 7.0, 325 pairs 8.1 /
+// 7.6 / 6.5.
 int cta_warps_for(const cwgpu_context* ctx, int64_t nlong) {
     if (ctx->cta_warps) return ctx->cta_warps;
     if (2 * nlong <= ctx->sm_count) return 16;
-    if (2 * nlong <= 5 * (int64_t)ctx->sm_count) return 8;
+    if (nlong <= 2 * (int64_t)ctx->sm_count) return 8;
     return 4;
 }
 
@@ -1038,11 +1039,14 @@ cudaError_t launch_cta(const cwgpu_context* ctx, const cwgpu::PairArgs& g, int p
 }
 
 // Long pairs of a launch run one CTA per pair when there are few of them: at
-// most cta_pairs, or, by default, a quarter of the long-pair kernel's warps
-// (below that one warp per pair leaves most SMs idle; measured crossover on
-// 1523-residue families between 190 and 1,770 pairs).
+// most cta_pairs, or, by default, two fifths of the long-pair kernel's warps
+// (below that one warp per pair leaves the SMs too few warps to hide a pair's
+// own latency). Measured on families of 400 / 1523 / 3000 residues, one warp
+// against 4-warp CTAs: 780 pairs 1.26 / 5.3 / 20.4 against 1.05 / 3.7 / 10.6 ms,
+// 1,176 pairs 1.26 / 6.0 against 1.07 / 4.5, 1,770 pairs 1.47 / 6.1 against 1.53 /
+// 6.1.
 bool use_cta(const cwgpu_context* ctx, int64_t nlong) {
-    const int64_t limit = ctx->cta_pairs >= 0 ? ctx->cta_pairs : (int64_t)ctx->grid * kWarpsPerBlock / 4;
+    const int64_t limit = ctx->cta_pairs >= 0 ? ctx->cta_pairs : (int64_t)ctx->grid * kWarpsPerBlock * 2 / 5;
     return nlong > 0 && nlong <= limit && ctx->grid_cta[log2_warps(cta_warps_for(ctx, nlong))] > 0;
 }
 

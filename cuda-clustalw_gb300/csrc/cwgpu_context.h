@@ -56,7 +56,7 @@ struct cwgpu_context {
     int tiny_m = 32, tiny_n = 16;    // Myers-Miller frames solved one per lane
     int short_rows = 128;            // pairs with a first sequence this short: short-pair kernel
     // One CTA per pair (k_pairwise_cta) for launches of at most cta_pairs long
-    // pairs (-1: a quarter of the long-pair kernel's warps): cta_warps warps
+    // pairs (-1: two fifths of the long-pair kernel's warps): cta_warps warps
     // per CTA (0: chosen by pairs per SM), Myers-Miller frames of at least
     // cta_large_rows rows divided by the whole CTA (0: per pair, the larger of
     // 512 and a third of its diff() box).
