@@ -885,16 +885,26 @@ void path_sizes(int nseqs, int n, int m, int grid, size_t* bytes, long long* slo
     *bytes = want;
 }
 
+// Without them (no memory left) the kernels divide by Myers-Miller; as much is
+// not asked for again, so that plans made meanwhile stay valid.
 int ensure_path(cwgpu_context* ctx) {
     path_sizes(ctx->nseqs, ctx->lmax, ctx->lmax, ctx->grid, &ctx->path_bytes, &ctx->path_slots);
     const size_t need = ctx->lmax > ctx->short_rows ? ctx->path_bytes * (size_t)ctx->path_slots : 0;
-    if (need > ctx->path_cap) {
+    if (need > ctx->path_cap && (ctx->path_denied == 0 || need < ctx->path_denied)) {
         dfree(ctx->d_path);
         ctx->path_cap = 0;
         ctx->generation++;
-        CW_CUDA(ctx, cudaMalloc(&ctx->d_path, need));
-        ctx->path_cap = need;
+        const cudaError_t e = cudaMalloc(&ctx->d_path, need);
+        if (e == cudaErrorMemoryAllocation) {
+            cudaGetLastError();
+            ctx->d_path = nullptr;
+            ctx->path_denied = need;
+        } else {
+            CW_CUDA(ctx, e);
+            ctx->path_cap = need;
+        }
     }
+    if (need > ctx->path_cap) ctx->path_slots = ctx->path_bytes > 0 ? (long long)(ctx->path_cap / ctx->path_bytes) : 0;
     return CWGPU_OK;
 }
 

@@ -88,7 +88,7 @@ struct cwgpu_context {
     size_t scratch_bytes = 0;
     // Slices for cwgpu_path.cuh, one per warp of the long-pair kernel.
     unsigned char* d_path = nullptr;
-    size_t path_cap = 0, path_bytes = 0;
+    size_t path_cap = 0, path_bytes = 0, path_denied = 0;
     long long path_slots = 0;
     unsigned long long* d_counter = nullptr;  // [0] queue head, [1..3] cell counts, [4] short-pair queue head
     int* d_err = nullptr;

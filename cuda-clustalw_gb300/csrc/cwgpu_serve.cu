@@ -661,7 +661,10 @@ int cwgpu_server_create(int device, const int32_t* matrix, const cwgpu_params* p
         if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&s->rounds[i].s2, cudaStreamNonBlocking);
         if (e == cudaSuccess) e = cudaMalloc(&s->d_counter[i], 8 * sizeof(unsigned long long));
         if (e == cudaSuccess) e = cudaMalloc(&s->d_scratch[i], slots * 2 * (opts->max_seq_len + 1) * sizeof(int2));
-        if (e == cudaSuccess) e = cudaMalloc(&s->d_path[i], slots / 2 * s->path_bytes);
+        if (e == cudaSuccess && cudaMalloc(&s->d_path[i], slots / 2 * s->path_bytes) != cudaSuccess) {
+            cudaGetLastError();  // no memory left for them: Myers-Miller
+            s->d_path[i] = nullptr;
+        }
         if (e == cudaSuccess) e = cudaEventCreateWithFlags(&s->rounds[i].ev, cudaEventDisableTiming);
         if (e == cudaSuccess) e = cudaEventCreateWithFlags(&s->rounds[i].fork, cudaEventDisableTiming);
         if (e == cudaSuccess) e = cudaEventCreateWithFlags(&s->rounds[i].join, cudaEventDisableTiming);
