@@ -911,6 +911,7 @@ __device__ __noinline__ int path_walk(const int8_t* s1, int n, const int8_t* s2,
     int sp = 1;
     for (;;) {
         if (sp == 0 && nask == 0) break;
+        // Not yet dealt out, stack and asks hold fewer than 4 * 16 frames: there is room for them.
         if (nask > 0 && (sp == 0 || !dealt)) {
             while (nask > 0 && sp + 32 < cap - 96)
                 path_ask<NC>(seq1, n, seq2, m, p, A0, B0, se1, se2, go, ge, X, stack, sp, nlist, nask, dealt || w == 0);
