@@ -155,6 +155,7 @@ SIGNATURES = {
     "cwgpu_plan_results": (ctypes.c_int, [_vp, _vp, _vp]),
     "cwgpu_plan_device_dist": (_vp, [_vp]),
     "cwgpu_plan_cell_counts": (ctypes.c_int, [_vp, _vp]),
+    "cwgpu_plan_path_counts": (ctypes.c_int, [_vp, _vp]),
     "cwgpu_plan_kernel_count": (ctypes.c_int, [_vp]),
     "cwgpu_plan_pair_ctas": (ctypes.c_int, [_vp]),
     "cwgpu_plan_destroy": (None, [_vp]),
@@ -426,6 +427,12 @@ class Plan:
         """(forward, reverse, diff) cell updates of the last run, as the reference counts them."""
         c = np.zeros(3, dtype=np.int64)
         self.ctx._check(self._lib.cwgpu_plan_cell_counts(self._h, _ptr(c)), "cwgpu_plan_cell_counts")
+        return tuple(int(x) for x in c)
+
+    def path_counts(self):
+        """(pairs whose path came from kept rows, frames of those left to divisions) of the last run."""
+        c = np.zeros(2, dtype=np.int64)
+        self.ctx._check(self._lib.cwgpu_plan_path_counts(self._h, _ptr(c)), "cwgpu_plan_path_counts")
         return tuple(int(x) for x in c)
 
     def kernel_count(self):

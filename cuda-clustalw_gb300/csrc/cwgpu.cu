@@ -36,6 +36,7 @@ namespace {
 
 constexpr int kWarpsPerBlock = 4;  // warps (= concurrent pairs) per CTA
 constexpr int kCounterWords = 8;   // cwgpu_context::d_counter
+constexpr int kPathCounter = 5;    // of those, the path's: pairs, frames left over
 
 // RS = rows per lane of every sweep: cwgpu::kR for the long-pair kernel,
 // cwgpu::kRShort for pairs whose first sequence has at most
@@ -547,6 +548,7 @@ __device__ void cta_pair(const cwgpu::PairArgs& g, long long q, CtaCtl& C, const
                 }
             }
         }
+        if (rest >= 0 && threadIdx.x == 0 && g.cells) cwgpu::count_path(g, rest);
         if (rest != 0) {
             int id = 0, mt = 0, score = 0;
             long long ce = 0;
@@ -1432,6 +1434,17 @@ int cwgpu_plan_cell_counts(cwgpu_plan* p, int64_t* counts) {
     unsigned long long c[3];
     CW_CUDA(ctx, cudaMemcpy(c, ctx->d_counter + 1, sizeof(c), cudaMemcpyDeviceToHost));
     for (int i = 0; i < 3; ++i) counts[i] = (int64_t)c[i];
+    return CWGPU_OK;
+}
+
+int cwgpu_plan_path_counts(cwgpu_plan* p, int64_t* counts) {
+    if (!p || !counts) return CWGPU_ERR_ARG;
+    cwgpu_context* ctx = p->ctx;
+    CW_CUDA(ctx, cudaSetDevice(ctx->device));
+    CW_CUDA(ctx, cudaDeviceSynchronize());
+    unsigned long long c[2];
+    CW_CUDA(ctx, cudaMemcpy(c, ctx->d_counter + kPathCounter, sizeof(c), cudaMemcpyDeviceToHost));
+    for (int i = 0; i < 2; ++i) counts[i] = (int64_t)c[i];
     return CWGPU_OK;
 }
 

@@ -1346,6 +1346,12 @@ __device__ __forceinline__ LongPair long_pair(const PairArgs& g, long long q, lo
     return p;
 }
 
+// A pair whose path came from the kept rows, but for `rest` frames.
+__device__ __forceinline__ void count_path(const PairArgs& g, int rest) {
+    atomicAdd(g.cells + 4, 1ULL);
+    if (rest > 0) atomicAdd(g.cells + 5, (unsigned long long)rest);
+}
+
 static __device__ __noinline__ void finish_long(const PairArgs& g, long long q, long long slot, PairEnds e,
                                                 const Env& env) {
     const Env X = env;
@@ -1382,6 +1388,7 @@ static __device__ __noinline__ void finish_long(const PairArgs& g, long long q, 
             atomicAdd(g.cells + 0, (unsigned long long)p.n * p.m);
             atomicAdd(g.cells + 1, reverse_cells(e));
             atomicAdd(g.cells + 2, (unsigned long long)dcells);
+            if (rest >= 0) count_path(g, rest);
         }
     }
     __syncwarp();

@@ -170,6 +170,11 @@ void* cwgpu_plan_device_dist(cwgpu_plan* plan);
  * (:351-414), counts[2] diff() inner-loop iterations (:450-566). These are the
  * iteration counts the reference itself executes for the same pairs. */
 int cwgpu_plan_cell_counts(cwgpu_plan* plan, int64_t* counts);
+/* Waits, then returns which way the plan's last run went: counts[0] long pairs
+ * whose alignment path came from the rows their sweeps kept, counts[1] frames
+ * of those left to Myers-Miller divisions. The other pairs were divided
+ * throughout. Results do not depend on it. */
+int cwgpu_plan_path_counts(cwgpu_plan* plan, int64_t* counts);
 /* Kernels one cwgpu_plan_launch runs (0, 1 or 2: long-pair and short-pair). */
 int cwgpu_plan_kernel_count(const cwgpu_plan* plan);
 /* 1 if the plan's long pairs run one CTA per pair (cwgpu_cta_tuning), 0 if
