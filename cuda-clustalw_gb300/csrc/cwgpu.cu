@@ -452,7 +452,7 @@ __device__ void cta_pair(const cwgpu::PairArgs& g, long long q, CtaCtl& C, const
         cwgpu::Best rb;
         cwgpu::Task t = cwgpu::local_task(s1, n, s2, m, go, nullptr);
         cwgpu::PathMem pm;
-        const bool path = !GEN && g.path && ge >= 1 && go <= cwgpu::kMaxPathOpen &&
+        const bool path = !GEN && g.path && cwgpu::path_penalties(n, m, go, ge) &&
                           cwgpu::path_mem(n, m, nw, g.path + (size_t)blockIdx.x * ca.path_bytes, ca.path_bytes, pm);
         cwgpu::RowSave save{path ? pm.fwd : nullptr, pm.stride, pm.every, 0, 1, n};
 #pragma unroll 1
@@ -509,7 +509,7 @@ __device__ void cta_pair(const cwgpu::PairArgs& g, long long q, CtaCtl& C, const
             // the whole CTA: one column of 100 DNA sequences of 1523 residues
             // 1.95 to 1.6 ms, the 15 pairs of six proteins of 3000 3.9 to 2.8
             // to 3.5 ms (by family).
-            if (path && max_score > 0) {
+            if (path && cwgpu::path_scores(max_score, go)) {
                 int2* const band = bufs + stride / 2;  // of warp 0: no sweep uses it
                 const cwgpu::PathMem own = cwgpu::path_of_warp(pm, warp);
                 if (threadIdx.x == 0) C.path_bad = 0;

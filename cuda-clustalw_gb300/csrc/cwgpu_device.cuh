@@ -1341,7 +1341,7 @@ __device__ __forceinline__ LongPair long_pair(const PairArgs& g, long long q, lo
     p.s2 = g.codes + g.offs[p.sj];
     p.go = g.go_table[min(p.n, p.m)];
     p.buf = g.scratch + (size_t)slot * 2 * (g.lmax + 1);
-    p.path = g.path && slot < g.path_slots && g.ge >= 1 && p.go <= kMaxPathOpen &&
+    p.path = g.path && slot < g.path_slots && path_penalties(p.n, p.m, p.go, g.ge) &&
              path_mem(p.n, p.m, 1, g.path + (size_t)slot * g.path_bytes, g.path_bytes, p.pm);
     return p;
 }
@@ -1362,7 +1362,7 @@ static __device__ __noinline__ void finish_long(const PairArgs& g, long long q, 
     int mm = 0, ident = 0, matches = 0;
     long long dcells = 0;
     int rest = -1;  // frames for mm_align; -1: the pair's own
-    if (p.path && e.max_score > 0 &&
+    if (p.path && path_scores(e.max_score, p.go) &&
         path_rows(p.pm, bufB, A0, B0, e.se1, e.se2, e.max_score, p.go, 0, 1) &&
         path_fill<true, false>(p.s1, p.n, p.s2, p.pm, bufB, A0, B0, e.se1, e.se2, e.max_score, p.go, g.ge, X, 0, 1)) {
         rest = path_walk<true, false>(p.s1, p.n, p.s2, p.m, p.pm, bufB, A0, B0, e.se1, e.se2, p.go, g.ge, X, ident, matches,

@@ -33,17 +33,32 @@
 //    through H of one cell (kPathTight). The few frames that are left, and those
 //    in boxes too wide for the slice, go to mm_align.
 //
-// Needs 0 <= gapOpen <= kMaxPathOpen and gapExtend >= 1: with a free extension
-// a gap at the box's corner would tie with the local optimum.
+// Needs gapExtend >= 1 (with a free extension a gap at the box's corner would
+// tie with the local optimum) and penalties and scores that stay far from the
+// placeholder for cells outside the rows' ranges (path_penalties, path_scores).
 #pragma once
 
 namespace cwgpu {
 
-constexpr int kMaxPathOpen = 1 << 26;
-constexpr int kPathLow = -(1 << 28);  // below every value of a cell on an optimal path
+constexpr int kPathLow = -(1 << 29);  // the value of a cell that no path is taken through
+constexpr int kMaxPathScore = 1 << 27;
+constexpr int kMaxPathGap = 1 << 28;
 constexpr int kPathRows = 4;          // rows per lane in the boxes
 constexpr int kMaxPathG = 4;          // rows between saved rows: 32 * 1, 2 or 4
 constexpr int kPathRing = 4;          // steps of forward values in flight
+
+// Whether kPathLow stands below everything it is compared with, and no sum of
+// two values leaves 32 bits. The saved rows and the boxes hold whole-pair
+// values, 0 to maxScore on an optimal path; the walk counts from a row where H
+// is 0, so there a cell on one has -maxScore to maxScore, a midpoint at least
+// -maxScore. Out of a placeholder a half gains at most maxScore + gapOpen and the
+// other half holds at most as much: 3 * (maxScore + gapOpen) < -kPathLow keeps
+// their sum below the midpoint's. Downwards a gap may run on from a
+// placeholder for as many columns as there are.
+__device__ __forceinline__ bool path_penalties(int n, int m, int go, int ge) {
+    return ge >= 1 && go <= kMaxPathScore && (long long)ge * max(n, m) <= kMaxPathGap;
+}
+__device__ __forceinline__ bool path_scores(int best, int go) { return best > 0 && best <= kMaxPathScore - go; }
 
 // A row's cells on optimal paths: through H, inside a vertical gap (no kind at
 // all: the row's box was too wide).

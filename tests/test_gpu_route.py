@@ -40,3 +40,51 @@ def test_route_is_reported(oracle_mod):
         assert run(ctx, oracle_mod, shorts, matrix, params, pairs) == (0, 0)  # the short-pair kernel divides
         free = dict(params, pw_gap_extend=0.0)
         assert run(ctx, oracle_mod, longs, matrix, free, pairs) == (0, 0)
+
+
+def gapped_pair(seed, head, middle, tail):
+    """A sequence with `middle` letters that match nothing, and one without
+    them; at the joint 17 letters that match on either side of the gap."""
+    rng = np.random.default_rng(seed)
+    a, b = (rng.integers(0, 4, size=k).astype(np.int8) for k in (head, tail))
+    joint = rng.integers(4, 8, size=(3, 17)).astype(np.int8)
+    return [np.concatenate([a, joint[0], np.full(middle, 8, np.int8), joint[1], b]), np.concatenate([a, joint[2], b])]
+
+
+def scaled_scheme(match, mismatch, gap_open, gap_extend):
+    """DNA rules (gap open 200, extension 100 per unit) over nine letters, of
+    which 4 to 7 all match each other."""
+    from clustalw_gb300 import load_matrix
+
+    matrix, params = load_matrix("dna")
+    matrix = np.full((32, 32), mismatch, dtype=np.int32)
+    matrix[np.arange(4), np.arange(4)] = match
+    matrix[4:8, 4:8] = match
+    return matrix, dict(params, pw_gap_open=gap_open, pw_gap_extend=gap_extend)
+
+
+@pytest.mark.parametrize("warps", [0, 16])  # one warp per pair, one CTA per pair
+@pytest.mark.parametrize(
+    "name, sizes, scheme, kept",
+    [
+        # A gap between two blocks of equal score that costs more than 2^28.
+        ("costly gap", (9104, 8768, 16704), (32767, -32768, 0.5, 327.67), 0),
+        # maxScore + gapOpen at 2^27: 4097 matches less the gap, and one more.
+        ("largest score", (1500, 300, 2580), (32767, -32768, 1.0, 1.0), 1),
+        ("score beyond", (1500, 300, 2581), (32767, -32768, 1.0, 1.0), 0),
+        # gapExtend times the longer sequence at 2^28: 8192 residues, and 8193.
+        ("largest gap", (4100, 7, 4051), (300, -300, 1.0, 327.67), 1),
+        ("gap beyond", (4100, 7, 4052), (300, -300, 1.0, 327.67), 0),
+    ],
+)
+def test_path_only_within_its_numbers(oracle_mod, warps, name, sizes, scheme, kept):
+    from clustalw_gb300 import native
+
+    matrix, params = scaled_scheme(*scheme)
+    with native.Context(0) as ctx:
+        if warps:
+            ctx.set_cta_tuning(1 << 30, warps)
+        else:
+            ctx.set_cta_tuning(max_pairs=0)
+        route = run(ctx, oracle_mod, gapped_pair(1, *sizes), matrix, params, np.array([[0, 1]], dtype=np.int32))
+        assert route[0] == kept
