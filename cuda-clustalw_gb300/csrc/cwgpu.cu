@@ -143,6 +143,8 @@ auto pair_kernel(bool general) {
 constexpr int kCtaMaxWarps = 16;
 constexpr int kCtaStack = 64;
 constexpr int kCtaSmall = 256;
+constexpr int kCtaFill = 32;  // frames taken from a list at a time, into either
+static_assert(kCtaFill <= kCtaStack && kCtaFill + 8 <= kCtaSmall, "");
 constexpr int kRootBit = 1 << 30;  // in Frame.z (M < 2^17): the pair's top frame
 
 struct CtaCtl {
@@ -310,8 +312,12 @@ __device__ void cta_diff(CtaCtl& C, const int8_t* s1, const int8_t* s1r, int n, 
         const int ns = C.nstack;
         if (ns == 0) {
             if (!list || next >= nlist) break;
-            __syncthreads();  // every thread has seen the empty stack before it is filled
-            const int upto = min(nlist, next + kCtaStack / 2);
+            // Room for all of the next frames in either place; the divisions
+            // that follow want four more places in C.small each.
+            if (C.nsmall > kCtaSmall - kCtaFill - 4)
+                cta_small_frames<RS, GEN>(C, s1, s1r, n, s2, s2r, m, go, ge, bufA, bufB, X, ca, ident, match, ncell);
+            __syncthreads();  // every thread has seen both counts before they change
+            const int upto = min(nlist, next + kCtaFill);
             if (threadIdx.x == 0) {
                 for (int k = next; k < upto; ++k) {
                     if (cta_large(list[k].z, list[k].w & ((1 << 29) - 1), large_rows))
@@ -321,9 +327,6 @@ __device__ void cta_diff(CtaCtl& C, const int8_t* s1, const int8_t* s1r, int n, 
                 }
             }
             next = upto;
-            __syncthreads();
-            if (C.nsmall > kCtaSmall - kCtaStack)
-                cta_small_frames<RS, GEN>(C, s1, s1r, n, s2, s2r, m, go, ge, bufA, bufB, X, ca, ident, match, ncell);
             __syncthreads();
             continue;
         }

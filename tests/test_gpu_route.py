@@ -10,9 +10,10 @@ pytestmark = pytest.mark.gpu
 FIELDS = ("fwd_score", "se1", "se2", "sb1", "sb2", "mm_score", "n_ident", "n_match")
 
 
-def run(ctx, oracle_mod, seqs, matrix, params, pairs):
+def run(ctx, oracle_mod, seqs, matrix, params, pairs, want=None):
     """The pairs of kept rows and the frames left over of one checked run."""
-    want = oracle_mod.align_pairs(seqs, matrix, params, pairs)
+    if want is None:
+        want = oracle_mod.align_pairs(seqs, matrix, params, pairs)
     ctx.set_matrix(matrix)
     ctx.set_params(params)
     ctx.upload_seqs(seqs)
@@ -88,3 +89,34 @@ def test_path_only_within_its_numbers(oracle_mod, warps, name, sizes, scheme, ke
             ctx.set_cta_tuning(max_pairs=0)
         route = run(ctx, oracle_mod, gapped_pair(1, *sizes), matrix, params, np.array([[0, 1]], dtype=np.int32))
         assert route[0] == kept
+
+
+def with_insertions(seed, parts, rows, columns):
+    """A sequence of parts * rows letters, and one with `columns` random ones in
+    the middle of each part: not at the rows diff() divides at down to the parts."""
+    rng = np.random.default_rng(seed)
+    halves = [rng.integers(0, 20, size=rows // 2).astype(np.int8) for _ in range(2 * parts)]
+    second = []
+    for a, b in zip(halves[::2], halves[1::2]):
+        second += [a, rng.integers(0, 20, size=columns).astype(np.int8), b]
+    return [np.concatenate(halves), np.concatenate(second)]
+
+
+def test_many_frames_left_to_a_cta(oracle_mod):
+    """Insertions wider than a box leave a frame each: more than the CTA takes
+    from its list at a time, and, divided by the CTA down to two rows, more
+    than its stack for one-warp frames holds."""
+    from clustalw_gb300 import load_matrix, native
+
+    matrix, params = load_matrix("dna")
+    matrix = np.array(matrix)
+    matrix[:20, :20] = np.where(np.eye(20, dtype=bool), 9, -4)
+    params = dict(params, int_scale=1, pw_gap_open=10.0, pw_gap_extend=1.0)
+    seqs, pairs = with_insertions(1, 64, 100, 430), np.array([[0, 1]], dtype=np.int32)
+    want = oracle_mod.align_pairs(seqs, matrix, params, pairs)
+    with native.Context(0) as ctx:
+        for warps in (2, 4, 16):
+            for large_rows in (2, 40, 0):
+                ctx.set_cta_tuning(1 << 30, warps, large_rows)
+                kept, left = run(ctx, oracle_mod, seqs, matrix, params, pairs, want)
+                assert kept == 1 and left > 32
