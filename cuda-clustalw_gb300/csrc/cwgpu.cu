@@ -512,17 +512,17 @@ __device__ void cta_pair(const cwgpu::PairArgs& g, long long q, CtaCtl& C, const
             // the whole CTA: one column of 100 DNA sequences of 1523 residues
             // 1.95 to 1.6 ms, the 15 pairs of six proteins of 3000 3.9 to 2.8
             // to 3.5 ms (by family).
-            if (path && cwgpu::path_scores(max_score, go)) {
+            if (path && cwgpu::path_scores(max_score, go) && se1 - A0 >= cwgpu::kMinPathRows) {
                 int2* const band = bufs + stride / 2;  // of warp 0: no sweep uses it
                 const cwgpu::PathMem own = cwgpu::path_of_warp(pm, warp);
                 if (threadIdx.x == 0) C.path_bad = 0;
                 __syncthreads();
                 if (!cwgpu::path_rows(pm, band, A0, B0, se1, se2, max_score, go, warp, nw)) C.path_bad = 1;
                 __syncthreads();
-                const bool rows_bad = C.path_bad;
+                const bool skip = C.path_bad || !cwgpu::path_pays(pm, A0, B0, se1, se2);
                 __syncthreads();  // every thread has read it before a warp sets it again
-                if (!rows_bad && !cwgpu::path_fill<true, true>(s1, n, s2, own, band, A0, B0, se1, se2, max_score, go, ge, X,
-                                                         warp, nw))
+                if (skip || !cwgpu::path_fill<true, true>(s1, n, s2, own, band, A0, B0, se1, se2, max_score, go, ge, X,
+                                                     warp, nw))
                     C.path_bad = 1;
                 __syncthreads();
                 if (!C.path_bad) {

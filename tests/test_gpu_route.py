@@ -29,11 +29,22 @@ def run(ctx, oracle_mod, seqs, matrix, params, pairs, want=None):
     return route
 
 
+def related(n, length, seed):
+    """Copies of one sequence with a tenth of the residues replaced and a few lost."""
+    rng = np.random.default_rng(seed)
+    root = rng.integers(0, 20, size=length).astype(np.int8)
+    out = []
+    for _ in range(n):
+        s = np.where(rng.random(length) < 0.1, rng.integers(0, 20, size=length), root).astype(np.int8)
+        out.append(np.delete(s, rng.integers(0, length, size=3)))
+    return out
+
+
 def test_route_is_reported(oracle_mod):
     from clustalw_gb300 import load_matrix, native, synth
 
     matrix, params = load_matrix("protein")
-    longs, shorts = synth.protein_family(6, 420, 3), synth.protein_family(6, 90, 4)
+    longs, shorts = related(6, 420, 3), related(6, 90, 4)
     pairs = synth.all_pairs(6)
     with native.Context(0) as ctx:
         ctx.set_cta_tuning(max_pairs=0)
@@ -120,3 +131,31 @@ def test_many_frames_left_to_a_cta(oracle_mod):
                 ctx.set_cta_tuning(1 << 30, warps, large_rows)
                 kept, left = run(ctx, oracle_mod, seqs, matrix, params, pairs, want)
                 assert kept == 1 and left > 32
+
+
+@pytest.mark.parametrize("warps", [0, 4])
+def test_weak_alignments_are_divided(oracle_mod, warps):
+    """Unrelated sequences leave nearly every column within a gap opening of the
+    optimum, where kept rows cost more than divisions; so they do for boxes of few rows."""
+    from clustalw_gb300 import load_matrix, native, synth
+
+    matrix, params = load_matrix("protein")
+    rng = np.random.default_rng(4)
+    weak = [rng.integers(0, 20, size=600).astype(np.int8) for _ in range(8)]
+    core = related(6, 60, 9)
+    local = [np.concatenate([rng.integers(0, 20, size=250), c, rng.integers(0, 20, size=250)]).astype(np.int8) for c in core]
+    strict, strict_params = load_matrix("dna")
+    strict[:20, :20] = np.where(np.eye(20, dtype=bool), 9, -6)
+    strict_params = dict(strict_params, int_scale=1, pw_gap_open=10.0, pw_gap_extend=1.0)
+    with native.Context(0) as ctx:
+        if warps:
+            ctx.upload_seqs(synth.protein_family(60, 700, 1))
+            ctx.set_matrix(matrix)
+            ctx.set_params(params)
+            ctx.align_pairs(np.array([[0, 1]], dtype=np.int32))  # memory for the kept rows of the small sets too
+            ctx.set_cta_tuning(1 << 30, warps)
+        else:
+            ctx.set_cta_tuning(max_pairs=0)
+        assert run(ctx, oracle_mod, weak, matrix, params, synth.all_pairs(8)) == (0, 0)
+        assert run(ctx, oracle_mod, local, strict, strict_params, synth.all_pairs(6)) == (0, 0)
+        assert run(ctx, oracle_mod, related(8, 600, 2), matrix, params, synth.all_pairs(8))[0] == 28
