@@ -36,7 +36,7 @@ namespace {
 
 constexpr int kWarpsPerBlock = 4;  // warps (= concurrent pairs) per CTA
 constexpr int kCounterWords = 8;   // cwgpu_context::d_counter
-constexpr int kPathCounter = 5;    // of those, the path's: pairs, frames left over
+constexpr int kPathCounter = 5;    // of those, the path's: pairs, frames left over (then divide_weak's)
 
 // RS = rows per lane of every sweep: cwgpu::kR for the long-pair kernel,
 // cwgpu::kRShort for pairs whose first sequence has at most

@@ -1352,6 +1352,19 @@ __device__ __forceinline__ void count_path(const PairArgs& g, int rest) {
     if (rest > 0) atomicAdd(g.cells + 5, (unsigned long long)rest);
 }
 
+// Whether this pair is divided because the path would cost more: when it is weak
+// and most of the launch's pairs before it were. A few weak pairs among related
+// ones take the path like the others: an SM whose warps run both ways at a time
+// loses more to instruction fetches (300 x 180 proteins, 6 % of the pairs weak:
+// 8.6 ms by the path alone, 10.5 by divisions alone, 10.7 with the weak pairs
+// divided; 300 unrelated sequences of 400: 32.1, 21.2 and 21.5).
+__device__ __forceinline__ bool divide_weak(const PairArgs& g, bool weak) {
+    unsigned long long seen = 0;  // weak pairs << 32 | pairs
+    if ((threadIdx.x & 31) == 0 && g.cells) seen = atomicAdd(g.cells + 6, ((unsigned long long)weak << 32) + 1);
+    seen = __shfl_sync(kFull, seen, 0);
+    return weak && 2 * (seen >> 32) >= (seen & 0xffffffffu);
+}
+
 static __device__ __noinline__ void finish_long(const PairArgs& g, long long q, long long slot, PairEnds e,
                                                 const Env& env) {
     const Env X = env;
@@ -1362,9 +1375,9 @@ static __device__ __noinline__ void finish_long(const PairArgs& g, long long q, 
     int mm = 0, ident = 0, matches = 0;
     long long dcells = 0;
     int rest = -1;  // frames for mm_align; -1: the pair's own
-    if (p.path && path_scores(e.max_score, p.go) && e.se1 - A0 >= kMinPathRows &&
+    if (p.path && path_scores(e.max_score, p.go) &&
         path_rows(p.pm, bufB, A0, B0, e.se1, e.se2, e.max_score, p.go, 0, 1) &&
-        path_pays(p.pm, A0, B0, e.se1, e.se2) &&
+        !divide_weak(g, e.se1 - A0 < kMinPathRows || !path_pays(p.pm, A0, B0, e.se1, e.se2)) &&
         path_fill<true, false>(p.s1, p.n, p.s2, p.pm, bufB, A0, B0, e.se1, e.se2, e.max_score, p.go, g.ge, X, 0, 1)) {
         rest = path_walk<true, false>(p.s1, p.n, p.s2, p.m, p.pm, bufB, A0, B0, e.se1, e.se2, p.go, g.ge, X, ident, matches,
                                dcells, 0, 1);
