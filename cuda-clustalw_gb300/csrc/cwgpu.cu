@@ -117,13 +117,14 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32, 5)
     }
 }
 
-// The kernel for pairs whose rows per lane are RS.
+// The kernel for pairs whose rows per lane are RS. Without kept rows the
+// long-pair kernel is the one that has the divisions inline: beside the path's
+// code they wait for instructions (300 unrelated sequences of 200 residues 6.4
+// ms, in k_pairwise_long 8.9).
 template <int RS>
-auto pair_kernel(bool general) {
-    if constexpr (RS == cwgpu::kR)
-        return general ? k_pairwise<RS, true> : k_pairwise_long;
-    else
-        return general ? k_pairwise<RS, true> : k_pairwise<RS, false>;
+auto pair_kernel(bool general, bool path) {
+    if (RS == cwgpu::kR && path && !general) return k_pairwise_long;
+    return general ? k_pairwise<RS, true> : k_pairwise<RS, false>;
 }
 
 // ---- one CTA per pair: the pair's stripes shared by the warps of a CTA ------
@@ -815,12 +816,12 @@ int refresh_derived(cwgpu_context* ctx) {
 
 size_t block_smem(int K, int warps) { return (size_t)cwgpu::warp_region_bytes(K) * warps; }
 
-// CTAs of k_pairwise<RS> (either form) that fit on all SMs at once for an
+// CTAs of the kernels for RS rows per lane that fit on all SMs at once for an
 // alphabet of K codes.
 template <int RS>
 cudaError_t pair_grid(int K, int sm_count, int* grid) {
     int fit = INT_MAX;
-    for (auto* k : {pair_kernel<RS>(false), pair_kernel<RS>(true)}) {
+    for (auto* k : {pair_kernel<RS>(false, false), pair_kernel<RS>(true, false), pair_kernel<RS>(false, true)}) {
         int per_sm = 0;
         cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                              (int)block_smem(CWGPU_NUMRES, kWarpsPerBlock));
@@ -896,7 +897,7 @@ void path_sizes(int nseqs, int n, int m, int grid, size_t* bytes, long long* slo
 // not asked for again, so that plans made meanwhile stay valid.
 int ensure_path(cwgpu_context* ctx) {
     path_sizes(ctx->nseqs, ctx->lmax, ctx->lmax, ctx->grid, &ctx->path_bytes, &ctx->path_slots);
-    const size_t need = ctx->lmax > ctx->short_rows ? ctx->path_bytes * (size_t)ctx->path_slots : 0;
+    const size_t need = ctx->lmax > ctx->short_rows && ctx->lmax >= cwgpu::kMinPathLength ? ctx->path_bytes * (size_t)ctx->path_slots : 0;
     if (need > ctx->path_cap && (ctx->path_denied == 0 || need < ctx->path_denied)) {
         dfree(ctx->d_path);
         ctx->path_cap = 0;
@@ -964,7 +965,7 @@ cwgpu::PairArgs make_args(cwgpu_context* ctx, const int32_t* d_pairs, const int3
     g.tiny_m = ctx->tiny_m;
     g.tiny_n = ctx->tiny_n;
     g.general = ctx->general_gaps;
-    g.path = ctx->d_path;
+    g.path = ctx->lmax >= cwgpu::kMinPathLength ? ctx->d_path : nullptr;
     g.path_bytes = ctx->path_bytes;
     g.path_slots = ctx->path_slots;
     return g;
@@ -1016,7 +1017,7 @@ cudaError_t launch_persistent(const cwgpu::PairArgs& g, int max_grid, size_t sme
     attr[0].val.priority = priority;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, pair_kernel<RS>(g.general), g, -1LL);
+    return cudaLaunchKernelEx(&cfg, pair_kernel<RS>(g.general, g.path), g, -1LL);
 }
 
 // Warps per CTA for a launch of nlong long pairs: the knob, or, when it is 0,
@@ -1561,8 +1562,8 @@ int cwgpu_align_pairs_plain(cwgpu_context* ctx, const int32_t* pairs, int64_t np
     if (e == cudaSuccess) {
         cwgpu::PairArgs g = make_args(ctx, d_pairs, nullptr, npairs, d_dist, d_stats);
         for (int64_t q = 0; q < npairs && e == cudaSuccess; ++q) {
-            auto* const k = short_pair(ctx, pairs, q) ? pair_kernel<cwgpu::kRShort>(g.general)
-                                                      : pair_kernel<cwgpu::kR>(g.general);
+            auto* const k = short_pair(ctx, pairs, q) ? pair_kernel<cwgpu::kRShort>(g.general, false)
+                                                      : pair_kernel<cwgpu::kR>(g.general, g.path);
             k<<<1, 32, block_smem(ctx->K, 1), ctx->stream>>>(g, (long long)q);
             e = cudaGetLastError();
         }

@@ -160,6 +160,7 @@ struct Round {
     unsigned char* d = nullptr;
     size_t cap_d = 0;
     int64_t n = 0, nlong = 0, nseq = 0;
+    int lmax = 0;  // of the sequences of the round's jobs
     bool stats = false;
     // byte offsets: pairs at 0, then order, items, sequence offsets, lengths,
     // residue counts (copied), then distances and statistics (device only)
@@ -397,12 +398,14 @@ int64_t build_round(cwgpu_server* s, Round& r) {
     std::vector<uint16_t> key((size_t)n);
     std::vector<int64_t> start(2 * kBuckets + 1, 0);
     int64_t k = 0, base = 0;
+    r.lmax = 0;
     for (const Take& t : taken) {
         const Job* j = t.j;
         const int64_t codes_off = (int64_t)(j->desc.codes - reinterpret_cast<const int8_t*>(s->arena));
         for (int i = 0; i < j->nseqs; ++i) {
             soffs[base + i] = codes_off + j->offs[i];
             slens[base + i] = j->lens[i];
+            r.lmax = std::max(r.lmax, (int)j->lens[i]);
             snres[base + i] = j->nres[i];
         }
         int32_t si = t.si0, sj = t.sj0;
@@ -472,7 +475,7 @@ int launch_round(cwgpu_server* s, int ri, int64_t nitems) {
         gl.tiny_m = 32;
         gl.tiny_n = cwgpu::kTinyMaxN;
         gl.general = s->general_gaps;
-        gl.path = s->d_path[ri];
+        gl.path = r.lmax >= cwgpu::kMinPathLength ? s->d_path[ri] : nullptr;
         gl.path_bytes = s->path_bytes;
         gl.path_slots = 5LL * s->sm_count * wpc;
         cwgpu::PairArgs gs = gl;

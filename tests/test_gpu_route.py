@@ -159,3 +159,22 @@ def test_weak_alignments_are_divided(oracle_mod, warps):
         assert run(ctx, oracle_mod, weak, matrix, params, synth.all_pairs(8)) == (0, 0)
         assert run(ctx, oracle_mod, local, strict, strict_params, synth.all_pairs(6)) == (0, 0)
         assert run(ctx, oracle_mod, related(8, 600, 2), matrix, params, synth.all_pairs(8))[0] == 28
+
+
+@pytest.mark.parametrize("warps", [0, 2])
+def test_sets_of_one_stripe_are_divided(oracle_mod, warps):
+    """Kept rows only in sets with more than 256 residues in some sequence."""
+    from clustalw_gb300 import load_matrix, native
+
+    matrix, params = load_matrix("protein")
+    a, b = related(2, 303, 5)
+    pairs = np.array([[0, 1], [1, 0]], dtype=np.int32)
+    with native.Context(0) as ctx:
+        if warps:
+            ctx.set_cta_tuning(1 << 30, warps)
+        else:
+            ctx.set_cta_tuning(max_pairs=0)
+        for n, kept in ((130, 0), (256, 0), (257, 2), (300, 2)):
+            # More short sequences: a set of two would leave two warps too small a slice.
+            seqs = [a[:n], b[:n]] + [b[:40]] * 8
+            assert run(ctx, oracle_mod, seqs, matrix, params, pairs)[0] == kept
