@@ -320,17 +320,21 @@ __host__ __device__ inline bool padding_sound(int go, int ge) {
 // the instruction cache.
 // The maximum is tracked per lane on the step's maximum over the lane's rows;
 // only when it reaches the lane's own maximum is its row looked up.
-// GEN: gap penalties outside the range the padding rows are sound for
-// (padding_sound): rows of the stripe past the task's last row pass the row
-// above through, two selects per cell, so the segment's last used lane still
-// emits the last real row.
+// PARTIAL: gap penalties outside the range the padding rows are sound for
+// (padding_sound) and a stripe that the task's last row may end inside: the rows
+// past it pass the row above through, two selects per cell, so the segment's
+// last used lane still emits the last real row. One copy of the step, which
+// tests its range: with three the general kernels, which have most forms of it,
+// wait for instructions (proteins with a negative gap opening, 100 x 400 and 60 x
+// 1000: 4.60 and 6.50 ms against 4.13 and 6.83; the selects in every stripe, as
+// once, 4.51 and 7.18).
 // A lane with `writer` set stores its last row's (H, E) to `own`; the row above
 // the stripe is read from `above`.
 // MW: the stripe is one of a sweep shared by several warps (MwSync): before a
 // chunk of the row above is loaded the predecessor's progress is awaited, and
 // the lane with the boundary row publishes its progress between chunks (inside
 // the step, with its column test, a column sweep of 1523 x 1523 took 855 k cycles instead of 760 k).
-template <int R, int W, int MODE, bool GEN, bool NC, bool MW = false>
+template <int R, int W, int MODE, bool PARTIAL, bool NC, bool MW = false>
 __device__ __forceinline__ void run_stripe(int nsteps, int fill, bool first, const Task& T, SweepState<R>& S, int sl,
                                            int nvalid, const int2* above, int2* own, bool writer, int ge, int goe,
                                            int thresh, const uint16_t* prof_lane, const StripeIO& io = StripeIO{},
@@ -364,7 +368,7 @@ __device__ __forceinline__ void run_stripe(int nsteps, int fill, bool first, con
             const int g = h - goe;
             d = S.hl[k];
             S.fp[k] = __viaddmax_s32(S.fp[k], -ge, g);
-            if (GEN) {
+            if (PARTIAL) {
                 const bool v = k < nvalid;
                 const int en = __viaddmax_s32(e, -ge, g);
                 elast = v ? e : elast;
@@ -427,14 +431,19 @@ __device__ __forceinline__ void run_stripe(int nsteps, int fill, bool first, con
     };
 
     int t = 0;
-    for (; t < fill; ++t) step(t, true);
+    if (!PARTIAL)
+        for (; t < fill; ++t) step(t, true);
     publish(t);  // the fill may have been all of it
     if (t == W) next_chunk(t);
     while (t < nsteps) {
         const int tend = min(nsteps, (t | (W - 1)) + 1);
-        for (; t < tend; t += 2) {  // fill and W are even: at most one step past nsteps
-            step(t, false);
-            step(t + 1, false);
+        if (PARTIAL) {
+            for (; t < tend; ++t) step(t, true);
+        } else {
+            for (; t < tend; t += 2) {  // fill and W are even: at most one step past nsteps
+                step(t, false);
+                step(t + 1, false);
+            }
         }
         publish(t);
         if (t < nsteps) next_chunk(t);
@@ -594,8 +603,13 @@ __device__ __forceinline__ void sweep(const Task& T, int go, int ge, int track, 
         const int gbest = best.val;
         stripe_begin<R, MODE, GEN, NC>(T, S, lrow0, gbest, ge, goe, track, X, lane);
         stripe_chunks<R, W, rows_in_l2<MODE, false>()>(T, S, above, s == 0, sl, ge, goe);
-        run_stripe<R, W, MODE, GEN, NC>(nsteps_max, fill_steps(__reduce_max_sync(kFull, lused)), s == 0, T, S, sl, nvalid,
-                                        above, own, writer, ge, goe, thresh, prof_lane);
+        const int fill = fill_steps(__reduce_max_sync(kFull, lused));
+        if (GEN && (MODE == MODE_GLOBAL || !__all_sync(kFull, seg_rows == RPS)))
+            run_stripe<R, W, MODE, GEN, NC>(nsteps_max, fill, s == 0, T, S, sl, nvalid, above, own, writer, ge, goe,
+                                            thresh, prof_lane);
+        else
+            run_stripe<R, W, MODE, false, NC>(nsteps_max, fill, s == 0, T, S, sl, nvalid, above, own, writer, ge, goe,
+                                              thresh, prof_lane);
         if (MODE != MODE_GLOBAL)
             above = reinterpret_cast<const int2*>(__shfl_sync(kFull, reinterpret_cast<unsigned long long>(own), W - 1));
         if (MODE != MODE_GLOBAL) {
@@ -663,8 +677,12 @@ __device__ __forceinline__ void sweep_mw(const Task& T, int go, int ge, int trac
         stripe_begin<R, MODE, GEN, NC>(T, S, lrow0, gbest, ge, goe, track, X, lane);
         if (s > 0) mw_wait(mw, io.pred_slot, mw_word(mw, s - 1, min(T.cols, 2 * W)));
         stripe_chunks<R, W, rows_in_l2<MODE, true>()>(T, S, above, s == 0, sl, ge, goe);
-        run_stripe<R, W, MODE, GEN, NC, true>(nsteps, fill_steps(lused), s == 0, T, S, sl, nvalid, above, own, writer,
-                                              ge, goe, thresh, prof_lane, io, &mw);
+        if (GEN && (MODE == MODE_GLOBAL || seg_rows < RPS))
+            run_stripe<R, W, MODE, GEN, NC, true>(nsteps, fill_steps(lused), s == 0, T, S, sl, nvalid, above, own,
+                                                  writer, ge, goe, thresh, prof_lane, io, &mw);
+        else
+            run_stripe<R, W, MODE, false, NC, true>(nsteps, fill_steps(lused), s == 0, T, S, sl, nvalid, above, own,
+                                                    writer, ge, goe, thresh, prof_lane, io, &mw);
         if (MODE != MODE_GLOBAL) {
             const int wv = stripe_best<R>(S, lrow0, gbest, best);
             if (wv >= thresh && lane == 0) atomicMin((int*)stop, s);
