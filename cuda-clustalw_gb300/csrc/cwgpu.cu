@@ -878,26 +878,38 @@ int cta_grid(cwgpu_context* ctx, int warps, int* grid) {
     return CWGPU_OK;
 }
 
-// Slices for cwgpu_path.cuh: as many as the kernel has warps and the set has
-// ordered pairs, each large enough for the finest row spacing at the longest
-// lengths, or for what kPathBudget leaves it (the kernel then picks a wider
-// spacing, or Myers-Miller for pairs that do not fit).
+// Slices for cwgpu_path.cuh, each large enough for the finest row spacing at
+// the longest lengths, or for what kPathBudget leaves it (the kernel then picks
+// a wider spacing, or Myers-Miller for pairs that do not fit): one per warp of
+// the long-pair kernel or per CTA of k_pairwise_cta, whichever form a launch
+// takes, and no more than the set has ordered pairs. A CTA's warps have working
+// arrays of their own, so its slice is the larger one.
 constexpr size_t kPathBudget = (size_t)4 << 30;
 
-void path_sizes(int nseqs, int n, int m, int grid, size_t* bytes, long long* slots) {
-    *slots = std::min<long long>((long long)grid * kWarpsPerBlock, (long long)nseqs * nseqs);
-    *bytes = 0;
-    if (*slots < 1 || n < 1) return;
-    size_t want = cwgpu::path_bytes(n, m, 1);
-    want = std::min((want + 255) & ~(size_t)255, (kPathBudget / (size_t)*slots) & ~(size_t)255);
-    *bytes = want;
+size_t path_slice(int lmax, int warps, long long slots) {
+    if (slots < 1 || lmax < 1) return 0;
+    const size_t want = (cwgpu::path_bytes(lmax, lmax, 1, warps) + 255) & ~(size_t)255;
+    return std::min(want, (kPathBudget / (size_t)slots) & ~(size_t)255);
+}
+
+// The bytes of all slices of any launch over the set.
+size_t path_need(cwgpu_context* ctx) {
+    const long long pairs = (long long)ctx->nseqs * ctx->nseqs;
+    ctx->path_slots = std::min<long long>((long long)ctx->grid * kWarpsPerBlock, pairs);
+    ctx->path_bytes = path_slice(ctx->lmax, 1, ctx->path_slots);
+    if (ctx->lmax <= ctx->short_rows || ctx->lmax < cwgpu::kMinPathLength) return 0;
+    size_t need = ctx->path_bytes * (size_t)ctx->path_slots;
+    for (int l = 1; l <= 4; ++l) {
+        const long long ctas = std::min<long long>(ctx->grid_cta[l], pairs);
+        need = std::max(need, path_slice(ctx->lmax, 1 << l, ctas) * (size_t)ctas);
+    }
+    return need;
 }
 
 // Without them (no memory left) the kernels divide by Myers-Miller; as much is
 // not asked for again, so that plans made meanwhile stay valid.
 int ensure_path(cwgpu_context* ctx) {
-    path_sizes(ctx->nseqs, ctx->lmax, ctx->lmax, ctx->grid, &ctx->path_bytes, &ctx->path_slots);
-    const size_t need = ctx->lmax > ctx->short_rows && ctx->lmax >= cwgpu::kMinPathLength ? ctx->path_bytes * (size_t)ctx->path_slots : 0;
+    const size_t need = path_need(ctx);
     if (need > ctx->path_cap && (ctx->path_denied == 0 || need < ctx->path_denied)) {
         dfree(ctx->d_path);
         ctx->path_cap = 0;
@@ -912,7 +924,8 @@ int ensure_path(cwgpu_context* ctx) {
             ctx->path_cap = need;
         }
     }
-    if (need > ctx->path_cap) ctx->path_slots = ctx->path_bytes > 0 ? (long long)(ctx->path_cap / ctx->path_bytes) : 0;
+    if (need > ctx->path_cap && ctx->path_bytes > 0)
+        ctx->path_slots = std::min(ctx->path_slots, (long long)(ctx->path_cap / ctx->path_bytes));
     return CWGPU_OK;
 }
 
@@ -1042,7 +1055,7 @@ cudaError_t launch_cta(const cwgpu_context* ctx, const cwgpu::PairArgs& g, int p
     CtaArgs ca;
     ca.large_rows = ctx->cta_large_rows;
     ca.limit_ns = 4000000000ULL;  // no legitimate hand-over waits this long
-    ca.path_bytes = (ctx->path_cap / (size_t)grid) & ~(size_t)255;
+    ca.path_bytes = std::min(path_slice(ctx->lmax, warps, grid), (ctx->path_cap / (size_t)grid) & ~(size_t)255);
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)grid);
     cfg.blockDim = dim3(warps * 32);

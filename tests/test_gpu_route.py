@@ -178,3 +178,19 @@ def test_sets_of_one_stripe_are_divided(oracle_mod, warps):
             # More short sequences: a set of two would leave two warps too small a slice.
             seqs = [a[:n], b[:n]] + [b[:40]] * 8
             assert run(ctx, oracle_mod, seqs, matrix, params, pairs)[0] == kept
+
+
+@pytest.mark.parametrize("warps", [0, 2, 4, 8, 16])
+@pytest.mark.parametrize("n, length", [(3, 300), (4, 700), (10, 500), (6, 1523), (40, 300)])
+def test_slices_fit_the_form_that_runs(oracle_mod, n, length, warps):
+    """A new context's memory for kept rows is enough for a set's pairs, whichever
+    form and width they run in; so the route does not depend on what the context
+    held before."""
+    from clustalw_gb300 import load_matrix, native, synth
+
+    matrix, params = load_matrix("protein")
+    pairs = synth.all_pairs(n)[-15:]
+    with native.Context(0) as ctx:
+        if warps:
+            ctx.set_cta_tuning(1 << 30, warps)
+        assert run(ctx, oracle_mod, related(n, length, 7), matrix, params, pairs)[0] == len(pairs)
