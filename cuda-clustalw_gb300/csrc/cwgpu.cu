@@ -1034,13 +1034,15 @@ cudaError_t launch_persistent(const cwgpu::PairArgs& g, int max_grid, size_t sme
 }
 
 // Warps per CTA for a launch of nlong long pairs: the knob, or, when it is 0,
-// 16 for at most half a pair per SM, 8 up to 2 pairs per SM, else 4. Measured
-// on families of 1523 residues with 16 / 8 / 4 warps: 91 pairs 1.49 / 1.49 /
-// 1.84 ms, 231 pairs 3.10 / 2.64 / 3.00, 325 pairs 3.13 / 2.53 / 2.16; of 3000
-// residues: 91 pairs 4.4 / 4.7 / 6.1, 231 pairs 5.2 / 6.0 / 7.0, 325 pairs 8.1 /
-// 7.6 / 6.5.
+// 16 for at most half a pair per SM, 8 up to 2 pairs per SM, else 4; always 4
+// for sets of one stripe, which have no stripes to share. Each measured in a
+// new context, on families of 1523 residues with 16 / 8 / 4 warps: 28 pairs 1.46 /
+// 1.43 / 1.80 ms, 153 pairs 1.91 / 1.49 / 1.88, 300 pairs 3.17 / 2.46 / 2.78, 435
+// pairs 4.04 / 3.43 / 2.93; of 3000 residues: 15 pairs 3.19 / 3.66 / 4.81, 78 pairs
+// 4.77 / 5.14 / 6.18; of 200: 28 pairs 0.276 / 0.253 / 0.241.
 int cta_warps_for(const cwgpu_context* ctx, int64_t nlong) {
     if (ctx->cta_warps) return ctx->cta_warps;
+    if (ctx->lmax < cwgpu::kMinPathLength) return 4;
     if (2 * nlong <= ctx->sm_count) return 16;
     if (nlong <= 2 * (int64_t)ctx->sm_count) return 8;
     return 4;
@@ -1072,13 +1074,18 @@ cudaError_t launch_cta(const cwgpu_context* ctx, const cwgpu::PairArgs& g, int p
 // Long pairs of a launch run one CTA per pair when there are few of them: at
 // most cta_pairs, or, by default, two fifths of the long-pair kernel's warps
 // (below that one warp per pair leaves the SMs too few warps to hide a pair's
-// own latency). Measured on families of 400 / 1523 / 3000 residues, one warp
-// against 4-warp CTAs: 780 pairs 1.26 / 5.3 / 20.4 against 1.05 / 3.7 / 10.6 ms,
-// 1,176 pairs 1.26 / 6.0 against 1.07 / 4.5, 1,770 pairs 1.47 / 6.1 against 1.53 /
-// 6.1.
+// own latency); in sets of one stripe, as many CTAs as run at once. Measured in
+// new contexts, one warp against 4-warp CTAs, families of 400 / 1523 residues: 780
+// pairs 1.11 / 7.0 against 0.79 / 4.6 ms, 990 pairs 1.16 / 7.1 against 0.82 / 4.9, 1,485
+// pairs 1.44 / 7.5 against 1.10 / 6.2; unrelated sequences of 400 / 1000: 990 pairs
+// 1.01 / 3.95 against 1.08 / 3.36, 1,485 pairs 1.14 / 4.30 against 1.47 / 4.48; families
+// of 130 / 200: 595 pairs 0.23 / 0.33 against 0.24 / 0.31, 780 pairs 0.25 / 0.36 against
+// 0.25 / 0.48, 990 pairs 0.26 / 0.37 against 0.27 / 0.51.
 bool use_cta(const cwgpu_context* ctx, int64_t nlong) {
-    const int64_t limit = ctx->cta_pairs >= 0 ? ctx->cta_pairs : (int64_t)ctx->grid * kWarpsPerBlock * 2 / 5;
-    return nlong > 0 && nlong <= limit && ctx->grid_cta[log2_warps(cta_warps_for(ctx, nlong))] > 0;
+    const int ctas = ctx->grid_cta[log2_warps(cta_warps_for(ctx, nlong))];
+    int64_t limit = ctx->lmax < cwgpu::kMinPathLength ? ctas : (int64_t)ctx->grid * kWarpsPerBlock * 2 / 5;
+    if (ctx->cta_pairs >= 0) limit = ctx->cta_pairs;
+    return nlong > 0 && nlong <= limit && ctas > 0;
 }
 
 // The queue-counter reset and one persistent launch per kernel: long pairs

@@ -233,8 +233,9 @@ int cwgpu_get_tuning(const cwgpu_context* ctx, cwgpu_tuning* tuning);
  * smaller frames go to a stack in shared memory from which the warps take
  * frames and to which they give back the children they make. Defaults:
  * max_pairs -1 (two fifths of the long-pair kernel's resident warps, 1,216 on a
- * GB300), warps 0 (16, 8 or 4 as the launch has at most 0.5, 2 or more pairs
- * per SM), large_rows 0 (per pair, the larger of 512 and a third of the rows
+ * GB300; in sets of at most 256 residues as many CTAs as run at once, 608),
+ * warps 0 (16, 8 or 4 as the launch has at most 0.5, 2 or more pairs per SM; 4 in
+ * sets of at most 256 residues), large_rows 0 (per pair, the larger of 512 and a third of the rows
  * of its diff() box: the top two levels of the recursion); max_pairs 0 turns
  * it off. The reference's own GPU form also
  * runs one CTA per pair (G/cuda/cudaFullPairwiseAlign.cu:369-468), as one

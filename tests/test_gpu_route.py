@@ -194,3 +194,33 @@ def test_slices_fit_the_form_that_runs(oracle_mod, n, length, warps):
         if warps:
             ctx.set_cta_tuning(1 << 30, warps)
         assert run(ctx, oracle_mod, related(n, length, 7), matrix, params, pairs)[0] == len(pairs)
+
+
+def test_weak_pairs_among_related_ones_take_the_path(oracle_mod):
+    """In a launch of mostly related pairs the weak ones go the same way; the
+    longer ones here reach the choice after the others."""
+    from clustalw_gb300 import load_matrix, native, synth
+
+    matrix, params = load_matrix("protein")
+    rng = np.random.default_rng(8)
+    seqs = related(22, 300, 1) + [rng.integers(0, 20, size=600).astype(np.int8) for _ in range(8)]
+    weak = synth.all_pairs(8) + 22
+    pairs = np.concatenate([synth.all_pairs(22), weak, weak[:, ::-1]]).astype(np.int32)
+    with native.Context(0) as ctx:
+        ctx.set_cta_tuning(max_pairs=0)
+        kept, left = run(ctx, oracle_mod, seqs, matrix, params, pairs)
+        assert kept > 231 and left > 0
+
+
+@pytest.mark.parametrize("n, length, ctas", [(20, 200, 1), (30, 250, 1), (38, 250, 0), (45, 200, 0), (45, 300, 1)])
+def test_sets_of_one_stripe_run_as_many_ctas_as_fit(n, length, ctas):
+    from clustalw_gb300 import load_matrix, native, synth
+
+    matrix, params = load_matrix("protein")
+    with native.Context(0) as ctx:
+        ctx.set_matrix(matrix)
+        ctx.set_params(params)
+        ctx.upload_seqs(related(n, length, 3))
+        plan = ctx.plan(synth.all_pairs(n))
+        assert plan.pair_ctas() == bool(ctas)
+        plan.close()
