@@ -169,7 +169,7 @@ struct CtaCtl {
 struct CtaArgs {
     int large_rows;
     unsigned long long limit_ns;
-    size_t path_bytes;  // of a CTA's slice of PairArgs::path
+    size_t path_bytes;  // a CTA's slice of PairArgs::path at most
 };
 
 // Maximum value, then lowest key, over the warps' results in C.
@@ -456,8 +456,10 @@ __device__ void cta_pair(const cwgpu::PairArgs& g, long long q, CtaCtl& C, const
         cwgpu::Best rb;
         cwgpu::Task t = cwgpu::local_task(s1, n, s2, m, go, nullptr);
         cwgpu::PathMem pm;
-        const bool path = !GEN && g.path && cwgpu::path_penalties(n, m, go, ge) &&
-                          cwgpu::path_mem(n, m, nw, g.path + (size_t)blockIdx.x * ca.path_bytes, ca.path_bytes, pm);
+        const cwgpu::PathPool pool = g.path ? *g.path : cwgpu::PathPool{nullptr, 0};
+        const size_t slice = min(ca.path_bytes, pool.bytes / gridDim.x & ~(size_t)255);
+        const bool path = !GEN && cwgpu::path_penalties(n, m, go, ge) &&
+                          cwgpu::path_mem(n, m, nw, pool.base + blockIdx.x * slice, slice, pm);
         cwgpu::RowSave save{path ? pm.fwd : nullptr, pm.stride, pm.every, 0, 1, n};
 #pragma unroll 1
         for (int pass = 0; pass < 2; ++pass) {
@@ -745,7 +747,7 @@ int stage_inputs(cwgpu_context* ctx) {
     if (total > ctx->cap_in) {
         dfree(ctx->d_in);
         ctx->cap_in = 0;
-        CW_CUDA(ctx, cudaMalloc(&ctx->d_in, total));
+        CW_CUDA(ctx, cwgpu_malloc(ctx->path, &ctx->d_in, total));
         ctx->cap_in = total;
     }
     if (!ctx->ev_in) CW_CUDA(ctx, cudaEventCreateWithFlags(&ctx->ev_in, cudaEventDisableTiming));
@@ -895,10 +897,10 @@ size_t path_slice(int lmax, int warps, long long slots) {
 // The bytes of all slices of any launch over the set.
 size_t path_need(cwgpu_context* ctx) {
     const long long pairs = (long long)ctx->nseqs * ctx->nseqs;
-    ctx->path_slots = std::min<long long>((long long)ctx->grid * kWarpsPerBlock, pairs);
-    ctx->path_bytes = path_slice(ctx->lmax, 1, ctx->path_slots);
+    const long long slots = std::min<long long>((long long)ctx->grid * kWarpsPerBlock, pairs);
+    ctx->path_bytes = path_slice(ctx->lmax, 1, slots);
     if (ctx->lmax <= ctx->short_rows || ctx->lmax < cwgpu::kMinPathLength) return 0;
-    size_t need = ctx->path_bytes * (size_t)ctx->path_slots;
+    size_t need = ctx->path_bytes * (size_t)slots;
     for (int l = 1; l <= 4; ++l) {
         const long long ctas = std::min<long long>(ctx->grid_cta[l], pairs);
         need = std::max(need, path_slice(ctx->lmax, 1 << l, ctas) * (size_t)ctas);
@@ -906,27 +908,12 @@ size_t path_need(cwgpu_context* ctx) {
     return need;
 }
 
-// Without them (no memory left) the kernels divide by Myers-Miller; as much is
-// not asked for again, so that plans made meanwhile stay valid.
-int ensure_path(cwgpu_context* ctx) {
+// After a call's own buffers, which come first; asked for once per set.
+cudaError_t ensure_path(cwgpu_context* ctx) {
     const size_t need = path_need(ctx);
-    if (need > ctx->path_cap && (ctx->path_denied == 0 || need < ctx->path_denied)) {
-        dfree(ctx->d_path);
-        ctx->path_cap = 0;
-        ctx->generation++;
-        const cudaError_t e = cudaMalloc(&ctx->d_path, need);
-        if (e == cudaErrorMemoryAllocation) {
-            cudaGetLastError();
-            ctx->d_path = nullptr;
-            ctx->path_denied = need;
-        } else {
-            CW_CUDA(ctx, e);
-            ctx->path_cap = need;
-        }
-    }
-    if (need > ctx->path_cap && ctx->path_bytes > 0)
-        ctx->path_slots = std::min(ctx->path_slots, (long long)(ctx->path_cap / ctx->path_bytes));
-    return CWGPU_OK;
+    if (need <= ctx->path_asked) return cudaSuccess;
+    ctx->path_asked = need;
+    return ctx->path.grow(need);
 }
 
 int ensure_scratch(cwgpu_context* ctx) {
@@ -944,11 +931,11 @@ int ensure_scratch(cwgpu_context* ctx) {
     if (need > ctx->scratch_bytes) {
         dfree(ctx->d_scratch);
         ctx->scratch_bytes = 0;
-        CW_CUDA(ctx, cudaMalloc(&ctx->d_scratch, need));
+        CW_CUDA(ctx, cwgpu_malloc(ctx->path, &ctx->d_scratch, need));
         ctx->scratch_bytes = need;
         ctx->generation++;
     }
-    return ensure_path(ctx);
+    return CWGPU_OK;
 }
 
 cwgpu::PairArgs make_args(cwgpu_context* ctx, const int32_t* d_pairs, const int32_t* d_order, int64_t npairs,
@@ -978,9 +965,8 @@ cwgpu::PairArgs make_args(cwgpu_context* ctx, const int32_t* d_pairs, const int3
     g.tiny_m = ctx->tiny_m;
     g.tiny_n = ctx->tiny_n;
     g.general = ctx->general_gaps;
-    g.path = ctx->lmax >= cwgpu::kMinPathLength ? ctx->d_path : nullptr;
+    g.path = ctx->lmax >= cwgpu::kMinPathLength && ctx->path.base ? ctx->path.cell : nullptr;
     g.path_bytes = ctx->path_bytes;
-    g.path_slots = ctx->path_slots;
     return g;
 }
 
@@ -1057,7 +1043,7 @@ cudaError_t launch_cta(const cwgpu_context* ctx, const cwgpu::PairArgs& g, int p
     CtaArgs ca;
     ca.large_rows = ctx->cta_large_rows;
     ca.limit_ns = 4000000000ULL;  // no legitimate hand-over waits this long
-    ca.path_bytes = std::min(path_slice(ctx->lmax, warps, grid), (ctx->path_cap / (size_t)grid) & ~(size_t)255);
+    ca.path_bytes = path_slice(ctx->lmax, warps, grid);
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)grid);
     cfg.blockDim = dim3(warps * 32);
@@ -1148,6 +1134,65 @@ int check_kernel_error(cwgpu_context* ctx) {
 }
 
 }  // namespace
+
+cudaError_t cwgpu_path_memory::publish(unsigned char* p, size_t n) {
+    cudaError_t e = cudaDeviceSynchronize();  // a launch reads the cell more than once
+    const cwgpu::PathPool pool{p, n};
+    if (e == cudaSuccess) e = cudaMemcpy(cell, &pool, sizeof(pool), cudaMemcpyHostToDevice);
+    if (e != cudaSuccess) return e;
+    base = p;
+    bytes = n;
+    return cudaSuccess;
+}
+
+cudaError_t cwgpu_path_memory::create() {
+    const cudaError_t e = cudaMalloc(&cell, sizeof(cwgpu::PathPool));
+    return e == cudaSuccess ? publish(nullptr, 0) : e;
+}
+
+void cwgpu_path_memory::destroy() {
+    dfree(base);
+    bytes = 0;
+    dfree(cell);
+}
+
+cudaError_t cwgpu_path_memory::release() {
+    unsigned char* p = base;
+    if (!p) return cudaSuccess;
+    const cudaError_t e = publish(nullptr, 0);
+    if (e == cudaSuccess) cudaFree(p);
+    return e;
+}
+
+cudaError_t cwgpu_path_memory::grow(size_t need) {
+    if (need <= bytes) return cudaSuccess;
+    size_t avail = 0, all = 0;
+    cudaError_t e = cudaMemGetInfo(&avail, &all);
+    const size_t want = std::min(need, (avail + bytes) / 4) & ~(size_t)255;
+    if (e != cudaSuccess || want <= bytes) return e;
+    e = release();
+    if (e != cudaSuccess) return e;
+    unsigned char* p = nullptr;
+    e = cudaMalloc(&p, want);
+    if (e == cudaErrorMemoryAllocation) {
+        cudaGetLastError();
+        return cudaSuccess;
+    }
+    return e == cudaSuccess ? publish(p, want) : e;
+}
+
+cudaError_t cwgpu_malloc(cwgpu_path_memory& path, void** p, size_t n) {
+    cudaError_t e = cudaMalloc(p, n);
+    if (e != cudaErrorMemoryAllocation) return e;
+    cudaGetLastError();
+    *p = nullptr;
+    if (!path.base) return e;
+    const cudaError_t r = path.release();
+    if (r != cudaSuccess) return r;
+    e = cudaMalloc(p, n);
+    if (e == cudaErrorMemoryAllocation) cudaGetLastError();
+    return e;
+}
 
 int cwgpu_stage_inputs(cwgpu_context* ctx) { return stage_inputs(ctx); }
 
@@ -1251,6 +1296,7 @@ int cwgpu_create(int device, cwgpu_context** out) {
     if (e == cudaSuccess) e = cudaMemset(ctx->d_counter, 0, kCounterWords * sizeof(unsigned long long));
     if (e == cudaSuccess) e = cudaMalloc(&ctx->d_err, sizeof(int));
     if (e == cudaSuccess) e = cudaMemset(ctx->d_err, 0, sizeof(int));
+    if (e == cudaSuccess) e = ctx->path.create();
     if (e != cudaSuccess) {
         cwgpu_destroy(ctx);
         return e == cudaErrorMemoryAllocation ? CWGPU_ERR_OOM : CWGPU_ERR_CUDA;
@@ -1269,7 +1315,7 @@ void cwgpu_destroy(cwgpu_context* ctx) {
     if (ctx->h_io) cudaFreeHost(ctx->h_io);
     if (ctx->ev_in) cudaEventDestroy(ctx->ev_in);
     dfree(ctx->d_scratch);
-    dfree(ctx->d_path);
+    ctx->path.destroy();
     dfree(ctx->d_counter);
     dfree(ctx->d_err);
     dfree(ctx->d_call);
@@ -1369,6 +1415,7 @@ int cwgpu_upload_seqs(cwgpu_context* ctx, int32_t nseqs, const int8_t* codes, co
     memcpy(ctx->dense_of, dense_of, sizeof(dense_of));
     memcpy(ctx->code_of, code_of, sizeof(code_of));
     ctx->has_seqs = true;
+    ctx->path_asked = 0;
     ctx->in_dirty = true;
     ctx->generation++;
     return CWGPU_OK;
@@ -1388,10 +1435,11 @@ int cwgpu_plan_create(cwgpu_context* ctx, const int32_t* pairs, int64_t npairs, 
     p->ctx = ctx;
     p->npairs = npairs;
     const size_t np = (size_t)std::max<int64_t>(npairs, 1);
-    cudaError_t e = cudaMalloc(&p->d_pairs, sizeof(int32_t) * 2 * np);
-    if (e == cudaSuccess) e = cudaMalloc(&p->d_order, sizeof(int32_t) * np);
-    if (e == cudaSuccess) e = cudaMalloc(&p->d_dist, sizeof(float) * np);
-    if (e == cudaSuccess) e = cudaMalloc(&p->d_stats, sizeof(cwgpu_pair_stats) * np);
+    cudaError_t e = cwgpu_malloc(ctx->path, &p->d_pairs, sizeof(int32_t) * 2 * np);
+    if (e == cudaSuccess) e = cwgpu_malloc(ctx->path, &p->d_order, sizeof(int32_t) * np);
+    if (e == cudaSuccess) e = cwgpu_malloc(ctx->path, &p->d_dist, sizeof(float) * np);
+    if (e == cudaSuccess) e = cwgpu_malloc(ctx->path, &p->d_stats, sizeof(cwgpu_pair_stats) * np);
+    if (e == cudaSuccess) e = ensure_path(ctx);
     if (e == cudaSuccess && npairs > 0) {
         std::vector<int32_t> order((size_t)npairs);
         work_order(ctx, pairs, npairs, order.data(), &p->nlong);
@@ -1526,9 +1574,10 @@ int cwgpu_align_pairs(cwgpu_context* ctx, const int32_t* pairs, int64_t npairs, 
     if (total > ctx->cap_call) {
         dfree(ctx->d_call);
         ctx->cap_call = 0;
-        CW_CUDA(ctx, cudaMalloc(&ctx->d_call, total));
+        CW_CUDA(ctx, cwgpu_malloc(ctx->path, &ctx->d_call, total));
         ctx->cap_call = total;
     }
+    CW_CUDA(ctx, ensure_path(ctx));
     CW_CUDA(ctx, pinned_grow(ctx->h_io, ctx->cap_h_io, total));
     int64_t nlong = 0;
     unsigned char* h = ctx->h_io;
@@ -1574,9 +1623,10 @@ int cwgpu_align_pairs_plain(cwgpu_context* ctx, const int32_t* pairs, int64_t np
     int32_t* d_pairs = nullptr;
     float* d_dist = nullptr;
     cwgpu_pair_stats* d_stats = nullptr;
-    cudaError_t e = cudaMalloc(&d_pairs, sizeof(int32_t) * 2 * npairs);
-    if (e == cudaSuccess) e = cudaMalloc(&d_dist, sizeof(float) * npairs);
-    if (e == cudaSuccess) e = cudaMalloc(&d_stats, sizeof(cwgpu_pair_stats) * npairs);
+    cudaError_t e = cwgpu_malloc(ctx->path, &d_pairs, sizeof(int32_t) * 2 * npairs);
+    if (e == cudaSuccess) e = cwgpu_malloc(ctx->path, &d_dist, sizeof(float) * npairs);
+    if (e == cudaSuccess) e = cwgpu_malloc(ctx->path, &d_stats, sizeof(cwgpu_pair_stats) * npairs);
+    if (e == cudaSuccess) e = ensure_path(ctx);
     if (e == cudaSuccess) e = cudaMemcpy(d_pairs, pairs, sizeof(int32_t) * 2 * npairs, cudaMemcpyHostToDevice);
     if (e == cudaSuccess) e = cudaMemsetAsync(ctx->d_counter, 0, kCounterWords * sizeof(unsigned long long), ctx->stream);
     if (e == cudaSuccess) {

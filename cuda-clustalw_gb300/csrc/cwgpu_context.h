@@ -26,6 +26,35 @@ int cwgpu_stage_inputs(cwgpu_context* ctx);
 // reset first, gs.counter = gl.counter + 4). cwgpu.cu.
 namespace cwgpu {
 struct PairArgs;
+struct PathPool;
+}
+
+// Device memory for kept rows (cwgpu_path.cuh), of a context or a round. Pairs
+// without a slice of it are divided instead, so it only ever takes memory that
+// is free, and gives it back when a buffer that must be had does not fit.
+// Launches hold the address of `cell`, which says where it is: it may move or go
+// between them (never while one runs), also for plans and graphs made earlier.
+struct cwgpu_path_memory {
+    cwgpu::PathPool* cell = nullptr;  // on the device
+    unsigned char* base = nullptr;
+    size_t bytes = 0;
+
+    cudaError_t create();
+    void destroy();
+    // At least `need` bytes, or a quarter of the free memory if that is less.
+    cudaError_t grow(size_t need);
+    cudaError_t release();
+
+private:
+    cudaError_t publish(unsigned char* p, size_t n);
+};
+
+// cudaMalloc that gives the memory for kept rows back and tries again when
+// there is too little.
+cudaError_t cwgpu_malloc(cwgpu_path_memory& path, void** p, size_t bytes);
+template <class T>
+cudaError_t cwgpu_malloc(cwgpu_path_memory& path, T** p, size_t bytes) {
+    return cwgpu_malloc(path, reinterpret_cast<void**>(p), bytes);
 }
 cudaError_t cwgpu_pair_kernel_grids(int K, int sm_count, int* grid, int* grid_short);
 int cwgpu_pair_kernel_warps_per_cta();
@@ -86,10 +115,9 @@ struct cwgpu_context {
     int go_len = 0;
     int2* d_scratch = nullptr;
     size_t scratch_bytes = 0;
-    // Slices for cwgpu_path.cuh, one per warp of the long-pair kernel.
-    unsigned char* d_path = nullptr;
-    size_t path_cap = 0, path_bytes = 0, path_denied = 0;
-    long long path_slots = 0;
+    cwgpu_path_memory path;
+    size_t path_bytes = 0;  // of a slice of the long-pair kernel
+    size_t path_asked = 0;  // most asked for since the sequences were uploaded
     unsigned long long* d_counter = nullptr;  // [0] queue head, [1..3] cell counts, [4] short-pair queue head
     int* d_err = nullptr;
     int grid = 0;        // persistent CTAs of the long-pair kernel

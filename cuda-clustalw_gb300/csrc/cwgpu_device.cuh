@@ -1184,9 +1184,8 @@ struct PairArgs {
     int gp1, gp2;  // remapped gap codes
     int K;         // remapped alphabet size
     int tiny_m, tiny_n;
-    unsigned char* path;  // the warps' slices for cwgpu_path.cuh, path_bytes each; nullptr: none
-    size_t path_bytes;
-    long long path_slots;  // warps that have a slice
+    const PathPool* path;  // on the device, for cwgpu_path.cuh; nullptr: none
+    size_t path_bytes;     // of a warp's slice of it
     int general;  // host: gap penalties outside padding_sound somewhere, take the GEN kernels
 };
 
@@ -1359,8 +1358,9 @@ __device__ __forceinline__ LongPair long_pair(const PairArgs& g, long long q, lo
     p.s2 = g.codes + g.offs[p.sj];
     p.go = g.go_table[min(p.n, p.m)];
     p.buf = g.scratch + (size_t)slot * 2 * (g.lmax + 1);
-    p.path = g.path && slot < g.path_slots && path_penalties(p.n, p.m, p.go, g.ge) &&
-             path_mem(p.n, p.m, 1, g.path + (size_t)slot * g.path_bytes, g.path_bytes, p.pm);
+    const PathPool pool = g.path ? *g.path : PathPool{nullptr, 0};
+    p.path = (size_t)(slot + 1) * g.path_bytes <= pool.bytes && path_penalties(p.n, p.m, p.go, g.ge) &&
+             path_mem(p.n, p.m, 1, pool.base + (size_t)slot * g.path_bytes, g.path_bytes, p.pm);
     return p;
 }
 

@@ -730,11 +730,11 @@ int ensure_tables(cwgpu_context* ctx, const Params& P) {
     F->d_start = nullptr;
     const size_t total = std::max<size_t>(ctx->host_codes.size(), 16);
     const int ns = std::max(1, ctx->nseqs);
-    FAST_CUDA(ctx, cudaMalloc(&F->d_orig, total));
-    FAST_CUDA(ctx, cudaMalloc(&F->d_kcode, total * sizeof(int16_t)));
-    FAST_CUDA(ctx, cudaMalloc(&F->d_pos, total * sizeof(uint16_t)));
-    FAST_CUDA(ctx, cudaMalloc(&F->d_start, (size_t)ns * (P.limit + 2) * sizeof(int32_t)));
-    if (!F->d_counter) FAST_CUDA(ctx, cudaMalloc(&F->d_counter, sizeof(unsigned long long)));
+    FAST_CUDA(ctx, cwgpu_malloc(ctx->path, &F->d_orig, total));
+    FAST_CUDA(ctx, cwgpu_malloc(ctx->path, &F->d_kcode, total * sizeof(int16_t)));
+    FAST_CUDA(ctx, cwgpu_malloc(ctx->path, &F->d_pos, total * sizeof(uint16_t)));
+    FAST_CUDA(ctx, cwgpu_malloc(ctx->path, &F->d_start, (size_t)ns * (P.limit + 2) * sizeof(int32_t)));
+    if (!F->d_counter) FAST_CUDA(ctx, cwgpu_malloc(ctx->path, &F->d_counter, sizeof(unsigned long long)));
     FAST_CUDA(ctx, cudaMemcpy(F->d_orig, ctx->host_codes.data(), ctx->host_codes.size(), cudaMemcpyHostToDevice));
     if (ctx->nseqs > 0) {
         k_fast_prep<<<ctx->nseqs, 256, sizeof(int) * (P.limit + 2), ctx->stream>>>(
@@ -772,7 +772,7 @@ int run_fast(cwgpu_context* ctx, const Params& P, const int32_t* d_pairs, const 
         if (F->d_ovf) FAST_CUDA(ctx, cudaFree(F->d_ovf));
         F->d_ovf = nullptr;
         F->ovf_bytes = 0;
-        FAST_CUDA(ctx, cudaMalloc(&F->d_ovf, ovf));
+        FAST_CUDA(ctx, cwgpu_malloc(ctx->path, &F->d_ovf, ovf));
         F->ovf_bytes = ovf;
     }
     const long long sort_stride = 2LL * ctx->lmax + 4;
@@ -781,7 +781,7 @@ int run_fast(cwgpu_context* ctx, const Params& P, const int32_t* d_pairs, const 
         if (F->d_sort) FAST_CUDA(ctx, cudaFree(F->d_sort));
         F->d_sort = nullptr;
         F->sort_bytes = 0;
-        FAST_CUDA(ctx, cudaMalloc(&F->d_sort, sortb));
+        FAST_CUDA(ctx, cwgpu_malloc(ctx->path, &F->d_sort, sortb));
         F->sort_bytes = sortb;
     }
     Args A;
@@ -858,10 +858,10 @@ int cwgpu_fast_align_pairs(cwgpu_context* ctx, const cwgpu_fast_params* p, const
         F->d_dist = nullptr;
         F->d_stats = nullptr;
         F->cap_pairs = 0;
-        FAST_CUDA(ctx, cudaMalloc(&F->d_pairs, sizeof(int32_t) * 2 * npairs));
-        FAST_CUDA(ctx, cudaMalloc(&F->d_order, sizeof(int32_t) * npairs));
-        FAST_CUDA(ctx, cudaMalloc(&F->d_dist, sizeof(double) * npairs));
-        FAST_CUDA(ctx, cudaMalloc(&F->d_stats, sizeof(cwgpu_fast_stats) * npairs));
+        FAST_CUDA(ctx, cwgpu_malloc(ctx->path, &F->d_pairs, sizeof(int32_t) * 2 * npairs));
+        FAST_CUDA(ctx, cwgpu_malloc(ctx->path, &F->d_order, sizeof(int32_t) * npairs));
+        FAST_CUDA(ctx, cwgpu_malloc(ctx->path, &F->d_dist, sizeof(double) * npairs));
+        FAST_CUDA(ctx, cwgpu_malloc(ctx->path, &F->d_stats, sizeof(cwgpu_fast_stats) * npairs));
         F->cap_pairs = npairs;
     }
     int32_t* d_pairs = F->d_pairs;

@@ -65,6 +65,12 @@ __device__ __forceinline__ bool path_penalties(int n, int m, int go, int ge) {
 }
 __device__ __forceinline__ bool path_scores(int best, int go) { return best > 0 && best <= kMaxPathScore - go; }
 
+// The memory for all slices as the launches find it: nullptr, 0 if there is none.
+struct PathPool {
+    unsigned char* base;
+    size_t bytes;
+};
+
 // A row's cells on optimal paths: through H, inside a vertical gap (no kind at
 // all: the row's box was too wide).
 enum { kPathH = 1, kPathD = 2, kPathTight = 4 };

@@ -192,8 +192,8 @@ struct cwgpu_server {
     cudaStream_t upload = nullptr;  // job uploads, waited for before the job's first round
     unsigned long long* d_counter[2] = {nullptr, nullptr};
     int2* d_scratch[2] = {nullptr, nullptr};
-    unsigned char* d_path[2] = {nullptr, nullptr};  // the long-pair kernel's slices (PairArgs::path)
-    size_t path_bytes = 0;
+    cwgpu_path_memory path[2];
+    size_t path_bytes = 0;  // of a slice of the long-pair kernel
     int32_t* d_go = nullptr;  // gap-open penalty by min(n, m), 0..max_seq_len
     int grid = 0, grid_short = 0, grid_K = -1;
     int prio_low = 0, prio_high = 0;
@@ -475,9 +475,8 @@ int launch_round(cwgpu_server* s, int ri, int64_t nitems) {
         gl.tiny_m = 32;
         gl.tiny_n = cwgpu::kTinyMaxN;
         gl.general = s->general_gaps;
-        gl.path = r.lmax >= cwgpu::kMinPathLength ? s->d_path[ri] : nullptr;
+        gl.path = r.lmax >= cwgpu::kMinPathLength && s->path[ri].base ? s->path[ri].cell : nullptr;
         gl.path_bytes = s->path_bytes;
-        gl.path_slots = 5LL * s->sm_count * wpc;
         cwgpu::PairArgs gs = gl;
         gs.order = gl.order + r.nlong;
         gs.npairs = r.n - r.nlong;
@@ -664,10 +663,8 @@ int cwgpu_server_create(int device, const int32_t* matrix, const cwgpu_params* p
         if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&s->rounds[i].s2, cudaStreamNonBlocking);
         if (e == cudaSuccess) e = cudaMalloc(&s->d_counter[i], 8 * sizeof(unsigned long long));
         if (e == cudaSuccess) e = cudaMalloc(&s->d_scratch[i], slots * 2 * (opts->max_seq_len + 1) * sizeof(int2));
-        if (e == cudaSuccess && cudaMalloc(&s->d_path[i], slots / 2 * s->path_bytes) != cudaSuccess) {
-            cudaGetLastError();  // no memory left for them: Myers-Miller
-            s->d_path[i] = nullptr;
-        }
+        if (e == cudaSuccess) e = s->path[i].create();
+        if (e == cudaSuccess) e = s->path[i].grow(slots / 2 * s->path_bytes);
         if (e == cudaSuccess) e = cudaEventCreateWithFlags(&s->rounds[i].ev, cudaEventDisableTiming);
         if (e == cudaSuccess) e = cudaEventCreateWithFlags(&s->rounds[i].fork, cudaEventDisableTiming);
         if (e == cudaSuccess) e = cudaEventCreateWithFlags(&s->rounds[i].join, cudaEventDisableTiming);
@@ -710,7 +707,7 @@ void cwgpu_server_destroy(cwgpu_server* s) {
         if (r.d) cudaFree(r.d);
         if (s->d_counter[i]) cudaFree(s->d_counter[i]);
         if (s->d_scratch[i]) cudaFree(s->d_scratch[i]);
-        if (s->d_path[i]) cudaFree(s->d_path[i]);
+        s->path[i].destroy();
         if (s->streams[i]) cudaStreamDestroy(s->streams[i]);
     }
     if (s->upload) cudaStreamDestroy(s->upload);
