@@ -522,7 +522,7 @@ __device__ void cta_pair(const cwgpu::PairArgs& g, long long q, CtaCtl& C, const
                 __syncthreads();
                 if (!cwgpu::path_rows(pm, band, A0, B0, se1, se2, max_score, go, warp, nw)) C.path_bad = 1;
                 __syncthreads();
-                const bool skip = C.path_bad || !cwgpu::path_pays(pm, A0, B0, se1, se2);
+                const bool skip = C.path_bad || !cwgpu::path_pays<16>(pm, A0, B0, se1, se2);
                 __syncthreads();  // every thread has read it before a warp sets it again
                 if (skip || !cwgpu::path_fill<true, true>(s1, n, s2, own, band, A0, B0, se1, se2, max_score, go, ge, X,
                                                      warp, nw))

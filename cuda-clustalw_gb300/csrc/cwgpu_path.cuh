@@ -471,12 +471,18 @@ constexpr int kMinPathRows = 64;  // of a box
 // 1523 residues, 8 % on unrelated ones. Boxes of fewer than 64 rows have too
 // little to divide (unrelated sequences of 30 to 2000 residues, most boxes that
 // small: within 3 % of the cheaper with this line, 8 % without).
+// A launch of few pairs, a CTA each, ends with its slowest pair, and there the
+// walk's asks are a chain while the divisions are shared by the warps: the line
+// is at a sixteenth (k cycles of 8 warps, path against divisions: 425 rows with 10
+// % of the columns near 1,066 against 709, 540 rows with 14 % 1,194 against 971; of 16
+// warps 2,741 rows with 20 % 5,270 against 3,900).
+template <int SHARE>
 __device__ __forceinline__ bool path_pays(const PathMem& p, int A0, int B0, int se1, int se2) {
     const int saved = path_box_count(p, A0, se1) - 1;
     int near = 0;
     for (int b = threadIdx.x & 31; b < saved; b += 32) near += p.span[b].w - p.span[b].z + 1;
     near = __reduce_add_sync(kFull, near);
-    return 4ll * p.every * near <= (long long)(se1 - A0) * (se2 - B0);
+    return (long long)SHARE * p.every * near <= (long long)(se1 - A0) * (se2 - B0);
 }
 
 // The entries of the rows between them; warp w of nw, boxes dealt in runs of
