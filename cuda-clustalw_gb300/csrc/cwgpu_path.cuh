@@ -475,14 +475,17 @@ constexpr int kMinPathRows = 64;  // of a box
 // walk's asks are a chain while the divisions are shared by the warps: the line
 // is at a sixteenth (k cycles of 8 warps, path against divisions: 425 rows with 10
 // % of the columns near 1,066 against 709, 540 rows with 14 % 1,194 against 971; of 16
-// warps 2,741 rows with 20 % 5,270 against 3,900).
+// warps 2,741 rows with 20 % 5,270 against 3,900, 2,907 with 9 % 2,730 against 3,930), and
+// from 1250 rows on, where the divisions outgrow the asks, at that many times
+// more (one pair of unrelated sequences of 30000 193 ms against 237).
 template <int SHARE>
 __device__ __forceinline__ bool path_pays(const PathMem& p, int A0, int B0, int se1, int se2) {
     const int saved = path_box_count(p, A0, se1) - 1;
     int near = 0;
     for (int b = threadIdx.x & 31; b < saved; b += 32) near += p.span[b].w - p.span[b].z + 1;
     near = __reduce_add_sync(kFull, near);
-    return (long long)SHARE * p.every * near <= (long long)(se1 - A0) * (se2 - B0);
+    const long long columns = (long long)SHARE * p.every * near, box = (long long)(se1 - A0) * (se2 - B0);
+    return columns <= box || (SHARE == 16 && 1250 * columns <= box * (se1 - A0));
 }
 
 // The entries of the rows between them; warp w of nw, boxes dealt in runs of
