@@ -300,12 +300,14 @@ void finish_job(cwgpu_server* s, Job* j) {
     s->jobs_done++;
 }
 
-cudaError_t grow_dev(unsigned char*& p, size_t& cap, size_t need) {
+// Short of memory, the rounds' kept rows give way.
+cudaError_t grow_dev(cwgpu_server* s, unsigned char*& p, size_t& cap, size_t need) {
     if (need <= cap && p) return cudaSuccess;
     if (p) cudaFree(p);
     p = nullptr;
     cap = 0;
-    const cudaError_t e = cudaMalloc(&p, need);
+    cudaError_t e = cwgpu_malloc(s->path[0], &p, need);
+    if (e == cudaErrorMemoryAllocation) e = cwgpu_malloc(s->path[1], &p, need);
     if (e == cudaSuccess) cap = need;
     return e;
 }
@@ -384,7 +386,7 @@ int64_t build_round(cwgpu_server* s, Round& r) {
     r.o_dist = r.bytes_in;
     r.o_stats = r.o_dist + up(4 * (size_t)n);
     r.bytes_all = r.o_stats + (stats ? sizeof(cwgpu_pair_stats) * (size_t)n : 0);
-    if (grow_pinned(r.h, r.cap_h, r.bytes_in) != cudaSuccess || grow_dev(r.d, r.cap_d, r.bytes_all) != cudaSuccess)
+    if (grow_pinned(r.h, r.cap_h, r.bytes_in) != cudaSuccess || grow_dev(s, r.d, r.cap_d, r.bytes_all) != cudaSuccess)
         return -1;
     int32_t* pairs = reinterpret_cast<int32_t*>(r.h);
     int32_t* ord = reinterpret_cast<int32_t*>(r.h + r.o_order);
@@ -664,11 +666,12 @@ int cwgpu_server_create(int device, const int32_t* matrix, const cwgpu_params* p
         if (e == cudaSuccess) e = cudaMalloc(&s->d_counter[i], 8 * sizeof(unsigned long long));
         if (e == cudaSuccess) e = cudaMalloc(&s->d_scratch[i], slots * 2 * (opts->max_seq_len + 1) * sizeof(int2));
         if (e == cudaSuccess) e = s->path[i].create();
-        if (e == cudaSuccess) e = s->path[i].grow(slots / 2 * s->path_bytes);
         if (e == cudaSuccess) e = cudaEventCreateWithFlags(&s->rounds[i].ev, cudaEventDisableTiming);
         if (e == cudaSuccess) e = cudaEventCreateWithFlags(&s->rounds[i].fork, cudaEventDisableTiming);
         if (e == cudaSuccess) e = cudaEventCreateWithFlags(&s->rounds[i].join, cudaEventDisableTiming);
     }
+    // Kept rows take what everything that must be had has left.
+    for (int i = 0; i < 2 && e == cudaSuccess; ++i) e = s->path[i].grow(slots / 2 * s->path_bytes);
     if (e != cudaSuccess) {
         cwgpu_server_destroy(s);
         return e == cudaErrorMemoryAllocation ? CWGPU_ERR_OOM : CWGPU_ERR_CUDA;

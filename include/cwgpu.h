@@ -82,7 +82,12 @@ typedef struct cwgpu_context cwgpu_context;
 /* ---- context ------------------------------------------------------------ */
 
 /* Creates a context on CUDA device `device`. No reference counterpart: the
- * reference class allocates its scratch in pairwiseAlign (:74-78). */
+ * reference class allocates its scratch in pairwiseAlign (:74-78). Besides the
+ * buffers a call needs, a context that aligns sequences of more than 256
+ * residues holds memory for rows its sweeps keep: up to 4 GiB, at most a quarter
+ * of what was free on the device. It is optional (pairs without it take longer,
+ * results are the same) and is given back when one of the context's buffers
+ * does not fit; other users of the device see it as taken. */
 int cwgpu_create(int device, cwgpu_context** out);
 /* Frees all device memory of the context. Replaces ~FullPairwiseAlign. */
 void cwgpu_destroy(cwgpu_context* ctx);
@@ -263,7 +268,10 @@ int cwgpu_cta_wait_probe(cwgpu_context* ctx, int64_t timeout_ns, int32_t* timed_
  * order as job slots and budget memory free up; their sequences and distances
  * stay resident until released. A scheduler thread runs rounds: one persistent
  * launch over pairs mixed from every admitted job, two rounds in flight, so
- * jobs that arrive while others run join the next round. */
+ * jobs that arrive while others run join the next round. Besides the budget a
+ * server holds its rounds' boundary rows and buffers and, if it takes sequences
+ * of more than 256 residues, memory for kept rows as a context does: up to 2 GiB,
+ * at most a quarter of what was free for each of the two rounds. */
 enum { CWGPU_JOB_QUEUED = 0, CWGPU_JOB_RUNNING = 1, CWGPU_JOB_DONE = 2, CWGPU_JOB_FAILED = 3 };
 typedef struct cwgpu_server_opts {
     int64_t memory_budget_bytes; /* arena for resident job data and results */

@@ -96,3 +96,29 @@ def test_memory_is_asked_for_again(held):
                 plan.close()
     assert kept[0][0] < kept[1][0] == len(pairs)
     assert np.array_equal(kept[0][1], kept[1][1])
+
+
+def test_a_server_needs_only_its_own_buffers():
+    """Created with room for the job memory and the boundary rows, but not for
+    kept rows beside them, and with buffers of a first round to come."""
+    from clustalw_gb300 import load_matrix, native, serve, synth
+
+    matrix, params = load_matrix("protein")
+    jobs = [related(40, 400, 5), related(300, 40, 6)]
+    with native.Context(0) as ctx:  # kernels loaded and stacks taken before memory is short
+        ctx.set_matrix(matrix)
+        ctx.set_params(params)
+        want = []
+        for seqs in jobs:
+            ctx.upload_seqs(seqs)
+            ctx.set_cta_tuning(max_pairs=0)
+            want.append(ctx.align_pairs(synth.all_pairs(len(seqs))))
+    # 512 MB of job memory; rows: 2 rounds x 6,080 warps x 2 x 4,097 x 8 bytes = 797 MB;
+    # one round's kept rows would be 1 GB more.
+    with device_full(leave=2000 * MB):
+        with serve.Server(matrix, params, memory_budget=512 * MB) as server:
+            ids = [server.submit(seqs) for seqs in jobs]
+            for job, w in zip(ids, want):
+                server.wait(job)
+                assert np.array_equal(server.result(job)[0], w)
+                server.release(job)
