@@ -1169,7 +1169,7 @@ cudaError_t cwgpu_path_memory::grow(size_t need) {
     size_t avail = 0, all = 0;
     cudaError_t e = cudaMemGetInfo(&avail, &all);
     const size_t want = std::min(need, (avail + bytes) / 4) & ~(size_t)255;
-    if (e != cudaSuccess || want <= bytes) return e;
+    if (e != cudaSuccess || want <= bytes || (want < need && want < 2 * bytes)) return e;  // not for little more
     e = release();
     if (e != cudaSuccess) return e;
     unsigned char* p = nullptr;

@@ -671,7 +671,8 @@ int cwgpu_server_create(int device, const int32_t* matrix, const cwgpu_params* p
         if (e == cudaSuccess) e = cudaEventCreateWithFlags(&s->rounds[i].join, cudaEventDisableTiming);
     }
     // Kept rows take what everything that must be had has left.
-    for (int i = 0; i < 2 && e == cudaSuccess; ++i) e = s->path[i].grow(slots / 2 * s->path_bytes);
+    for (int i = 0; i < 2 && e == cudaSuccess && opts->max_seq_len >= cwgpu::kMinPathLength; ++i)
+        e = s->path[i].grow(slots / 2 * s->path_bytes);
     if (e != cudaSuccess) {
         cwgpu_server_destroy(s);
         return e == cudaErrorMemoryAllocation ? CWGPU_ERR_OOM : CWGPU_ERR_CUDA;

@@ -224,3 +224,29 @@ def test_sets_of_one_stripe_run_as_many_ctas_as_fit(n, length, ctas):
         plan = ctx.plan(synth.all_pairs(n))
         assert plan.pair_ctas() == bool(ctas)
         plan.close()
+
+
+@pytest.mark.parametrize("warps", [2, 8, 16])
+@pytest.mark.parametrize("scheme", ["protein", "dna"])
+@pytest.mark.parametrize("kind", ["gaps", "close gaps", "wide gaps", "ties", "edges"])
+def test_a_cta_walks_the_path(oracle_mod, kind, scheme, warps):
+    """Rows, boxes and frames dealt over a CTA's warps, in a new context: gaps of
+    two and more rows at every recursion level, gaps wider than a box, ties, and
+    lengths around the rows kept and the rows of lanes and stripes."""
+    from clustalw_gb300 import load_matrix, native, synth
+    from test_gpu_path import sequences
+
+    seqs = sequences(kind, 200 + len(kind))
+    matrix, params = load_matrix(scheme)
+    if scheme == "dna":
+        seqs = [(s % 4).astype(np.int8) for s in seqs]
+        matrix[:20, :20] = np.where(np.eye(20, dtype=bool), 9, -4)
+        params = dict(params, int_scale=1, pw_gap_open=5.0, pw_gap_extend=2.0)
+    up = synth.all_pairs(len(seqs))
+    pairs = np.concatenate([up, up[:, ::-1]])
+    with native.Context(0) as ctx:
+        ctx.set_cta_tuning(1 << 30, warps)
+        kept, left = run(ctx, oracle_mod, seqs, matrix, params, pairs)
+    assert kept > 0
+    if kind == "edges":
+        assert (kept, left) == (len(pairs), 0)
