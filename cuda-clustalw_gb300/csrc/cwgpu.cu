@@ -160,6 +160,7 @@ struct CtaCtl {
     int mm;  // diff()'s score of the pair
     int nstack, nsmall, small_next;
     int path_bad;                  // a warp found the path cannot be had from the kept rows
+    int path_near;                 // columns near the optimum in the kept rows
     int path_rest[kCtaMaxWarps];   // frames each warp leaves to diff()'s divisions
     int lock, active;  // the shared frame stack `small`: its lock, warps holding a frame from it
     int4 stack[kCtaStack];  // large frames: (A, B, M | root, N | tb << 29 | te << 30)
@@ -518,11 +519,13 @@ __device__ void cta_pair(const cwgpu::PairArgs& g, long long q, CtaCtl& C, const
             if (path && cwgpu::path_scores(max_score, go) && se1 - A0 >= cwgpu::kMinPathRows) {
                 int2* const band = bufs + stride / 2;  // of warp 0: no sweep uses it
                 const cwgpu::PathMem own = cwgpu::path_of_warp(pm, warp);
-                if (threadIdx.x == 0) C.path_bad = 0;
+                if (threadIdx.x == 0) C.path_bad = C.path_near = 0;
                 __syncthreads();
-                if (!cwgpu::path_rows(pm, band, A0, B0, se1, se2, max_score, go, warp, nw)) C.path_bad = 1;
+                int near;
+                if (!cwgpu::path_rows(pm, band, A0, B0, se1, se2, max_score, go, warp, nw, near)) C.path_bad = 1;
+                if (lane == 0) atomicAdd(&C.path_near, near);
                 __syncthreads();
-                const bool skip = C.path_bad || !cwgpu::path_pays<16>(pm, A0, B0, se1, se2);
+                const bool skip = C.path_bad || !cwgpu::path_pays<16>(C.path_near, pm.every, se1 - A0, se2 - B0);
                 __syncthreads();  // every thread has read it before a warp sets it again
                 if (skip || !cwgpu::path_fill<true, true>(s1, n, s2, own, band, A0, B0, se1, se2, max_score, go, ge, X,
                                                      warp, nw))

@@ -1393,9 +1393,10 @@ static __device__ __noinline__ void finish_long(const PairArgs& g, long long q, 
     int mm = 0, ident = 0, matches = 0;
     long long dcells = 0;
     int rest = -1;  // frames for mm_align; -1: the pair's own
+    int near;
     if (p.path && path_scores(e.max_score, p.go) &&
-        path_rows(p.pm, bufB, A0, B0, e.se1, e.se2, e.max_score, p.go, 0, 1) &&
-        !divide_weak(g, e.se1 - A0 < kMinPathRows || !path_pays<4>(p.pm, A0, B0, e.se1, e.se2)) &&
+        path_rows(p.pm, bufB, A0, B0, e.se1, e.se2, e.max_score, p.go, 0, 1, near) &&
+        !divide_weak(g, e.se1 - A0 < kMinPathRows || !path_pays<4>(near, p.pm.every, e.se1 - A0, e.se2 - B0)) &&
         path_fill<true, false>(p.s1, p.n, p.s2, p.pm, bufB, A0, B0, e.se1, e.se2, e.max_score, p.go, g.ge, X, 0, 1)) {
         rest = path_walk<true, false>(p.s1, p.n, p.s2, p.m, p.pm, bufB, A0, B0, e.se1, e.se2, p.go, g.ge, X, ident, matches,
                                dcells, 0, 1);

@@ -435,9 +435,11 @@ __device__ __forceinline__ int path_box_count(const PathMem& p, int A0, int se1)
 
 // The entries of the saved rows, and the box's own first and last row; warp w
 // of nw. One warp follows the columns down; several start every row at the
-// box's first. False if a row has no cell on an optimal path.
+// box's first. near: the columns near the optimum, added up over the warp's rows.
+// False if a row has no cell on an optimal path.
 __device__ inline bool path_rows(const PathMem& p, int2* band, int A0, int B0, int se1, int se2, int best, int go, int w,
-                                 int nw) {
+                                 int nw, int& near) {
+    near = 0;
     const int lane = threadIdx.x & 31;
     if (lane == 0 && w == 0) {
         band[0] = path_entry(0, 0, kPathH);
@@ -449,6 +451,7 @@ __device__ inline bool path_rows(const PathMem& p, int2* band, int A0, int B0, i
         int lo, hi, kinds, near_lo, near_hi;
         if (nw > 1) jl = B0;
         if (!path_row(p, i, jl, se2, best, go, lo, hi, kinds, near_lo, near_hi)) return false;
+        near += near_hi - near_lo + 1;
         if (lane == 0) {
             band[i - A0] = path_entry(lo - B0, hi - B0, kinds);
             p.span[b] = make_int4(lo, hi, near_lo, near_hi);
@@ -479,13 +482,9 @@ constexpr int kMinPathRows = 64;  // of a box
 // from 1250 rows on, where the divisions outgrow the asks, at that many times
 // more (one pair of unrelated sequences of 30000 193 ms against 237).
 template <int SHARE>
-__device__ __forceinline__ bool path_pays(const PathMem& p, int A0, int B0, int se1, int se2) {
-    const int saved = path_box_count(p, A0, se1) - 1;
-    int near = 0;
-    for (int b = threadIdx.x & 31; b < saved; b += 32) near += p.span[b].w - p.span[b].z + 1;
-    near = __reduce_add_sync(kFull, near);
-    const long long columns = (long long)SHARE * p.every * near, box = (long long)(se1 - A0) * (se2 - B0);
-    return columns <= box || (SHARE == 16 && 1250 * columns <= box * (se1 - A0));
+__device__ __forceinline__ bool path_pays(int near, int every, int rows, int cols) {
+    const long long columns = (long long)SHARE * every * near, box = (long long)rows * cols;
+    return columns <= box || (SHARE == 16 && 1250 * columns <= box * rows);
 }
 
 // The entries of the rows between them; warp w of nw, boxes dealt in runs of
