@@ -41,10 +41,10 @@ constexpr int kPathCounter = 5;    // of those, the path's: pairs, frames left o
 // RS = rows per lane of every sweep: cwgpu::kR for the long-pair kernel,
 // cwgpu::kRShort for pairs whose first sequence has at most
 // cwgpu_tuning::short_rows residues (128 by default: one 4-row stripe).
-// Separate kernels keep the long-pair code exactly as tuned. Both are held to
-// 5 CTAs (20 warps) per SM, i.e. 96 registers: measured faster than the 113
-// registers and 4 CTAs per SM the compiler picks for the long-pair kernel
-// unbounded (1000 x 1523 protein family, 200 sequences: 110.3 vs 114.7 ms).
+// k_pairwise divides every pair; long pairs run it in sets without kept rows
+// (pair_kernel), else k_pairwise_long. All are held to 5 CTAs (20 warps) per SM,
+// i.e. 96 registers; with 4 CTAs 200 x 1523 proteins took 50.8 ms against 48.6 and
+// 300 x 97 3.42 against 3.32, 200 x 1002 DNA 24.7 against 25.3.
 // GEN: any gap penalties (cwgpu::padding_sound says when the other form holds).
 template <int RS, bool GEN>
 __global__ void __launch_bounds__(kWarpsPerBlock * 32, 5)
@@ -514,8 +514,8 @@ __device__ void cta_pair(const cwgpu::PairArgs& g, long long q, CtaCtl& C, const
             // The path from the kept rows (cwgpu_path.cuh): rows, boxes and the
             // walk's frames dealt over the warps. Against diff()'s divisions by
             // the whole CTA: one column of 100 DNA sequences of 1523 residues
-            // 1.95 to 1.6 ms, the 15 pairs of six proteins of 3000 3.9 to 2.8
-            // to 3.5 ms (by family).
+            // 1.95 to 1.6 ms, the 15 pairs of six proteins of 3000 3.9 to 2.3
+            // to 4.9 ms (by family: weak pairs leave large frames to one warp).
             if (path && cwgpu::path_scores(max_score, go) && se1 - A0 >= cwgpu::kMinPathRows) {
                 int2* const band = bufs + stride / 2;  // of warp 0: no sweep uses it
                 const cwgpu::PathMem own = cwgpu::path_of_warp(pm, warp);
@@ -1026,9 +1026,9 @@ cudaError_t launch_persistent(const cwgpu::PairArgs& g, int max_grid, size_t sme
 // 16 for at most half a pair per SM, 8 up to 2 pairs per SM, else 4; always 4
 // for sets of one stripe, which have no stripes to share. Each measured in a
 // new context, on families of 1523 residues with 16 / 8 / 4 warps: 28 pairs 1.46 /
-// 1.43 / 1.80 ms, 153 pairs 1.91 / 1.49 / 1.88, 300 pairs 3.17 / 2.46 / 2.78, 435
-// pairs 4.04 / 3.43 / 2.93; of 3000 residues: 15 pairs 3.19 / 3.66 / 4.81, 78 pairs
-// 4.77 / 5.14 / 6.18; of 200: 28 pairs 0.276 / 0.253 / 0.241.
+// 1.43 / 1.80 ms, 153 pairs 1.91 / 1.53 / 2.20, 300 pairs 2.89 / 2.14 / 2.58, 435
+// pairs 3.68 / 2.90 / 2.73; of 3000 residues: 15 pairs 3.19 / 3.69 / 4.82, 78 pairs
+// 4.72 / 5.14 / 6.13; of 200: 28 pairs 0.275 / 0.250 / 0.241.
 int cta_warps_for(const cwgpu_context* ctx, int64_t nlong) {
     if (ctx->cta_warps) return ctx->cta_warps;
     if (ctx->lmax < cwgpu::kMinPathLength) return 4;
@@ -1065,11 +1065,10 @@ cudaError_t launch_cta(const cwgpu_context* ctx, const cwgpu::PairArgs& g, int p
 // (below that one warp per pair leaves the SMs too few warps to hide a pair's
 // own latency); in sets of one stripe, as many CTAs as run at once. Measured in
 // new contexts, one warp against 4-warp CTAs, families of 400 / 1523 residues: 780
-// pairs 1.11 / 7.0 against 0.79 / 4.6 ms, 990 pairs 1.16 / 7.1 against 0.82 / 4.9, 1,485
-// pairs 1.44 / 7.5 against 1.10 / 6.2; unrelated sequences of 400 / 1000: 990 pairs
-// 1.01 / 3.95 against 1.08 / 3.36, 1,485 pairs 1.14 / 4.30 against 1.47 / 4.48; families
-// of 130 / 200: 595 pairs 0.23 / 0.33 against 0.24 / 0.31, 780 pairs 0.25 / 0.36 against
-// 0.25 / 0.48, 990 pairs 0.26 / 0.37 against 0.27 / 0.51.
+// pairs 1.10 / 6.6 against 0.76 / 4.2 ms, 990 pairs 1.17 / 7.1 against 0.81 / 4.7, 1,485
+// pairs 1.47 / 7.7 against 1.09 / 6.4; unrelated sequences of 400 / 1000: 990 pairs
+// 1.01 / 3.88 against 1.06 / 3.19, 1,485 pairs 1.14 / 4.33 against 1.43 / 4.42; families
+// of 200: 435 pairs 0.32 against 0.27, 780 pairs 0.36 against 0.48.
 bool use_cta(const cwgpu_context* ctx, int64_t nlong) {
     const int ctas = ctx->grid_cta[log2_warps(cta_warps_for(ctx, nlong))];
     int64_t limit = ctx->lmax < cwgpu::kMinPathLength ? ctas : (int64_t)ctx->grid * kWarpsPerBlock * 2 / 5;

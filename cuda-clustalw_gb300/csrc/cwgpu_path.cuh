@@ -802,9 +802,8 @@ __device__ inline int path_extent(const int2* band, int A, int M, int most) {
 // + (type 2), or -1 if a row of a box left out is in the way, or mm_align's
 // steps cost less (a row or 32 columns here about as much as three cells of the
 // frame there). A lane alone spent 150 to 300 cycles per cell on frames this
-// wide, up to 27 million per pair of weak alignments of 1600 residues (of 46 in
-// all); row by row 250. A call of its own: inlined it took registers from the
-// walk (200 x 1523: 52.1 against 51.4 ms).
+// wide, the warp 250 per row. A call of its own: inlined it took registers from
+// the walk (200 x 1523: 52.1 against 51.4 ms).
 template <bool NC>
 __device__ __noinline__ int path_midpoint_warp(const int8_t* s1, const int8_t* s2, const int2* band, int2* rows, int A,
                                                int B, int M, int N, int tb, int te, int go, int ge, int nw,
