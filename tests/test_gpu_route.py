@@ -250,3 +250,17 @@ def test_a_cta_walks_the_path(oracle_mod, kind, scheme, warps):
     assert kept > 0
     if kind == "edges":
         assert (kept, left) == (len(pairs), 0)
+
+
+@pytest.mark.parametrize("length, kept", [(1500, 1), (2200, 1), (3060, 1), (3200, 0)])
+def test_rows_kept_further_apart_and_not_at_all(oracle_mod, length, kept):
+    """With a slice for every warp of the long-pair kernel (sets of 56 sequences
+    and more) one holds rows every 32 of 1500 residues, every 64 of 2200, every
+    128 of 3060 and none of 3200."""
+    from clustalw_gb300 import load_matrix, native
+
+    matrix, params = load_matrix("protein")
+    seqs = related(2, length + 3, 4) + related(62, 40, 5)
+    with native.Context(0) as ctx:
+        ctx.set_cta_tuning(max_pairs=0)
+        assert run(ctx, oracle_mod, seqs, matrix, params, np.array([[0, 1]], dtype=np.int32))[0] == kept
